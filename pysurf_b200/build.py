@@ -14,14 +14,17 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIBRARY = os.path.join(HERE, 'libpysurf_b200.so')
-SOURCES = ['csrc/sph_kernels.cu', 'csrc/sph_sweep_kernels.cu', 'csrc/sph_system.cu', 'csrc/sph_noalloc.cu',
-           'csrc/sph_surface.cu', 'csrc/sph_merge.cu']
+OBJECTS = os.path.join(HERE, '_build')
+# each unit's source and definitions, compiled side by side; the sweeps once a dimension
+UNITS = [('csrc/sph_sweep_kernels.cu', ['-DSPH_SWEEP_DIM=3']), ('csrc/sph_sweep_kernels.cu', ['-DSPH_SWEEP_DIM=2']),
+         ('csrc/sph_classic_sweeps.cu', []), ('csrc/sph_kernels.cu', []), ('csrc/sph_system.cu', []), ('csrc/sph_noalloc.cu', []),
+         ('csrc/sph_surface.cu', []), ('csrc/sph_merge.cu', [])]
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
-FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC', '-shared']
+FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC']
 
 
 def inputs() -> list:
-    files = [os.path.join(HERE, s) for s in SOURCES]
+    files = [os.path.join(HERE, s) for s, _ in UNITS]
     files += glob.glob(os.path.join(HERE, 'csrc', '*.cuh')) + glob.glob(os.path.join(HERE, 'csrc', '*.h'))
     files.append(os.path.join(ROOT, 'include', 'pysurf_b200.h'))
     return files
@@ -38,9 +41,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not stale():
         return LIBRARY
     nvcc = os.environ.get('NVCC', 'nvcc')
-    command = [nvcc] + ARCH + FLAGS + ['-o', LIBRARY] + [os.path.join(HERE, s) for s in SOURCES]
+    os.makedirs(OBJECTS, exist_ok=True)
+    objects, running = [], []
+    for k, (source, defines) in enumerate(UNITS):
+        objects.append(os.path.join(OBJECTS, f'unit{k}.o'))
+        command = [nvcc] + ARCH + FLAGS + defines + ['-c', '-o', objects[-1], os.path.join(HERE, source)]
+        if verbose:
+            print(' '.join(command), flush=True)
+        running.append((command, subprocess.Popen(command, cwd=HERE)))
+    failed = [command for command, process in running if process.wait() != 0]
+    if failed:
+        raise subprocess.CalledProcessError(1, failed[0])
+    command = [nvcc] + ARCH + ['-shared', '-o', LIBRARY] + objects
     if verbose:
-        print(' '.join(command))
+        print(' '.join(command), flush=True)
     subprocess.check_call(command, cwd=HERE)
     return LIBRARY
 

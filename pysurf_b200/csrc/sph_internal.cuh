@@ -31,17 +31,11 @@
 namespace sph {
 
 constexpr int kBlock = 128;                 // threads per sweep block
-#ifndef SPH_SWEEP_MIN_BLOCKS
-#define SPH_SWEEP_MIN_BLOCKS 8
-#endif
-#ifndef SPH_SWEEP_MIN_BLOCKS_3D
-#define SPH_SWEEP_MIN_BLOCKS_3D 6
-#endif
-// Resident sweep blocks an SM, which caps a sweep's registers: in 2D 8 blocks of 128 (64 registers)
-// give the warps that hide the neighbours' load latency; the 3D sweeps' 3 x 3 sums want about 105
-// registers, and 6 blocks (80 registers, a few spilled) ran faster than 4 (none spilled) or 5.
+// Resident sweep blocks an SM, which caps a sweep's registers: the momentum sweep runs fastest at 5 in 2D
+// (0.084 ms on the 64-ppd beach against 0.088 at 6) and 4 in 3D (16.5 ms on the 20-ppd ridge against 20.1
+// at 5).
 template <int D>
-constexpr int sweepMinBlocks() { return D == 2 ? SPH_SWEEP_MIN_BLOCKS : SPH_SWEEP_MIN_BLOCKS_3D; }
+constexpr int sweepMinBlocks() { return D == 2 ? 5 : 4; }
 constexpr float kViscositySoftening = 0.01f;   // mu_ij's r^2 + 0.01 h^2 (src/pysurf/sphSolver.py:213)
 constexpr float kCloseDistance = 0.3f;      // limiter fade (src/pysurf/sphSolver.py:220-221)
 constexpr float kFoldWidth = 0.2f;
@@ -108,10 +102,12 @@ struct Params {
     float spacingKernel, shiftThreshold, lopsidedness;
     double shiftScale;      // c0 Ma 4 h: the size CFL Ma (2h)^2 = shiftScale dt
     double shiftDt;         // the host-step call's dt (the device steps take ctl->dt)
-    // neighbour table: up to listCap entries a particle (a multiple of 4), entry k of slot i at
-    // 4 ((k / 4) listStride + i) + k % 4; listCap 0: no table, the sweeps walk the cells
+    // neighbour table: up to listCap entries a particle (a multiple of 8), entry k of slot i at
+    // 4 ((k / 4) listStride + i) + k % 4, fluid neighbours from the front (0, 1, ...) and boundary
+    // neighbours from the back (listCap - 1, listCap - 2, ...); listCap 0: no table, the sweeps walk the cells
     int listCap;
     int listStride;
+    int together;           // the classic scheme's rows: both kinds from the front, in the walk's order
     // energy budget (src/pysurf/sphEnergy.py): each particle's running total of each term, by caller
     // index, column t at t * energyStride; the momentum sweep's parts of a at q * energyStride + slot
     int budget;
@@ -128,6 +124,10 @@ struct Frame {
     int *cell;              // sorted cell index of each slot
     const int *cellStart;   // lower bound of each cell in the sorted order, numCells + 1 entries
     float4 *G0, *G1, *G2;   // velocity gradient rows (2D: G0 = (G00, G01, G10, G11))
+    // the slopes' coefficients, r . G r = sum over a <= b of them times r_a r_b: G_aa, and G_ab + G_ba.
+    // 2D: S0 = (G00, G01 + G10, G11, -); 3D: S0 = (00, 01 + 10, 02 + 20, 11), S1 = (12 + 21, 22)
+    float4 *S0;
+    float2 *S1;
     float4 *L0, *L1, *L2;   // correction matrix rows, same packing
     float4 *gradRho;        // renormalized density gradient
     float4 *acc;            // acceleration (w: unused)
@@ -140,8 +140,9 @@ struct Frame {
     float4 *shiftGrad, *shiftPlain, *shiftRhoGrad, *shift, *shiftDv;
     double *energy;         // energy budget: kEnergyTerms columns, by caller index
     float4 *parts;          // energy budget: pressure and viscosity of a from fluid and from boundary neighbours
+    unsigned *wallBits;     // one bit a slot, set where it is boundary, 32 slots a word
     int *nbr;               // neighbour table (chunks of four), top bit: a pair across the periodic seam
-    int *ncount;            // each slot's neighbour count (may exceed the table's capacity)
+    int2 *ncount;           // each slot's fluid and boundary neighbours (together they may exceed the row)
     // master (current buffers)
     double *x[3], *v[3], *rho, *m, *h;
     uint8_t *fluid;
@@ -194,49 +195,54 @@ __device__ __forceinline__ KernelAt kernelAt(float unit, float h)
     return k;
 }
 
+// The constants of two neighbours' pairs, side by side.
+struct KernelPair {
+    float2 invH, sigma, gradC, soft;
+    __device__ __forceinline__ KernelAt of(int q) const
+    {
+        return q ? KernelAt{invH.y, sigma.y, gradC.y, soft.y} : KernelAt{invH.x, sigma.x, gradC.x, soft.x};
+    }
+};
+__device__ __forceinline__ KernelPair kernelPair(const KernelAt &a, const KernelAt &b)
+{
+    return KernelPair{make_float2(a.invH, b.invH), make_float2(a.sigma, b.sigma), make_float2(a.gradC, b.gradC),
+                      make_float2(a.soft, b.soft)};
+}
+
 // A pair's kernel constants at h_ij: one set a thread when every particle has the same smoothing
-// length (then h_ij = hMax), else taken per pair.  HOLD (mixed lengths): the set is held at the
-// particle's own length instead, which every pair with a neighbour of the same length has
-// (0.5 (h + h) = h exactly), so those pairs, all but the few across a refinement zone's edge, take
-// the held set and the rest take theirs per pair, with the same bits either way.  It pays where a
-// sweep has registers to spare (measured: the refined 3D ridge's gradients 10.2 -> 9.7 ms, while
-// continuity, at its register cap, went 11.5 -> 12.2).
-template <int K, int D, bool HOLD = false>
+// length (then h_ij = hMax), else the set is held at the particle's own length, which every pair with
+// a neighbour of the same length has (0.5 (h + h) = h exactly), so those pairs, all but the few across
+// a refinement zone's edge, take the held set and the rest take theirs per pair, with the same bits
+// either way.
+template <int K, int D, bool MIXED>
 struct Smoothing {
     KernelAt fixed;
     float held;     // the length `fixed` is taken at
     float unit;
-    bool mixed;
-    __device__ __forceinline__ static float heldLength(const Params &P, float own)
+    // own: the particle's smoothing length
+    __device__ __forceinline__ explicit Smoothing(const Params &P, float own)
+        : fixed(kernelAt<K, D>(P.sigmaUnit, MIXED ? own : P.hMax)), held(own), unit(P.sigmaUnit) {}
+    __device__ __forceinline__ KernelPair at(const float2 &h) const
     {
-        return HOLD && P.mixedH && own > 0.0f ? own : P.hMax;
-    }
-    // own: the particle's smoothing length (HOLD only)
-    __device__ __forceinline__ explicit Smoothing(const Params &P, float own = 0.0f)
-        : fixed(kernelAt<K, D>(P.sigmaUnit, heldLength(P, own))), held(heldLength(P, own)), unit(P.sigmaUnit),
-          mixed(P.mixedH != 0) {}
-    __device__ __forceinline__ KernelAt at(float h) const
-    {
-        if constexpr (HOLD) {
-            if (h == held) return fixed;
-            return kernelAt<K, D>(unit, h);
-        } else {
-            return mixed ? kernelAt<K, D>(unit, h) : fixed;
-        }
+        if (!MIXED || (h.x == held && h.y == held)) return kernelPair(fixed, fixed);
+        return kernelPair(kernelAt<K, D>(unit, h.x), kernelAt<K, D>(unit, h.y));
     }
 };
 
-// W(q h), q < 2.
+// W(q h), q < 2.  Roundings are explicit, so every sweep that inlines these takes the same bits.
 template <int K>
 __device__ __forceinline__ float kernelValue(float q, const KernelAt &k)
 {
     if (K == 1) {
-        float rest = 1.0f - 0.5f * q, sq = rest * rest;
-        return k.sigma * sq * sq * (2.0f * q + 1.0f);
+        const float rest = __fmaf_rn(-0.5f, q, 1.0f), sq = __fmul_rn(rest, rest);
+        return __fmul_rn(__fmul_rn(__fmul_rn(k.sigma, sq), sq), __fmaf_rn(2.0f, q, 1.0f));
     }
-    if (q < 1.0f) return k.sigma * (1.0f - 1.5f * q * q + 0.75f * q * q * q);
-    float rest = 2.0f - q;
-    return k.sigma * 0.25f * rest * rest * rest;
+    if (q < 1.0f) {
+        const float q2 = __fmul_rn(q, q);
+        return __fmul_rn(k.sigma, __fmaf_rn(__fmul_rn(0.75f, q2), q, __fmaf_rn(-1.5f, q2, 1.0f)));
+    }
+    const float rest = __fsub_rn(2.0f, q);
+    return __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(k.sigma, 0.25f), rest), rest), rest);
 }
 
 // (dW/dr) / r at r = q h, 0 < q < 2.
@@ -244,12 +250,23 @@ template <int K>
 __device__ __forceinline__ float kernelGradient(float q, const KernelAt &k)
 {
     if (K == 1) {
-        float rest = 1.0f - 0.5f * q;
-        return k.gradC * rest * rest * rest;
+        const float rest = __fmaf_rn(-0.5f, q, 1.0f);
+        return __fmul_rn(__fmul_rn(__fmul_rn(k.gradC, rest), rest), rest);
     }
-    if (q < 1.0f) return k.gradC * (2.25f * q - 3.0f);
-    float rest = 2.0f - q;
-    return __fdividef(-0.75f * k.gradC * rest * rest, q);
+    if (q < 1.0f) return __fmul_rn(k.gradC, __fmaf_rn(2.25f, q, -3.0f));
+    const float rest = __fsub_rn(2.0f, q);
+    return __fdividef(__fmul_rn(__fmul_rn(__fmul_rn(-0.75f, k.gradC), rest), rest), q);
+}
+
+// (dW/dr) / r of two neighbours, each rounded as the single form.
+template <int K>
+__device__ __forceinline__ float2 kernelGradient(const float2 &q, const KernelPair &k)
+{
+    if (K == 1) {
+        const float2 rest = __ffma2_rn(make_float2(-0.5f, -0.5f), q, make_float2(1.0f, 1.0f));
+        return __fmul2_rn(__fmul2_rn(__fmul2_rn(k.gradC, rest), rest), rest);
+    }
+    return make_float2(kernelGradient<K>(q.x, k.of(0)), kernelGradient<K>(q.y, k.of(1)));
 }
 
 // (dW/dr) / r in float64 at a pair's float64 distance r, with the pair's (float32) kernel constants:
@@ -519,6 +536,26 @@ template <> __device__ __forceinline__ void storeMatrix<3>(float4 *R0, float4 *R
     R0[j] = make_float4(M[0][0], M[0][1], M[0][2], 0.0f);
     R1[j] = make_float4(M[1][0], M[1][1], M[1][2], 0.0f);
     R2[j] = make_float4(M[2][0], M[2][1], M[2][2], 0.0f);
+}
+
+// The slopes' coefficients of slot j (Frame::S0, S1), in the order (0,0), (0,1), (0,2), (1,1), ...
+template <int D> __device__ __forceinline__ void loadSlopes(const Frame &F, int j, float s[6])
+{
+    const float4 a = __ldg(&F.S0[j]);
+    s[0] = a.x; s[1] = a.y; s[2] = a.z;
+    if (D == 3) {
+        const float2 b = __ldg(&F.S1[j]);
+        s[3] = a.w; s[4] = b.x; s[5] = b.y;
+    }
+}
+template <int D> __device__ __forceinline__ void storeSlopes(const Frame &F, int j, const float G[3][3])
+{
+    if (D == 2) {
+        F.S0[j] = make_float4(G[0][0], G[0][1] + G[1][0], G[1][1], 0.0f);
+    } else {
+        F.S0[j] = make_float4(G[0][0], G[0][1] + G[1][0], G[0][2] + G[2][0], G[1][1]);
+        F.S1[j] = make_float2(G[1][2] + G[2][1], G[2][2]);
+    }
 }
 
 template <int D, class R> __device__ __forceinline__ R determinant(const R M[3][3])

@@ -172,6 +172,7 @@ __global__ void gatherKernel(Params P, int n, const int *perm, MasterView from, 
 {
     if (ctl && !ctl->active) return;
     int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned present = __ballot_sync(0xFFFFFFFFu, s < n);
     if (s >= n) return;
     int o = perm[s];
     double x[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
@@ -185,6 +186,8 @@ __global__ void gatherKernel(Params P, int n, const int *perm, MasterView from, 
     double m64 = from.m[o], h64 = from.h[o];
     float m = (float)m64, h = (float)h64;
     uint8_t fl = from.fluid[o];
+    const unsigned walls = __ballot_sync(present, !fl);
+    if ((s & 31) == 0) F.wallBits[s >> 5] = walls;
     to.rho[s] = rho;
     to.m[s] = m64;
     to.h[s] = h64;

@@ -34,6 +34,9 @@ struct Enforcement {
 
 enum class Stage { ShepardSum, ShepardApply, Wall, Gradients, Momentum, Kick, Continuity, Xsph, List, Closure, ShiftFields, Shift, ShiftDrift, FrameDensity };
 
+// Gradients: the whole velocity gradients rather than the slopes' coefficients that a step reads.
+constexpr int kWholeGradients = 2;
+
 struct LaunchArgs {
     Params P;
     Frame F;
@@ -42,14 +45,28 @@ struct LaunchArgs {
     int maxima;             // Momentum: fold the fluid maxima into ctl and take the time step
     Enforcement E;
     int flag;               // Wall: write the density too; Continuity / Xsph: the epilogue's mode
-    int wantG, wantL, wantRho;
+    int wantG, wantL, wantRho;  // Gradients: wantG the slopes' coefficients, or kWholeGradients
     float floorDet;
     const float *densities; // Xsph: the densities it divides by; null for the frame's
     int threads;            // threads per particle in the sweeps: 1, 2, 4 or 8
     int *maxCount;          // List: the largest neighbour count goes here (atomic max), when given
 };
 
-void launchStage(const LaunchArgs &A, Stage stage);
+// The stages of a 2D and a 3D system (sph_sweep_kernels.cu), and of the classic scheme, where it has its
+// own (sph_classic_sweeps.cu; false where it has none).
+void launchStage2(const LaunchArgs &A, Stage stage);
+void launchStage3(const LaunchArgs &A, Stage stage);
+bool launchClassicStage(const LaunchArgs &A, Stage stage);
+inline void launchStage(const LaunchArgs &A, Stage stage)
+{
+    LaunchArgs B = A;
+    if (A.P.together) {
+        if (launchClassicStage(A, stage)) return;
+        if (stage != Stage::List) B.P.listCap = 0;      // the paired sweeps' rows part the kinds: walk the cells
+    }
+    if (A.P.dim == 2) launchStage2(B, stage);
+    else launchStage3(B, stage);
+}
 
 // A merge of split particles (sph_merge.cu): the current master and the buffer it moves into, with
 // that buffer's frame, the step's parameters, the frame's accelerations and pressures, the energy

@@ -21,38 +21,23 @@
 
 #include "sph_enforce.cuh"
 #include "sph_kernels.h"
+#include "sph_step.cuh"
 #include "sph_sweeps.cuh"
 
 namespace sph {
 
-// Blocks an SM the energy budget's momentum and continuity sweeps are built for: their extra
-// accumulators need about 100 registers a thread in 2D (5 blocks of 128 threads leave 102).
+// Resident blocks of 128 threads an SM each sweep is built for, which caps its registers.  A sweep holds
+// two neighbours' rows, and the next two's in flight, so it wants 90 to 160 registers; each bound is the
+// fastest of those measured around it on the 64-ppd beach (2D) and the 20-ppd and the refined 11-ppd
+// ridge (3D).  The energy budget's sweeps carry more sums.
 template <int D>
-constexpr int budgetMinBlocks() { return D == 2 ? 5 : 4; }
-// The gradients and continuity sweeps carry float64 sums beside their float32 ones (M; the wall pairs'
-// terms), so they take more registers a thread and fewer resident blocks.  Continuity also keeps the
-// next neighbour's five rows in flight: at 4 blocks in 3D (128 registers, none spilled) it runs 16-25%
-// faster than at 5 (96, spilling) on the ridges, and at 5 in 2D (102) 3.5% faster than at 6 on the
-// beach (measured).
-#ifndef SPH_PRECISE_MIN_BLOCKS
-#define SPH_PRECISE_MIN_BLOCKS 5
-#endif
-#ifndef SPH_PRECISE_MIN_BLOCKS_3D
-#define SPH_PRECISE_MIN_BLOCKS_3D 4
-#endif
+constexpr int budgetMinBlocks() { return D == 2 ? 4 : 3; }
+// continuity: 5 in 2D (0.082 ms against 0.084 at 4), 4 in 3D (20.3 ms against 21.3 at 3)
 template <int D>
-constexpr int preciseMinBlocks() { return D == 2 ? SPH_PRECISE_MIN_BLOCKS : SPH_PRECISE_MIN_BLOCKS_3D; }
-// The 3D gradients sweep keeps three 3 x 3 float32 sums and the float64 M: at 4 blocks (128
-// registers) it ran 7-17% faster than at 5 on the ridges; in 2D 6 blocks (80 registers) ran 3%
-// faster than 5 on the beach (measured).
-#ifndef SPH_GRADIENT_MIN_BLOCKS
-#define SPH_GRADIENT_MIN_BLOCKS 6
-#endif
-#ifndef SPH_GRADIENT_MIN_BLOCKS_3D
-#define SPH_GRADIENT_MIN_BLOCKS_3D 4
-#endif
+constexpr int preciseMinBlocks() { return D == 2 ? 5 : 4; }
+// gradients: 5 in 2D (0.061 ms against 0.070 at 6), 3 in 3D (15.9 ms against 16.6 at 4)
 template <int D>
-constexpr int gradientMinBlocks() { return D == 2 ? SPH_GRADIENT_MIN_BLOCKS : SPH_GRADIENT_MIN_BLOCKS_3D; }
+constexpr int gradientMinBlocks() { return D == 2 ? 5 : 3; }
 
 // ------------------------------------------------------------------------------------------
 // The neighbour table
@@ -62,7 +47,25 @@ constexpr int gradientMinBlocks() { return D == 2 ? SPH_GRADIENT_MIN_BLOCKS : SP
 #define SPH_LIST_TRIM 1
 #endif
 
-// Each slot's neighbours in the walk's order (forEachNeighbour's, with its tests), from a group of
+// Whether a slot is fluid, and whether a run of slots holds a boundary slot, from the slots' bits (32 a
+// word, so a run of a stencil row is a few words).
+__device__ __forceinline__ bool isFluid(const Frame &F, int j)
+{
+    return !(__ldg(&F.wallBits[j >> 5]) >> (j & 31) & 1);
+}
+__device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
+{
+    unsigned any = 0;
+    for (int w = first >> 5; w <= (end - 1) >> 5; ++w) {
+        unsigned bits = __ldg(&F.wallBits[w]);
+        if (w == first >> 5) bits &= 0xFFFFFFFFu << (first & 31);
+        if (w == (end - 1) >> 5) bits &= 0xFFFFFFFFu >> (31 - ((end - 1) & 31));
+        any |= bits;
+    }
+    return any != 0;
+}
+
+// Each slot's neighbours in the walk's order (sumPairs', with its tests), from a group of
 // L lanes: lane t tests candidates t, t + L, ... of each run of the stencil, and the group's ballot
 // places the accepted ones in order.  The count is the whole count even when the row is full (the
 // sweeps then walk the cells for that slot).  maxCount: the largest count, when given.
@@ -73,7 +76,7 @@ constexpr int gradientMinBlocks() { return D == 2 ? SPH_GRADIENT_MIN_BLOCKS : SP
 // candidate the coarse test passes stays: the accepted neighbours and their order are those of the
 // whole stencil.  PRECISE: separations from point and remainder; MIXED: smoothing lengths differ.
 template <int D, int L, bool PRECISE, bool MIXED>
-__global__ void __launch_bounds__(kBlock) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
+__global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
     if (ctl && !ctl->active) return;
     const Group<L> G = groupOf<L>();
@@ -84,7 +87,7 @@ __global__ void __launch_bounds__(kBlock) listKernel(Params P, Frame F, const Co
     const unsigned lower = (1u << t) - 1u;
     const float4 Ai = __ldg(&F.pa[i]), Bi = __ldg(&F.pb[i]);
     const float hI = fabsf(signedLengthIn<D>(Ai, Bi));
-    // a boundary row holds its fluid neighbours only (forEachNeighbour says why)
+    // a boundary row holds its fluid neighbours only (Row says why)
     const bool fluidOnly = signedLengthIn<D>(Ai, Bi) <= 0.0f;
     float pi[3], li[3];
     pointIn<D>(Ai, pi);
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kBlock) listKernel(Params P, Frame F, const Co
     const int ownCell = F.cell[i];
     const float fineReach = hI + P.fineMax, fineLimit = kCandidateMargin * fineReach * fineReach;
     int *column = F.nbr + 4 * (size_t)i;
-    int count = 0;
+    int count = 0, wallCount = 0;
     // search s: grid level s >> 1 (coarse, fine), origin s & 1 (the particle, its periodic image)
     for (int search = 0; search < (MIXED ? 4 : 2); ++search) {
         const int level = MIXED ? search >> 1 : 0, image = search & 1;
@@ -123,59 +126,86 @@ __global__ void __launch_bounds__(kBlock) listKernel(Params P, Frame F, const Co
         const float fy = (float)(((double)pi[1] + (image ? shift64 : 0.0) - origin[1]) / width) - (float)box.cy;
         const bool trim = SPH_LIST_TRIM && fx >= 0.0f && fx < 1.0f && fy >= 0.0f && fy < 1.0f && fz >= 0.0f &&
                           fz < 1.0f;
-        for (int zz = box.z0; zz <= box.z1; ++zz) {
-            const int oz = zz - box.cz;
-            const float dz = oz > 0 ? (float)oz - fz : (oz < 0 ? fz - (float)(oz + 1) : 0.0f);
-            for (int yy = box.y0; yy <= box.y1; ++yy) {
+        // one run of candidates, L at a time; WALLED: it holds boundary slots
+        auto takeRun = [&](auto walled, int first, int end) {
+            constexpr bool WALLED = decltype(walled)::value;
+            for (int base = first; base < end; base += L) {
+                const int j = base + t;
+                bool accepted = false, fluidJ = true;
+                if (j < end && j != i) {
+                    const float4 A = __ldg(&F.pa[j]);
+                    float pj[3];
+                    pointIn<D>(A, pj);
+                    if (WALLED) fluidJ = isFluid(F, j);
+                    const float coarse = !WALLED || fluidJ || !fluidOnly ? coarseDistance2<D>(pi, pj, offset) : searchLimit;
+                    if (PRECISE && !image && level == 0 && coarse < sure) {
+                        accepted = true;
+                    } else if (coarse < searchLimit) {
+                        const float4 B = (D == 3 && PRECISE) || MIXED ? __ldg(&F.pb[j]) : A;
+                        float r2 = coarse;      // the float32 points' separation is the coarse one
+                        if (PRECISE) {
+                            float lj[3], d[3];
+                            remainderIn<D>(A, B, lj);
+                            r2 = separation2<D, 1>(P, pi, li, pj, lj, offset, image, shift64, d);
+                        }
+                        const float bound = MIXED ? support2(0.5f * (hI + fabsf(signedLengthIn<D>(A, B)))) : support;
+                        accepted = r2 < bound;
+                    }
+                }
+                const unsigned all = (L >= 32 ? 0u : 1u << L) - 1u;
+                const bool front = !WALLED || fluidJ || P.together;
+                const unsigned bits = (__ballot_sync(G.mask, accepted) >> shift) & all;
+                const unsigned walls = WALLED ? (__ballot_sync(G.mask, accepted && !front) >> shift) & all : 0u;
+                if (accepted) {
+                    const int k = front ? count + __popc(bits & ~walls & lower) : wallCount + __popc(walls & lower);
+                    if (k < P.listCap) {
+                        const int e = front ? k : P.listCap - 1 - k;
+                        column[((size_t)(e >> 2) * P.listStride) * 4 + (e & 3)] = image ? (j | (int)0x80000000) : j;
+                    }
+                }
+                count += __popc(bits & ~walls);
+                if (WALLED) wallCount += __popc(walls);
+            }
+        };
+        // lane t takes the run of every L-th stencil row, trimmed; the group then walks the rows in order
+        const int across = box.y1 - box.y0 + 1, rows = across * (box.z1 - box.z0 + 1);
+        for (int block = 0; block < rows; block += L) {
+            int runFirst = 0, runEnd = 0;
+            bool runWalls = false;
+            if (block + t < rows) {
+                const int zz = box.z0 + (D == 3 ? (block + t) / across : 0), yy = box.y0 + (block + t) % across;
                 int xa = box.x0, xb = box.x1;
+                bool empty = false;
                 if (trim) {
-                    const int oy = yy - box.cy;
+                    const int oz = zz - box.cz, oy = yy - box.cy;
+                    const float dz = oz > 0 ? (float)oz - fz : (oz < 0 ? fz - (float)(oz + 1) : 0.0f);
                     const float dy = oy > 0 ? (float)oy - fy : (oy < 0 ? fy - (float)(oy + 1) : 0.0f);
                     const float rem = R * R - dy * dy - dz * dz;
-                    if (rem < 0.0f) continue;
-                    const float ext = sqrtf(rem);
+                    empty = rem < 0.0f;
+                    const float ext = sqrtf(fmaxf(rem, 0.0f));
                     xa = max(box.x0, box.cx + (int)floorf(fx - ext));
                     xb = min(box.x1, box.cx + (int)floorf(fx + ext));
                 }
-                const int row = box.first + (zz * box.ny + yy) * box.nx;
-                const int first = __ldg(&F.cellStart[row + xa]), end = __ldg(&F.cellStart[row + xb + 1]);
-                for (int base = first; base < end; base += L) {
-                    const int j = base + t;
-                    bool accepted = false;
-                    if (j < end && j != i) {
-                        const float4 A = __ldg(&F.pa[j]);
-                        float pj[3];
-                        pointIn<D>(A, pj);
-                        const bool inRow = !fluidOnly || (D == 3 ? A.w > 0.0f : __ldg(&F.fluid[j]) != 0);
-                        const float coarse = inRow ? coarseDistance2<D>(pi, pj, offset) : searchLimit;
-                        if (PRECISE && !image && level == 0 && coarse < sure) {
-                            accepted = true;
-                        } else if (coarse < searchLimit) {
-                            const float4 B = (D == 3 && PRECISE) || MIXED ? __ldg(&F.pb[j]) : A;
-                            float r2 = coarse;      // the float32 points' separation is the coarse one
-                            if (PRECISE) {
-                                float lj[3], d[3];
-                                remainderIn<D>(A, B, lj);
-                                r2 = separation2<D, 1>(P, pi, li, pj, lj, offset, image, shift64, d);
-                            }
-                            const float bound = MIXED ? support2(0.5f * (hI + fabsf(signedLengthIn<D>(A, B)))) : support;
-                            accepted = r2 < bound;
-                        }
-                    }
-                    const unsigned bits = (__ballot_sync(G.mask, accepted) >> shift) & ((L >= 32 ? 0u : 1u << L) - 1u);
-                    if (accepted) {
-                        const int k = count + __popc(bits & lower);
-                        if (k < P.listCap)
-                            column[((size_t)(k >> 2) * P.listStride) * 4 + (k & 3)] = image ? (j | (int)0x80000000) : j;
-                    }
-                    count += __popc(bits);
+                if (!empty) {
+                    const int row = box.first + (zz * box.ny + yy) * box.nx;
+                    runFirst = __ldg(&F.cellStart[row + xa]);
+                    runEnd = __ldg(&F.cellStart[row + xb + 1]);
+                    runWalls = runHasWalls(F, runFirst, runEnd);
                 }
+            }
+            const unsigned walledRows = __ballot_sync(G.mask, runWalls) >> shift;
+            const int last = min(L, rows - block);
+            for (int q = 0; q < last; ++q) {
+                const int first = __shfl_sync(G.mask, runFirst, q, L), end = __shfl_sync(G.mask, runEnd, q, L);
+                // most runs hold no boundary slot: their candidates' kinds are not read
+                if (walledRows >> q & 1) takeRun(std::true_type{}, first, end);
+                else takeRun(std::false_type{}, first, end);
             }
         }
     }
     if (t != 0) return;
-    F.ncount[i] = count;
-    if (maxCount) atomicMax(maxCount, count);
+    F.ncount[i] = make_int2(count, wallCount);
+    if (maxCount) atomicMax(maxCount, count + wallCount);
 }
 
 // The same table from a warp that takes a batch of up to kBatch particles of one cell together
@@ -188,31 +218,24 @@ __global__ void __launch_bounds__(kBlock) listKernel(Params P, Frame F, const Co
 //
 // A warp owns the batches that start in its kBatch slots: a batch starts at a cell's first slot and
 // every kBatch slots after it, so each slot belongs to one batch.
-#ifndef SPH_LIST_BATCH
-#define SPH_LIST_BATCH 8
-#endif
-constexpr int kBatch = SPH_LIST_BATCH;
 
 // A batch member as the warp's lanes read it, in 16-byte rows so that each read is one shared load:
 // the run and flags decide whether the member takes a chunk at all, the point its coarse test, the
 // remainder only the few candidates near the edge of its support.  The set-up lane writes the
 // search's bounds into point.w and rest.w as each search starts.
-constexpr int kMemberSeam = 1;          // the member searches its periodic image too
-constexpr int kMemberFluidOnly = 2;     // a boundary member: its row holds fluid neighbours only
 struct alignas(16) BatchMember {
     float4 point;       // the float32 point; w: this search's sure bound (0 where none applies)
     float4 rest;        // the remainder; w: this search's coarse limit
-    int4 run;           // this row's run of candidates [x, y), the member's slot, its flags
     float4 bounds;      // the limit on the coarse grid, on the fine grid, the sure bound, hI
     double shift64;     // the periodic image's shift (0 when it is not searched)
     float offset;       // the shift as float32
-    float unused;
+    int walls;          // its boundary neighbours so far
 };
 
 // No blocks-a-multiprocessor bound: at the compiler's default the kernel keeps about 24 warps an
 // SM with a few spills, faster than 85-116 registers and no spills at 3 to 6 blocks, or 64
 // registers at 8 (measured).
-template <int D, bool PRECISE, bool MIXED>
+template <int D, int kBatch, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
     if (ctl && !ctl->active) return;
@@ -240,7 +263,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
         // lane p < count sets up member p
         float hIp = 0.0f, pip[3] = {0, 0, 0}, lip[3] = {0, 0, 0};
         double shiftp = 0.0;
-        bool seamp = false;
+        bool seamp = false, wholeRow = false;
         if (lane < count) {
             const int i = b0 + lane;
             const float4 Ai = __ldg(&F.pa[i]), Bi = __ldg(&F.pb[i]);
@@ -256,15 +279,17 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
             BatchMember &m = mine[lane];
             m.point = make_float4(pip[0], pip[1], pip[2], 0.0f);
             m.rest = make_float4(lip[0], lip[1], lip[2], 0.0f);
-            m.run = make_int4(0, 0, i, (seamp ? kMemberSeam : 0) |
-                                           (signedLengthIn<D>(Ai, Bi) <= 0.0f ? kMemberFluidOnly : 0));
+            m.walls = 0;
+            wholeRow = signedLengthIn<D>(Ai, Bi) > 0.0f;
             m.bounds = make_float4(kCandidateMargin * reach * reach, kCandidateMargin * fineReach * fineReach,
                                    PRECISE ? sureBound(P, support, hIp, pip) : 0.0f, hIp);
             m.shift64 = shiftp;
             m.offset = (float)shiftp;
         }
         const bool anySeam = __any_sync(0xFFFFFFFFu, seamp);
-        int counted[kBatch];
+        // the members that take boundary neighbours: a boundary member's row holds fluid neighbours only
+        const unsigned wholeRows = __ballot_sync(0xFFFFFFFFu, wholeRow);
+        int counted[kBatch];    // each member's fluid neighbours so far
 #pragma unroll
         for (int p = 0; p < kBatch; ++p) counted[p] = 0;
         // search s: grid level s >> 1 (coarse, fine), origin s & 1 (the particle, its periodic image)
@@ -306,6 +331,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
             const int zHi = __reduce_max_sync(0xFFFFFFFFu, takes ? box.z1 : INT_MIN);
             const int yLo = __reduce_min_sync(0xFFFFFFFFu, takes ? box.y0 : INT_MAX);
             const int yHi = __reduce_max_sync(0xFFFFFFFFu, takes ? box.y1 : INT_MIN);
+            __syncwarp();
             for (int zz = zLo; zz <= zHi; ++zz) {
                 for (int yy = yLo; yy <= yHi; ++yy) {
                     const int row = gridFirst + (zz * ny + yy) * nx;
@@ -332,17 +358,18 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                             b = __ldg(&F.cellStart[row + xb + 1]);
                         }
                     }
-                    if (lane < count) { mine[lane].run.x = a; mine[lane].run.y = b; }
                     const int uA = __reduce_min_sync(0xFFFFFFFFu, a < b ? a : INT_MAX);
                     const int uB = __reduce_max_sync(0xFFFFFFFFu, a < b ? b : INT_MIN);
-                    __syncwarp();
                     for (int base = uA; base < uB; base += 32) {
+                        // the members whose own run meets this chunk; a candidate of another member's run
+                        // lies past this one's reach, and its distance turns it away
+                        const unsigned takers = __ballot_sync(0xFFFFFFFFu, a < b && a < base + 32 && b > base);
                         const int j = base + lane;
-                        const bool valid = j < uB;
                         float4 A = make_float4(0, 0, 0, 0), B = A;
                         float pj[3] = {0, 0, 0}, lj[3] = {0, 0, 0}, hJ = 0.0f;
                         bool fluidJ = false;
-                        if (valid) {
+                        unsigned offered = 0;       // the members this candidate is offered to
+                        if (j < uB) {
                             A = __ldg(&F.pa[j]);
                             pointIn<D>(A, pj);
                             // the remainders with the point, although a candidate under `sure` needs
@@ -351,20 +378,21 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                             if (PRECISE) remainderIn<D>(A, D == 3 ? B : A, lj);
                             if (MIXED) hJ = fabsf(signedLengthIn<D>(A, B));
                             fluidJ = D == 3 ? A.w > 0.0f : __ldg(&F.fluid[j]) != 0;
+                            offered = fluidJ ? 0xFFFFFFFFu : wholeRows;
+                            if (j >= b0 && j < b0 + kBatch) offered &= ~(1u << (j - b0));      // not to itself
                         }
+                        const bool front = fluidJ || P.together;
+                        const unsigned fronts = __ballot_sync(0xFFFFFFFFu, front);
+                        const int entry = image ? (j | (int)0x80000000) : j;
 #pragma unroll
                         for (int p = 0; p < kBatch; ++p) {
-                            if (p >= count) continue;      // count is the warp's: the loop keeps its trip count
-                            const int4 run = mine[p].run;
-                            if (run.x >= run.y || run.y <= base || run.x >= base + 32) continue;   // the whole warp
-                            if (image && !(run.w & kMemberSeam)) continue;
+                            if (!(takers >> p & 1)) continue;       // the whole warp
+                            const float4 point = mine[p].point;
+                            const float mp[3] = {point.x, point.y, point.z};
+                            const float offset = image ? mine[p].offset : 0.0f;
+                            const float coarse = coarseDistance2<D>(mp, pj, offset);
                             bool accepted = false;
-                            if (valid && j >= run.x && j < run.y && j != run.z &&
-                                (fluidJ || !(run.w & kMemberFluidOnly))) {
-                                const float4 point = mine[p].point;
-                                const float mp[3] = {point.x, point.y, point.z};
-                                const float offset = image ? mine[p].offset : 0.0f;
-                                const float coarse = coarseDistance2<D>(mp, pj, offset);
+                            if (offered >> p & 1) {
                                 if (PRECISE && coarse < point.w) {
                                     accepted = true;
                                 } else {
@@ -384,28 +412,36 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                                 }
                             }
                             const unsigned bits = __ballot_sync(0xFFFFFFFFu, accepted);
-                            if (accepted) {
-                                const int k = counted[p] + __popc(bits & lower);
-                                if (k < P.listCap) {
-                                    int *column = F.nbr + 4 * (size_t)run.z;
-                                    column[((size_t)(k >> 2) * P.listStride) * 4 + (k & 3)] =
-                                        image ? (j | (int)0x80000000) : j;
-                                }
+                            const unsigned got = bits & fronts, walls = bits & ~fronts;
+                            int *column = F.nbr + 4 * (size_t)(b0 + p);
+                            if (accepted && front) {
+                                const int k = counted[p] + __popc(got & lower);
+                                if (k < P.listCap) column[((size_t)(k >> 2) * P.listStride) * 4 + (k & 3)] = entry;
                             }
-                            counted[p] += __popc(bits);
+                            counted[p] += __popc(got);
+                            if (walls) {        // the whole warp
+                                const int before = mine[p].walls;
+                                if (accepted && !front) {
+                                    const int w = before + __popc(walls & lower), e = P.listCap - 1 - w;
+                                    if (w < P.listCap) column[((size_t)(e >> 2) * P.listStride) * 4 + (e & 3)] = entry;
+                                }
+                                __syncwarp();
+                                if (lane == 0) mine[p].walls = before + __popc(walls);
+                                __syncwarp();
+                            }
                         }
                     }
-                    __syncwarp();
                 }
             }
+            __syncwarp();
         }
-        int own = 0;
+        int2 own = make_int2(0, 0);
 #pragma unroll
         for (int p = 0; p < kBatch; ++p)
-            if (lane == p) own = counted[p];
+            if (lane == p) own = make_int2(counted[p], mine[p].walls);
         if (lane < count) {
             F.ncount[b0 + lane] = own;
-            if (maxCount) atomicMax(maxCount, own);
+            if (maxCount) atomicMax(maxCount, own.x + own.y);
         }
         __syncwarp();
     }
@@ -415,31 +451,19 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
 // Sweep S: the Shepard filter
 // ------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ bool filterDue(const Control *ctl)
-{
-    if (!ctl) return true;
-    if (!ctl->active) return false;
-    if (ctl->filterInterval > 0) return ctl->step > 0 && ctl->step % ctl->filterInterval == 0;
-    return ctl->filterNow != 0;
-}
-
-template <int D, int K>
+template <int D, int K, bool FINE>
 struct ShepardVisit {
+    static constexpr bool kCopied = false;
     static constexpr bool kSkipCoincident = false;
     static constexpr bool kKinetic = false;
-    static constexpr bool kBoundaryRows = true;
-    static constexpr bool kWholeBoundaryRows = true;    // the host-step call returns boundary rows too
-    const Frame &F;
-    Smoothing<K, D> S;
+    static constexpr bool kAuxRow = D == 3;
+    Smoothing<K, D, FINE> S;
     float num, den;
-    __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *, float r, float h, bool, int, const float4 &B, const float4 &)
+    __device__ void operator()(int, const float *, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
-        const KernelAt k = S.at(h);
-        const float4 X = auxRow<D>(F, j);
-        float w = kernelValue<K>(r * k.invH, k);
-        num += massIn<D>(B) * w;
-        den += volumeIn<D>(B, X) * w;
+        const float w = kernelValue<K>(__fmul_rn(r, k.invH), k);
+        num = __fmaf_rn(massIn<D>(R.B), w, num);
+        den = __fmaf_rn(volumeIn<D>(R.B, R.X), w, den);
     }
 };
 
@@ -457,9 +481,12 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shepardKernel(Par
     // the particle itself first, as the reference's sums start (src/pysurf/sphGpu.py:781-783)
     float own = sigmaAt(P.sigmaUnit, hI, D);
     float mi = massOf<D>(F, i);
-    ShepardVisit<D, K> visit{F, Smoothing<K, D>(P), G.t == 0 ? mi * own : 0.0f,
+    ShepardVisit<D, K, FINE> visit{Smoothing<K, D, FINE>(P, hI), G.t == 0 ? mi * own : 0.0f,
                              G.t == 0 ? volumeOf<D>(F, i) * own : 0.0f};
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, hI, visit);
+    // the host-step call returns boundary rows too, over all their neighbours, which the table does not hold
+    const Row row = openRow<D, FINE>(P, F, i, G.t, hI, hs <= 0.0f);
+    sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, visit);
+    sumPairs<D, T, FINE, kWallPair>(P, F, row, false, visit);
     float num = groupSum<T>(visit.num, G.mask), den = groupSum<T>(visit.den, G.mask);
     if (G.t != 0) return;
     F.scalar[i] = num / den;
@@ -485,22 +512,21 @@ __global__ void applyShepardKernel(Params P, Frame F, const Control *ctl)
 // Sweep A: extrapolated wall pressure
 // ------------------------------------------------------------------------------------------
 
-template <int D, int K, bool HOLD = false>
+template <int D, int K, bool FINE>
 struct WallVisit {
+    static constexpr bool kCopied = false;
     static constexpr bool kSkipCoincident = false;
     static constexpr bool kKinetic = true;
-    static constexpr bool kBoundaryRows = true;         // it runs boundary rows only
     const Params &P; const Frame &F;
-    Smoothing<K, D, HOLD> S;
+    Smoothing<K, D, FINE> S;
     float weight, total;
-    __device__ bool accept(bool fluidJ) const { return fluidJ; }
-    __device__ void operator()(int j, const float *d, float r, float h, bool, int, const float4 &, const float4 &Kj)
+    __device__ void operator()(int j, const float *d, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
-        const KernelAt k = S.at(h);
-        float w = kernelValue<K>(r * k.invH, k);
-        float gd = P.g[0] * d[0] + P.g[1] * d[1] + (D == 3 ? P.g[2] * d[2] : 0.0f);
-        weight += w;
-        total += w * (pressureOf<D>(F, j) + densityIn<D>(Kj) * gd);
+        const float w = kernelValue<K>(__fmul_rn(r, k.invH), k);
+        float gd = __fmaf_rn(P.g[1], d[1], __fmul_rn(P.g[0], d[0]));
+        if (D == 3) gd = __fmaf_rn(P.g[2], d[2], gd);
+        weight = __fadd_rn(weight, w);
+        total = __fmaf_rn(w, __fmaf_rn(densityIn<D>(R.K), gd, pressureOf<D>(F, j)), total);
     }
 };
 
@@ -517,7 +543,7 @@ wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
     float hs = signedLength<D>(F, i);
     if (hs > 0.0f) return;
     WallVisit<D, K, FINE> visit{P, F, Smoothing<K, D, FINE>(P, -hs), 0.0f, 0.0f};
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, -hs, visit);
+    sumPairs<D, T, FINE, kCrossPair>(P, F, openRow<D, FINE>(P, F, i, G.t, -hs), true, visit);
     float weight = groupSum<T>(visit.weight, G.mask), total = groupSum<T>(visit.total, G.mask);
     if (G.t != 0) return;
     float p = 0.0f;
@@ -546,57 +572,84 @@ wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
 template <int D>
 __device__ __forceinline__ constexpr int packed(int a, int b) { return a * D - a * (a - 1) / 2 + (b - a); }
 
-template <int D, int K, bool HOLD = false>
+template <int D, int K, bool FINE>
 struct GradientVisit {
+    static constexpr bool kCopied = D == 3 && !FINE;
+    static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kPipelined = true;
     static constexpr bool kAuxRow = D == 3;
     static constexpr bool kKinetic = true;
-    const Frame &F;
-    Smoothing<K, D, HOLD> kernel;
+    Smoothing<K, D, FINE> S;
     bool wantG, wantL, wantRho;
     float vi[3], devI;
-    float S[3][3], Mf[D * (D + 1) / 2], gsum[3];     // Mf: its upper triangle, packed
-    float4 rowX;
+    // each lane's sums over its even and its odd neighbours: V (v_j - v_i) grad W, and M over the fluid
+    // (its upper triangle, packed)
+    float2 jump[D][D], Mf[D * (D + 1) / 2], gsum[D];
     double M[D * (D + 1) / 2];
-    __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *d, float r, float h, bool fluidJ, int, const float4 &B,
-                               const float4 &Kj)
+    struct Taken {
+        float volume[2];
+        float2 rel[D], difference;      // v_j - v_i, the deviations' difference
+    };
+    template <PairKind KIND>
+    __device__ __forceinline__ Taken take(const Neighbours &, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
-        const KernelAt k = kernel.at(h);
-        const float4 X = D == 3 ? rowX : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        Taken t;
+        t.volume[0] = volumeIn<D>(R0.B, R0.X);
+        t.volume[1] = volumeIn<D>(R1.B, R1.X);
+        float vj0[3], vj1[3];
+        velocityIn<D>(R0.K, vj0);
+        velocityIn<D>(R1.K, vj1);
+        if (KIND == kFluidPair)
+            for (int a = 0; a < D; ++a) t.rel[a] = make_float2(__fsub_rn(vj0[a], vi[a]), __fsub_rn(vj1[a], vi[a]));
+        t.difference = make_float2(__fsub_rn(deviationIn<D>(R0.B, R0.X), devI), __fsub_rn(deviationIn<D>(R1.B, R1.X), devI));
+        return t;
+    }
+    template <PairKind KIND>
+    __device__ __forceinline__ void finish(const Neighbours &N, const Taken &taken)
+    {
+        const float *volume = taken.volume;
         if (wantL) {
-            double dd[3] = {(double)d[0], (double)d[1], (double)d[2]}, r2 = 0.0;
-            for (int a = 0; a < D; ++a) r2 = fma(dd[a], dd[a], r2);
-            const double rf = (double)r, rr = fma(fma(-rf, rf, r2), 0.5 / rf, rf);
-            const double w64 = (double)volumeIn<D>(B, X) * kernelGradient64<K>(rr, k);
-            for (int a = 0; a < D; ++a) {
-                const double wa = -w64 * dd[a];
-                for (int b = a; b < D; ++b) M[packed<D>(a, b)] = fma(wa, dd[b], M[packed<D>(a, b)]);
+            for (int q = 0; q < 2; ++q) {
+                if (!N.live[q]) continue;
+                double dd[3], r2 = 0.0;
+                for (int a = 0; a < D; ++a) {
+                    dd[a] = (double)(q ? N.d[a].y : N.d[a].x);
+                    r2 = fma(dd[a], dd[a], r2);
+                }
+                // the root by one Newton step from float32's: r + (r2 - r^2) / (2 r), the small correction's
+                // divisor in float32
+                const double rf = (double)(q ? N.r.y : N.r.x);
+                const double rr = fma(fma(-rf, rf, r2), (double)(0.5f * (q ? N.inverse.y : N.inverse.x)), rf);
+                const double w64 = (double)volume[q] * kernelGradient64<K>(rr, N.k.of(q));
+                for (int a = 0; a < D; ++a) {
+                    const double wa = -w64 * dd[a];
+                    for (int b = a; b < D; ++b) M[packed<D>(a, b)] = fma(wa, dd[b], M[packed<D>(a, b)]);
+                }
             }
         }
-        float w = volumeIn<D>(B, X) * kernelGradient<K>(r * k.invH, k);
-        if (wantG && fluidJ) {
-            float vj[3];
-            velocityIn<D>(Kj, vj);
+        const float2 grad = kernelGradient<K>(mul2(N.r, N.k.invH), N.k);
+        const float2 w = make_float2(N.live[0] ? __fmul_rn(volume[0], grad.x) : 0.0f,
+                                     N.live[1] ? __fmul_rn(volume[1], grad.y) : 0.0f);
+        if (KIND == kFluidPair && wantG) {
             for (int a = 0; a < D; ++a) {
-                for (int b = 0; b < D; ++b) S[a][b] += w * (vj[a] - vi[a]) * d[b];
-                const float wa = -w * d[a];
-                for (int b = a; b < D; ++b) Mf[packed<D>(a, b)] += wa * d[b];
+                const float2 wv = mul2(w, taken.rel[a]);
+                for (int b = 0; b < D; ++b) jump[a][b] = fma2(wv, N.d[b], jump[a][b]);
+                const float2 wa = mul2(w, N.d[a]);     // minus M's weight; the sign comes off at the end
+                for (int b = a; b < D; ++b) Mf[packed<D>(a, b)] = fma2(wa, N.d[b], Mf[packed<D>(a, b)]);
             }
         }
         if (wantRho) {
-            float t = w * (deviationIn<D>(B, X) - devI);
-            for (int a = 0; a < D; ++a) gsum[a] += t * d[a];
+            const float2 t = mul2(w, taken.difference);
+            for (int a = 0; a < D; ++a) gsum[a] = fma2(t, N.d[a], gsum[a]);
         }
     }
 };
 
-template <int D, int T>
-__device__ __forceinline__ void groupSumMatrix(float M[3][3], unsigned mask)
+// A lane's two halves and then the group's sum.
+template <int T>
+__device__ __forceinline__ float groupSum(const float2 &value, unsigned mask)
 {
-    for (int a = 0; a < D; ++a)
-        for (int b = 0; b < D; ++b) M[a][b] = groupSum<T>(M[a][b], mask);
+    return groupSum<T>(__fadd_rn(value.x, value.y), mask);
 }
 
 template <int D, int K, int T, bool FINE>
@@ -612,32 +665,35 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
         if (G.t != 0) return;
         float zero[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
         float ident[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
-        if (wantG) storeMatrix<D>(F.G0, F.G1, F.G2, i, zero);
+        if (wantG == kWholeGradients) storeMatrix<D>(F.G0, F.G1, F.G2, i, zero);
         if (wantL) storeMatrix<D>(F.L0, F.L1, F.L2, i, ident);
         if (wantRho) F.gradRho[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
-    GradientVisit<D, K, FINE> visit{F, Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || wantRho != 0, wantRho != 0};
+    GradientVisit<D, K, FINE> visit{Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || wantRho != 0, wantRho != 0};
     velocityOf<D>(F, i, visit.vi);
     visit.devI = deviationOf<D>(F, i);
-    for (int a = 0; a < 3; ++a) {
-        visit.gsum[a] = 0.0f;
-        for (int b = 0; b < 3; ++b) visit.S[a][b] = 0.0f;
+    for (int a = 0; a < D; ++a) {
+        visit.gsum[a] = both(0.0f);
+        for (int b = 0; b < D; ++b) visit.jump[a][b] = both(0.0f);
     }
-    for (int q = 0; q < D * (D + 1) / 2; ++q) { visit.M[q] = 0.0; visit.Mf[q] = 0.0f; }
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, visit);
-    float Mf[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+    for (int q = 0; q < D * (D + 1) / 2; ++q) { visit.M[q] = 0.0; visit.Mf[q] = both(0.0f); }
+    const Row row = openRow<D, FINE>(P, F, i, G.t, hs);
+    sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, visit);
+    if (visit.wantL) sumPairs<D, T, FINE, kWallPair>(P, F, row, false, visit);
+    float Mf[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, jump[3][3] = {}, gsum[3] = {};
     if (wantG) {
-        groupSumMatrix<D, T>(visit.S, G.mask);
-        for (int a = 0; a < D; ++a)
-            for (int b = a; b < D; ++b) Mf[a][b] = Mf[b][a] = groupSum<T>(visit.Mf[packed<D>(a, b)], G.mask);
+        for (int a = 0; a < D; ++a) {
+            for (int b = 0; b < D; ++b) jump[a][b] = groupSum<T>(visit.jump[a][b], G.mask);
+            for (int b = a; b < D; ++b) Mf[a][b] = Mf[b][a] = -groupSum<T>(visit.Mf[packed<D>(a, b)], G.mask);
+        }
     }
     double M[3][3] = {{1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
     if (wantL || wantRho)
         for (int a = 0; a < D; ++a)
             for (int b = a; b < D; ++b) M[a][b] = M[b][a] = groupSum<T>(visit.M[packed<D>(a, b)], G.mask);
     if (wantRho)
-        for (int a = 0; a < D; ++a) visit.gsum[a] = groupSum<T>(visit.gsum[a], G.mask);
+        for (int a = 0; a < D; ++a) gsum[a] = groupSum<T>(visit.gsum[a], G.mask);
     if (G.t != 0) return;
     if (wantG) {
         float Gm[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -647,11 +703,13 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
             for (int a = 0; a < D; ++a)
                 for (int b = 0; b < D; ++b) {
                     float t = 0.0f;
-                    for (int c = 0; c < D; ++c) t += visit.S[a][c] * inv[c][b];
+                    for (int c = 0; c < D; ++c) t += jump[a][c] * inv[c][b];
                     Gm[a][b] = t;
                 }
         }
-        storeMatrix<D>(F.G0, F.G1, F.G2, i, Gm);
+        // the steps read the symmetric part alone; the whole matrix goes to the caller who asks for it
+        if (wantG == kWholeGradients) storeMatrix<D>(F.G0, F.G1, F.G2, i, Gm);
+        else storeSlopes<D>(F, i, Gm);
     }
     if (wantL || wantRho) {
         // L = M^-1 in float64, rounded once
@@ -666,7 +724,7 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
         if (wantRho) {
             float g[3] = {0.0f, 0.0f, 0.0f};
             for (int a = 0; a < D; ++a)
-                for (int b = 0; b < D; ++b) g[a] += L[a][b] * visit.gsum[b];
+                for (int b = 0; b < D; ++b) g[a] += L[a][b] * gsum[b];
             F.gradRho[i] = make_float4(g[0], g[1], g[2], 0.0f);
         }
     }
@@ -679,138 +737,142 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
 // BUDGET: the sum split for the energy budget too, into the pressure and the viscosity of fluid
 // and of boundary neighbours (src/pysurf/sphGpu.py:400-414).  COMP: the sum compensated (Dot2),
 // its running error in comp.
-template <int D, int K, bool BUDGET, bool COMP = false>
+template <int D, int K, bool BUDGET, bool FINE, bool COMP = false>
 struct MomentumVisit {
+    static constexpr bool kCopied = D == 2 || FINE;
+    static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kPipelined = true;
     static constexpr bool kAuxRow = D == 3;
     static constexpr bool kKinetic = true;
     const Params &P; const Frame &F;
-    Smoothing<K, D> S;
+    Smoothing<K, D, FINE> S;
     float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0
     float alphaI;                               // closure: this particle's eddy alpha
-    float slopeI[D * (D + 1) / 2];              // r . G_i r's coefficients: G_aa, and G_ab + G_ba (a < b)
-    float total[3];
-    float comp[COMP ? 3 : 1];
+    float slopeI[6];                            // r . G_i r's coefficients (Frame::S0, S1)
+    float2 total[D];                            // minus the sum, over the lane's even and odd neighbours
+    float2 comp[COMP ? D : 1];
     float parts[BUDGET ? 4 : 1][3];
-    float4 rowX;
-    __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *d, float r, float h, bool fluidJ, int, const float4 &B,
-                               const float4 &Kj)
+    struct Taken {
+        float2 plain;               // (v_i - v_j) . r
+        float2 density, pressure;   // rho_i + rho_j, p_i / rho_i^2 + p_j / rho_j^2
+        float mass[2], rho[2];
+        float s0[6], s1[6];         // the approaching neighbours' slopes' coefficients
+    };
+    template <PairKind KIND>
+    __device__ __forceinline__ Taken take(const Neighbours &N, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
-        const KernelAt k = S.at(h);
-        const float q = r * k.invH;
-        float vj[3];
-        velocityIn<D>(Kj, vj);
-        float rel[3] = {vi[0] - vj[0], vi[1] - vj[1], vi[2] - vj[2]};
-        float approach = rel[0] * d[0] + rel[1] * d[1] + (D == 3 ? rel[2] * d[2] : 0.0f);
-        const float plain = approach;           // before the limiter reconstructs it
-        float viscosity = 0.0f;
-        if (approach < 0.0f && P.limited && fluidJ) {
-            // the slopes r . G r along the pair, each a quadratic form in r: only G's symmetric part
-            // enters, so r's products d_a d_b (a <= b) serve both particles
-            float Gj[3][3];
-            loadMatrix<D>(F.G0, F.G1, F.G2, j, Gj);
-            float slopeIJ = 0.0f, slopeJ = 0.0f;
-            for (int a = 0; a < D; ++a)
-                for (int b = a; b < D; ++b) {
-                    const float dd = d[a] * d[b], gj = a == b ? Gj[a][a] : Gj[a][b] + Gj[b][a];
-                    slopeIJ += slopeI[packed<D>(a, b)] * dd;
-                    slopeJ += gj * dd;
-                }
-            float limiter = 0.0f;
-            if (slopeIJ * slopeJ > 0.0f) {
+        Taken t;
+        float vj0[3], vj1[3];
+        velocityIn<D>(R0.K, vj0);
+        velocityIn<D>(R1.K, vj1);
+        for (int a = 0; a < D; ++a) {
+            const float2 rel = make_float2(__fsub_rn(vi[a], vj0[a]), __fsub_rn(vi[a], vj1[a]));
+            t.plain = a == 0 ? mul2(rel, N.d[0]) : fma2(rel, N.d[a], t.plain);
+        }
+        for (int c = 0; c < 6; ++c) t.s0[c] = t.s1[c] = 0.0f;
+        if (KIND == kFluidPair && P.limited) {
+            if (t.plain.x < 0.0f) loadSlopes<D>(F, N.j[0], t.s0);
+            if (t.plain.y < 0.0f) loadSlopes<D>(F, N.j[1], t.s1);
+        }
+        t.rho[0] = densityIn<D>(R0.K);
+        t.rho[1] = densityIn<D>(R1.K);
+        t.density = make_float2(__fadd_rn(rhoI, t.rho[0]), __fadd_rn(rhoI, t.rho[1]));
+        t.pressure = make_float2(__fadd_rn(own, pressureRatioIn<D>(R0.K, R0.X)),
+                                 __fadd_rn(own, pressureRatioIn<D>(R1.K, R1.X)));
+        t.mass[0] = massIn<D>(R0.B);
+        t.mass[1] = massIn<D>(R1.B);
+        return t;
+    }
+    template <PairKind KIND>
+    __device__ __forceinline__ void finish(const Neighbours &N, const Taken &taken)
+    {
+        const float2 q = mul2(N.r, N.k.invH), grad = kernelGradient<K>(q, N.k);
+        const float2 plain = taken.plain;
+        const float *s0 = taken.s0, *s1 = taken.s1;
+        float2 approach = plain;
+        if (KIND == kFluidPair && P.limited) {
+            const bool limit0 = plain.x < 0.0f, limit1 = plain.y < 0.0f;
+            if (limit0 || limit1) {
+                // the slopes r . G r along the pair, each a quadratic form in r: only G's symmetric part
+                // enters, so r's products d_a d_b (a <= b) serve both particles
+                float2 slopeI2 = both(0.0f), slopeJ = both(0.0f);
+                for (int a = 0; a < D; ++a)
+                    for (int b = a; b < D; ++b) {
+                        const int c = packed<D>(a, b);
+                        const float2 dd = mul2(N.d[a], N.d[b]);
+                        slopeI2 = fma2(both(slopeI[c]), dd, slopeI2);
+                        slopeJ = make_float2(__fmaf_rn(s0[c], dd.x, slopeJ.x), __fmaf_rn(s1[c], dd.y, slopeJ.y));
+                    }
                 // 4 R / (1 + R)^2 at R = slopeI / slopeJ, as 4 slopeI slopeJ / (slopeI + slopeJ)^2
-                const float sum = slopeIJ + slopeJ;
-                // the fast division (2 ulp) takes 8% off the momentum sweep; its range limit (a
-                // denominator past 2^126) lies far beyond any pair's slopes
-                limiter = fminf(1.0f, __fdividef(4.0f * slopeIJ * slopeJ, sum * sum));
-                if (q < kCloseDistance) {
-                    float fade = (q - kCloseDistance) * (1.0f / kFoldWidth);
-                    limiter *= expf(-fade * fade);
+                const float2 sum = add2(slopeI2, slopeJ), product = mul2(slopeI2, slopeJ);
+                const float2 four = mul2(both(4.0f), product), square = mul2(sum, sum);
+                // the fast division takes 8% off the momentum sweep; its range limit (a denominator
+                // past 2^126) lies far beyond any pair's slopes
+                float2 limiter = make_float2(product.x > 0.0f ? fminf(1.0f, quickDivide(four.x, square.x)) : 0.0f,
+                                             product.y > 0.0f ? fminf(1.0f, quickDivide(four.y, square.y)) : 0.0f);
+                if (q.x < kCloseDistance || q.y < kCloseDistance) {
+                    const float fade0 = (q.x - kCloseDistance) * (1.0f / kFoldWidth);
+                    const float fade1 = (q.y - kCloseDistance) * (1.0f / kFoldWidth);
+                    if (q.x < kCloseDistance) limiter.x = __fmul_rn(limiter.x, expf(-__fmul_rn(fade0, fade0)));
+                    if (q.y < kCloseDistance) limiter.y = __fmul_rn(limiter.y, expf(-__fmul_rn(fade1, fade1)));
                 }
+                // (v_ij - (phi / 2) (G_i + G_j) r) . r = v_ij . r - (phi / 2) (r . G_i r + r . G_j r)
+                const float2 limited = fma2(mul2(both(-0.5f), limiter), sum, plain);
+                if (limit0) approach.x = limited.x;
+                if (limit1) approach.y = limited.y;
             }
-            // (v_ij - (phi / 2) (G_i + G_j) r) . r = v_ij . r - (phi / 2) (r . G_i r + r . G_j r)
-            approach = plain - 0.5f * limiter * (slopeIJ + slopeJ);
         }
-        if (approach < 0.0f) {
-            // -alpha c0 h (v_ij . r_ij) / ((r^2 + 0.01 h^2) (rho_i + rho_j) / 2); the denominator is
-            // a positive normal float for any physical pair, which __fdividef takes to 2 ulp
-            viscosity = __fdividef(viscosityScale * h * approach,
-                                   (r * r + k.soft) * (0.5f * (rhoI + densityIn<D>(Kj))));
-            if (!fluidJ) viscosity *= P.boundaryFactor;
+        // -alpha c0 h (v_ij . r_ij) / ((r^2 + 0.01 h^2) (rho_i + rho_j) / 2) where the pair approaches; the
+        // denominator is a positive normal float for any physical pair
+        const float2 closing = make_float2(fminf(approach.x, 0.0f), fminf(approach.y, 0.0f));
+        const float2 above = mul2(mul2(both(viscosityScale), N.h), closing);
+        const float2 mean = mul2(both(0.5f), taken.density);
+        const float2 below = mul2(fma2(N.r, N.r, N.k.soft), mean);
+        float2 viscosity = make_float2(quickDivide(above.x, below.x), quickDivide(above.y, below.y));
+        if (KIND == kWallPair) viscosity = mul2(viscosity, both(P.boundaryFactor));
+        if (KIND == kFluidPair && P.closure) {
+            if (N.live[0])
+                viscosity.x = __fadd_rn(viscosity.x, closureTerm(N.j[0], N.h.x, N.r.x, plain.x, taken.rho[0]));
+            if (N.live[1])
+                viscosity.y = __fadd_rn(viscosity.y, closureTerm(N.j[1], N.h.y, N.r.y, plain.y, taken.rho[1]));
         }
-        if (P.closure && fluidJ) {
-            // delta-LES-SPH: -(K nu / (c0 h) + harmonic mean of the alphas) c0 h rho0 (v_ij . r_ij) /
-            // (r^2 rho_i rho_j) on every fluid pair, approaching or not (src/pysurf/sphGpu.py:388-396)
-            const float alphaJ = __ldg(&F.eddy[j].x), both = alphaI + alphaJ;
-            const float mean = both > 0.0f ? 2.0f * alphaI * alphaJ / both : 0.0f;
-            viscosity += -(P.waterTerm / h + mean) * P.c0 * h * P.closureRho0 * plain
-                       / (r * r * rhoI * densityIn<D>(Kj));
-        }
-        const float ratioJ = D == 2 ? Kj.w : rowX.x;
-        // explicit roundings on the sum's path, so the budget's extra uses of its terms cannot
-        // change how the compiler fuses them: the tracked step is the plain step, bit for bit
-        const float pressureTerm = __fadd_rn(own, ratioJ);
-        float coefficient = -__fadd_rn(pressureTerm, viscosity) * massIn<D>(B);
-        float f = coefficient * kernelGradient<K>(q, k);
+        const float2 pressure = taken.pressure, stress = add2(pressure, viscosity);
+        const float m0 = taken.mass[0], m1 = taken.mass[1];
+        const float2 f = mul2(make_float2(N.live[0] ? __fmul_rn(stress.x, m0) : 0.0f,
+                                          N.live[1] ? __fmul_rn(stress.y, m1) : 0.0f), grad);
         if constexpr (COMP) {
-            for (int a = 0; a < D; ++a) addProduct(f, d[a], total[a], comp[a]);
+            for (int a = 0; a < D; ++a) {
+                addProduct(f.x, N.d[a].x, total[a].x, comp[a].x);
+                addProduct(f.y, N.d[a].y, total[a].y, comp[a].y);
+            }
         } else {
-            for (int a = 0; a < D; ++a) total[a] = __fmaf_rn(f, d[a], total[a]);
+            for (int a = 0; a < D; ++a) total[a] = fma2(f, N.d[a], total[a]);
         }
         if constexpr (BUDGET) {
-            const float grad = massIn<D>(B) * kernelGradient<K>(q, k);
-            const float fp = -pressureTerm * grad, fv = -viscosity * grad;
-            if (fluidJ) {
-                for (int a = 0; a < D; ++a) { parts[0][a] += fp * d[a]; parts[1][a] += fv * d[a]; }
-            } else {
-                for (int a = 0; a < D; ++a) { parts[2][a] += fp * d[a]; parts[3][a] += fv * d[a]; }
+            for (int s = 0; s < 2; ++s) {
+                if (!N.live[s]) continue;
+                const float weight = __fmul_rn(s ? m1 : m0, s ? grad.y : grad.x);
+                const float fp = -__fmul_rn(s ? pressure.y : pressure.x, weight);
+                const float fv = -__fmul_rn(s ? viscosity.y : viscosity.x, weight);
+                constexpr int side = KIND == kFluidPair ? 0 : 2;
+                for (int a = 0; a < D; ++a) {
+                    const float d = s ? N.d[a].y : N.d[a].x;
+                    parts[BUDGET ? side : 0][a] = __fmaf_rn(fp, d, parts[BUDGET ? side : 0][a]);
+                    parts[BUDGET ? side + 1 : 0][a] = __fmaf_rn(fv, d, parts[BUDGET ? side + 1 : 0][a]);
+                }
             }
         }
     }
-};
-
-__device__ __forceinline__ double cflTimeStep(double h, double c0, double vmax, double amax, double cfl, double maxdt)
-{
-    double dt = cfl * h / (c0 + vmax);
-    if (amax > 1e-12) dt = fmin(dt, cfl * sqrt(h / amax));
-    return fmin(dt, maxdt);
-}
-
-__device__ __forceinline__ double warpMax(double value)
-{
-    for (int offset = 16; offset > 0; offset >>= 1) value = fmax(value, __shfl_xor_sync(0xFFFFFFFFu, value, offset));
-    return value;
-}
-
-// The step's fluid maxima without a block barrier: each warp folds its lanes' values and lane 0
-// raises the running maxima (atomicMax on the bits of non-negative doubles, which is order-free);
-// the last warp to finish takes the time step in float64 and clears the running values.
-__device__ __forceinline__ void foldMaxima(Control *ctl, double speed, double accel, int warps)
-{
-    // non-negative, and a NaN counts as 0 as fmax would take it
-    speed = warpMax(speed > 0.0 ? speed : 0.0);
-    accel = warpMax(accel > 0.0 ? accel : 0.0);
-    if ((threadIdx.x & 31) != 0) return;
-    atomicMax(&ctl->vmaxBits, (unsigned long long)__double_as_longlong(speed));
-    atomicMax(&ctl->amaxBits, (unsigned long long)__double_as_longlong(accel));
-    __threadfence();
-    if (atomicAdd(&ctl->ticket, 1u) != (unsigned)(warps - 1)) return;
-    __threadfence();
-    const double vmax = __longlong_as_double((long long)atomicMax(&ctl->vmaxBits, 0ull));
-    const double amax = __longlong_as_double((long long)atomicMax(&ctl->amaxBits, 0ull));
-    ctl->vmax = vmax;
-    ctl->amax = amax;
-    ctl->vmaxBits = 0;
-    ctl->amaxBits = 0;
-    ctl->ticket = 0;
-    if (!ctl->hostDt) {
-        const double dt = cflTimeStep(ctl->hMin, ctl->soundSpeed, vmax, amax, ctl->cfl, ctl->maxTimeStep);
-        if (!(dt > 0.0) || !isfinite(dt)) ctl->error |= kErrTimeStep;
-        ctl->dt = dt;
+    // delta-LES-SPH: -(K nu / (c0 h) + harmonic mean of the alphas) c0 h rho0 (v_ij . r_ij) /
+    // (r^2 rho_i rho_j) on every fluid pair, approaching or not (src/pysurf/sphGpu.py:388-396)
+    __device__ __forceinline__ float closureTerm(int j, float h, float r, float plain, float rhoJ) const
+    {
+        const float alphaJ = __ldg(&F.eddy[j].x), sum = __fadd_rn(alphaI, alphaJ);
+        const float mean = sum > 0.0f ? __fdiv_rn(__fmul_rn(__fmul_rn(2.0f, alphaI), alphaJ), sum) : 0.0f;
+        const float scale = __fmul_rn(__fmul_rn(__fmul_rn(__fadd_rn(__fdiv_rn(P.waterTerm, h), mean), P.c0), h), P.closureRho0);
+        return __fdiv_rn(-__fmul_rn(scale, plain), __fmul_rn(__fmul_rn(__fmul_rn(r, r), rhoI), rhoJ));
     }
-}
+};
 
 // maxima: fold the fluid maxima into ctl and take the time step (the device steps); 0 for the
 // host-step sums.
@@ -827,27 +889,24 @@ momentumKernel(Params P, Frame F, Control *ctl, int maxima)
         if (hs <= 0.0f) {
             if (G.t == 0) F.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         } else {
-            MomentumVisit<D, K, BUDGET, COMP> visit{P, F, Smoothing<K, D>(P)};
+            MomentumVisit<D, K, BUDGET, FINE, COMP> visit{P, F, Smoothing<K, D, FINE>(P, hs)};
             velocityOf<D>(F, i, visit.vi);
             visit.rhoI = densityOf<D>(F, i);
             visit.own = pressureRatioOf<D>(F, i);
             visit.viscosityScale = -P.alpha * P.c0;
             visit.alphaI = P.closure ? F.eddy[i].x : 0.0f;
-            if (P.limited) {
-                float Gi[3][3];
-                loadMatrix<D>(F.G0, F.G1, F.G2, i, Gi);
-                for (int a = 0; a < D; ++a)
-                    for (int b = a; b < D; ++b) visit.slopeI[packed<D>(a, b)] = a == b ? Gi[a][a] : Gi[a][b] + Gi[b][a];
-            }
-            visit.total[0] = visit.total[1] = visit.total[2] = 0.0f;
-            if constexpr (COMP) for (int a = 0; a < 3; ++a) visit.comp[a] = 0.0f;
+            if (P.limited) loadSlopes<D>(F, i, visit.slopeI);
+            for (int a = 0; a < D; ++a) visit.total[a] = both(0.0f);
+            if constexpr (COMP) for (int a = 0; a < D; ++a) visit.comp[a] = both(0.0f);
             if constexpr (BUDGET)
                 for (int q = 0; q < 4; ++q) visit.parts[q][0] = visit.parts[q][1] = visit.parts[q][2] = 0.0f;
-            forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, visit);
-            if constexpr (COMP) {
-                for (int a = 0; a < D; ++a) visit.total[a] = groupSumCompensated<T>(visit.total[a], visit.comp[a], G.mask);
-            } else {
-                for (int a = 0; a < D; ++a) visit.total[a] = groupSum<T>(visit.total[a], G.mask);
+            const Row row = openRow<D, FINE>(P, F, i, G.t, hs);
+            sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, visit);
+            sumPairs<D, T, FINE, kWallPair>(P, F, row, false, visit);
+            float total[3] = {0.0f, 0.0f, 0.0f};
+            for (int a = 0; a < D; ++a) {
+                if constexpr (COMP) total[a] = -groupSumCompensated<T>(visit.total[a], visit.comp[a], G.mask);
+                else total[a] = -groupSum<T>(visit.total[a], G.mask);
             }
             if constexpr (BUDGET) {
                 for (int q = 0; q < 4; ++q) {
@@ -858,13 +917,7 @@ momentumKernel(Params P, Frame F, Control *ctl, int maxima)
                 }
             }
             if (G.t == 0) {
-                float a[3] = {visit.total[0] + P.g[0], visit.total[1] + P.g[1],
-                              D == 3 ? visit.total[2] + P.g[2] : 0.0f};
-                F.acc[i] = make_float4(a[0], a[1], a[2], 0.0f);
-                double v2 = 0.0;
-                for (int c = 0; c < D; ++c) v2 += F.v[c][i] * F.v[c][i];
-                speed = sqrt(v2);
-                accel = (double)sqrtf(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
+                takeAcceleration<D>(P, F, i, total, speed, accel);
             }
         }
     }
@@ -886,12 +939,12 @@ __global__ void closureKernel(Params P, Frame F, const Control *ctl)
         F.eddy[i] = make_float2(0.0f, 0.0f);
         return;
     }
-    float G[3][3];
-    loadMatrix<D>(F.G0, F.G1, F.G2, i, G);
+    float slopes[6];
+    loadSlopes<D>(F, i, slopes);
     float sum = 0.0f;
     for (int a = 0; a < D; ++a)
         for (int b = 0; b < D; ++b) {
-            const float e = 0.5f * (G[a][b] + G[b][a]);
+            const float e = a == b ? slopes[packed<D>(a, a)] : 0.5f * slopes[packed<D>(min(a, b), max(a, b))];
             sum += e * e;
         }
     const float scale = hs * sqrtf(2.0f * sum) / P.closureC0;
@@ -938,31 +991,6 @@ __global__ void kickKernel(Params P, Frame F, Control *ctl)
     F.low[i] = low;
 }
 
-// Drift (src/pysurf/sphGpu.py:1142-1186), the periodic wrap and the enforcement of one fluid slot.
-template <int D>
-__device__ __forceinline__ void driftAndEnforce(const Params &P, const Frame &F, const Enforcement &E, int i, double dt,
-                                                const double *transport, Control *ctl)
-{
-    double x[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, lift = 0.0;
-    for (int a = 0; a < D; ++a) {
-        v[a] = F.v[a][i];
-        const double start = F.x[a][i];
-        x[a] = start + (transport ? transport[a] : v[a]) * dt;
-        lift += P.gravity64[a] * (x[a] - start);
-    }
-    // the drift's change of potential energy, from the displacement as stored (src/pysurf/sphGpu.py:1168-1170)
-    if (P.budget) addEnergy(P, F, i, kDrift, -F.m[i] * lift);
-    if (P.period > 0.0) x[1] = x[1] - P.period * floor(x[1] / P.period);
-    enforceTracked(P, F, E, D, i, x, v);
-    bool finite = true;
-    for (int a = 0; a < D; ++a) {
-        F.x[a][i] = x[a];
-        F.v[a][i] = v[a];
-        finite = finite && isfinite(x[a]) && isfinite(v[a]);
-    }
-    if (!finite) atomicOr(&ctl->error, kErrNonFinite);
-}
-
 // ------------------------------------------------------------------------------------------
 // Sweep D: continuity with the density update, drift and enforcement
 // ------------------------------------------------------------------------------------------
@@ -978,144 +1006,187 @@ __device__ __forceinline__ void driftAndEnforce(const Params &P, const Frame &F,
 // and a boundary particle -- every pair of a boundary row, the wall's pairs of a fluid row -- take
 // their separation, distance, kernel gradient and term in float64, summed apart in float64 (cross).
 // Fluid pairs, whose velocity differences are small, keep float32 arithmetic.
-template <int D, int K, bool BUDGET, bool COMP = false>
+template <int D, int K, bool BUDGET, bool FINE, bool COMP = false>
 struct ContinuityVisit {
+    static constexpr bool kCopied = false;
+    static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kPipelined = true;
     static constexpr bool kAuxRow = D == 3;
     static constexpr bool kLowRow = true;
     static constexpr bool kKinetic = true;
-    static constexpr bool kBoundaryRows = true;         // every row
     const Params &P; const Frame &F;
-    Smoothing<K, D> S;
-    int self;               // this particle's slot
-    bool boundaryI, diffuses, corrected;
+    Smoothing<K, D, FINE> S;
+    bool diffuses, corrected;
     float vi[3], vlI[3], devI, devLoI, Li[3][3], gi[3];
     float deltaI;           // closure: this particle's eddy delta
-    float total, comp;
-    double cross;           // the fluid-boundary pairs' terms in float64
-    float plainFluid, plainWall, continuity, diffusive;     // BUDGET
-    float4 rowX, rowLow;
-    __device__ bool accept(bool fluidJ) const { return !(boundaryI && !fluidJ); }
-    __device__ void operator()(int j, const float *d, float r, float h, bool fluidJ, int image, const float4 &B,
-                               const float4 &Kj)
+    float2 total, comp;     // over the lane's even and odd neighbours
+    double x[D], v[D];      // the particle's position and velocity in float64
+    // the fluid-boundary pairs' sums in float64: m (dW/dr) / r (v_i - v_j)_a (x_i - x_j)_b where L enters
+    // (cross[a D + b]), else its trace alone (cross[0])
+    double cross[D * D];
+    float plainFluid, continuity, diffusive;    // BUDGET: the fluid pairs' parts
+    struct Taken {
+        float2 dv[D];                       // v_i - v_j
+        float mass[2];
+        float2 volume, devJ, leading, remainder;    // V_j; rho_j - rho_i from the deviations and their remainders
+    };
+    // the fluid-boundary pairs': x_i - x_j and v_i - v_j in float64
+    struct CrossTaken {
+        double dd[2][D], dv[2][D];
+        float mass[2];
+    };
+    template <PairKind KIND>
+    __device__ __forceinline__ auto take(const Neighbours &N, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
-        const KernelAt k = S.at(h);
-        float vj[3];
-        velocityIn<D>(Kj, vj);
-        const float4 lowJ = rowLow;
-        const float vlJ[3] = {lowJ.x, lowJ.y, lowJ.z};
-        if (boundaryI == fluidJ) {
-            // a fluid-boundary pair, in float64: x_i - x_j from the points and remainders, the distance
-            // by one Newton step from the float32 root, (dW/dr) / r, (v_i - v_j) . L_i (x_i - x_j)
-            const float4 A = __ldg(&F.pa[j]);
-            float pi[3], li[3], pj[3], lj[3];
-            pointOf<D>(F, self, pi);
-            remainderOf<D>(F, self, li);
-            pointIn<D>(A, pj);
-            remainderIn<D>(A, B, lj);
-            double dd[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
-            for (int a = 0; a < D; ++a) {
-                dd[a] = ((double)pi[a] - (double)pj[a]) + ((double)li[a] - (double)lj[a]);
-                if (a == 1 && image) dd[a] += pi[1] < 0.5f * P.periodF ? P.period : -P.period;
-                r2 = fma(dd[a], dd[a], r2);
-            }
-            const double rf = (double)r, rr = fma(fma(-rf, rf, r2), 0.5 / rf, rf);
-            const double grad = kernelGradient64<K>(rr, k);
-            double dot = 0.0;
-            for (int a = 0; a < D; ++a) {
-                double ld = dd[a];
-                if (corrected) {
-                    ld = 0.0;
-                    for (int b = 0; b < D; ++b) ld = fma((double)Li[a][b], dd[b], ld);
+        float vj0[3], vj1[3];
+        velocityIn<D>(R0.K, vj0);
+        velocityIn<D>(R1.K, vj1);
+        const float vl0[3] = {R0.L.x, R0.L.y, R0.L.z}, vl1[3] = {R1.L.x, R1.L.y, R1.L.z};
+        if constexpr (KIND == kCrossPair) {
+            CrossTaken t;
+            for (int q = 0; q < 2; ++q) {
+                const NeighbourRows &R = q ? R1 : R0;
+                float pj[3], lj[3];
+                pointIn<D>(R.A, pj);
+                remainderIn<D>(R.A, R.B, lj);
+                for (int a = 0; a < D; ++a) {
+                    t.dd[q][a] = x[a] - ((double)pj[a] + (double)lj[a]);
+                    if (a == 1 && N.image[q]) t.dd[q][a] += x[1] < 0.5 * P.period ? P.period : -P.period;
+                    t.dv[q][a] = v[a] - ((double)(q ? vj1[a] : vj0[a]) + (double)(q ? vl1[a] : vl0[a]));
                 }
-                dot = fma(((double)vi[a] + (double)vlI[a]) - ((double)vj[a] + (double)vlJ[a]), ld, dot);
+                t.mass[q] = massIn<D>(R.B);
             }
-            const double term = (double)massIn<D>(B) * dot * grad;
-            cross += term;
-            if constexpr (BUDGET) {
-                double plainDot = dot;
-                if (corrected) {
-                    plainDot = 0.0;
-                    for (int a = 0; a < D; ++a)
-                        plainDot = fma(((double)vi[a] + (double)vlI[a]) - ((double)vj[a] + (double)vlJ[a]), dd[a], plainDot);
-                }
-                const float plain = (float)((double)massIn<D>(B) * plainDot * grad);
-                continuity = __fadd_rn(continuity, (float)term);
-                if (fluidJ) plainFluid += plain; else plainWall += plain;
-            }
-            return;     // a pair with a boundary member does not diffuse
-        }
-        const float grad = kernelGradient<K>(r * k.invH, k);    // (dW/dr) / r
-        float dv[3];
-        for (int a = 0; a < D; ++a)
-            dv[a] = __fadd_rn(__fsub_rn(vi[a], vj[a]), __fsub_rn(vlI[a], vlJ[a]));
-        float dot = 0.0f;
-        if (corrected) {
-            for (int a = 0; a < D; ++a) {
-                float ld = 0.0f;
-                for (int b = 0; b < D; ++b) ld += Li[a][b] * d[b];
-                dot += dv[a] * ld;
-            }
+            return t;
         } else {
-            for (int a = 0; a < D; ++a) dot += dv[a] * d[a];
-        }
-        // explicit roundings on the sum's path (see the momentum sweep)
-        const float massDot = massIn<D>(B) * dot;
-        if constexpr (COMP) addProduct(massDot, grad, total, comp);
-        else total = __fmaf_rn(massDot, grad, total);
-        if constexpr (BUDGET) {
-            float plainDot = dot;
-            if (corrected) {
-                plainDot = 0.0f;
-                for (int a = 0; a < D; ++a) plainDot += dv[a] * d[a];
-            }
-            const float plain = massIn<D>(B) * plainDot * grad;
-            continuity = __fmaf_rn(massDot, grad, continuity);
-            if (fluidJ) plainFluid += plain; else plainWall += plain;
-        }
-        if (diffuses && fluidJ) {
-            const float4 X = D == 3 ? rowX : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float devJ = deviationIn<D>(B, X);
+            Taken t;
+            for (int a = 0; a < D; ++a)
+                t.dv[a] = add2(make_float2(__fsub_rn(vi[a], vj0[a]), __fsub_rn(vi[a], vj1[a])),
+                               make_float2(__fsub_rn(vlI[a], vl0[a]), __fsub_rn(vlI[a], vl1[a])));
+            t.mass[0] = massIn<D>(R0.B);
+            t.mass[1] = massIn<D>(R1.B);
+            t.volume = make_float2(N.live[0] ? volumeIn<D>(R0.B, R0.X) : 0.0f, N.live[1] ? volumeIn<D>(R1.B, R1.X) : 0.0f);
+            t.devJ = make_float2(deviationIn<D>(R0.B, R0.X), deviationIn<D>(R1.B, R1.X));
             // rho_j - rho_i from the float32 deviations and their remainders, so it keeps float64's
             // digits (the leading difference is exact for neighbours' nearly equal deviations)
-            const float remainder = __fsub_rn(lowJ.w, devLoI);
-            float difference;
+            t.leading = make_float2(__fsub_rn(t.devJ.x, devI), __fsub_rn(t.devJ.y, devI));
+            t.remainder = make_float2(__fsub_rn(R0.L.w, devLoI), __fsub_rn(R1.L.w, devLoI));
+            return t;
+        }
+    }
+    __device__ __forceinline__ void finishCross(const Neighbours &N, const CrossTaken &taken)
+    {
+        if (N.live[0]) wallPair<0>(N, taken);
+        if (N.live[1]) wallPair<1>(N, taken);
+    }
+    template <PairKind KIND, class T>
+    __device__ __forceinline__ void finish(const Neighbours &N, const T &taken)
+    {
+        if constexpr (KIND == kCrossPair) finishCross(N, taken);
+        else finishFluid(N, taken);
+    }
+    __device__ __forceinline__ void finishFluid(const Neighbours &N, const Taken &taken)
+    {
+        const float2 grad = kernelGradient<K>(mul2(N.r, N.k.invH), N.k);    // (dW/dr) / r
+        const float2 *dv = taken.dv;
+        float2 dot = both(0.0f);
+        if (corrected) {
+            for (int a = 0; a < D; ++a) {
+                float2 ld = mul2(both(Li[a][0]), N.d[0]);
+                for (int b = 1; b < D; ++b) ld = fma2(both(Li[a][b]), N.d[b], ld);
+                dot = a == 0 ? mul2(dv[a], ld) : fma2(dv[a], ld, dot);
+            }
+        } else {
+            for (int a = 0; a < D; ++a) dot = a == 0 ? mul2(dv[a], N.d[a]) : fma2(dv[a], N.d[a], dot);
+        }
+        const bool live0 = N.live[0], live1 = N.live[1];
+        const float m0 = taken.mass[0], m1 = taken.mass[1];
+        const float2 massDot = make_float2(live0 ? __fmul_rn(m0, dot.x) : 0.0f, live1 ? __fmul_rn(m1, dot.y) : 0.0f);
+        add(massDot, grad);
+        if constexpr (BUDGET) {
+            float2 plainDot = dot;
+            if (corrected)
+                for (int a = 0; a < D; ++a) plainDot = a == 0 ? mul2(dv[a], N.d[a]) : fma2(dv[a], N.d[a], plainDot);
+            const float2 plain = mul2(plainDot, grad);
+            if (live0) plainFluid = __fmaf_rn(m0, plain.x, plainFluid);
+            if (live1) plainFluid = __fmaf_rn(m1, plain.y, plainFluid);
+            if (live0) continuity = __fmaf_rn(massDot.x, grad.x, continuity);
+            if (live1) continuity = __fmaf_rn(massDot.y, grad.y, continuity);
+        }
+        if (diffuses) {
+            const float2 devJ = taken.devJ, leading = taken.leading, remainder = taken.remainder;
+            float2 difference;
             if (P.diffusion == 2) {
                 // less the hydrostatic difference k dz (1 + e)^-5 (src/pysurf/sphSolver.py:718-735), with
                 // k = rho0 g / c0^2 and e the pair's mean deviation over rho0.  Near rest it cancels most
                 // of rho_j - rho_i, so it is taken in two parts: k dz off the leading difference in one
                 // fused rounding, then the small k dz e S / (1 + e)^5 back on, where
                 // S = 1 + (1 + e) + ... + (1 + e)^4 makes (1 + e)^5 - 1 = e S without cancelling.
-                const float e = __fmul_rn(__fadd_rn(devI, devJ), P.halfInvRho0);
-                const float ratio = __fadd_rn(1.0f, e), sq = __fmul_rn(ratio, ratio), fifth = __fmul_rn(__fmul_rn(sq, sq), ratio);
-                const float S = __fadd_rn(__fadd_rn(__fadd_rn(1.0f, ratio), __fadd_rn(sq, __fmul_rn(sq, ratio))),
-                                          __fmul_rn(sq, sq));
-                const float slope = __fmul_rn(P.hydrostaticSlope, d[D - 1]);
-                const float leading = __fmaf_rn(-P.hydrostaticSlope, d[D - 1], __fsub_rn(devJ, devI));
-                difference = __fadd_rn(__fadd_rn(leading, remainder), __fdividef(__fmul_rn(__fmul_rn(slope, e), S), fifth));
+                const float2 e = mul2(make_float2(__fadd_rn(devI, devJ.x), __fadd_rn(devI, devJ.y)), both(P.halfInvRho0));
+                const float2 one = both(1.0f), ratio = add2(one, e), sq = mul2(ratio, ratio), fourth = mul2(sq, sq);
+                const float2 fifth = mul2(fourth, ratio);
+                const float2 sum = add2(add2(add2(one, ratio), fma2(sq, ratio, sq)), fourth);
+                const float2 slope = mul2(both(P.hydrostaticSlope), N.d[D - 1]);
+                const float2 back = mul2(mul2(slope, e), sum);
+                difference = add2(add2(fma2(both(-P.hydrostaticSlope), N.d[D - 1], leading), remainder),
+                                  make_float2(quickDivide(back.x, fifth.x), quickDivide(back.y, fifth.y)));
             } else {
-                difference = __fadd_rn(__fsub_rn(devJ, devI), remainder);
+                difference = add2(leading, remainder);
             }
             if (P.diffusion == 3) {
-                float4 gj = __ldg(&F.gradRho[j]);
-                float gjv[3] = {gj.x, gj.y, gj.z};
-                float t = 0.0f;
-                for (int a = 0; a < D; ++a) t += (gi[a] + gjv[a]) * d[a];
-                difference += 0.5f * t;
+                const float4 g0 = __ldg(&F.gradRho[N.j[0]]), g1 = __ldg(&F.gradRho[N.j[1]]);
+                const float gj0[3] = {g0.x, g0.y, g0.z}, gj1[3] = {g1.x, g1.y, g1.z};
+                float2 t = both(0.0f);
+                for (int a = 0; a < D; ++a)
+                    t = fma2(make_float2(__fadd_rn(gi[a], gj0[a]), __fadd_rn(gi[a], gj1[a])), N.d[a], t);
+                difference = fma2(both(0.5f), t, difference);
             }
             // 2 delta c0 h V_j (difference) (-(dW/dr) r) / (r^2 + 0.01 h^2), with (dW/dr) r = grad r^2;
             // with the closure, 2 delta c0 is 2 c0 times the harmonic mean of the two deltas
-            float factor = P.diffusionFactor;
-            if (P.closure) {
-                const float deltaJ = __ldg(&F.eddy[j].y), both = deltaI + deltaJ;
-                factor = both > 0.0f ? 2.0f * P.closureC0 * (2.0f * deltaI * deltaJ / both) : 0.0f;
+            float2 factor = both(P.diffusionFactor);
+            if (P.closure) factor = make_float2(pairFactor(N.j[0]), pairFactor(N.j[1]));
+            const float2 volume = taken.volume;
+            const float2 r2 = mul2(N.r, N.r), below = add2(r2, N.k.soft);
+            const float2 head = mul2(mul2(mul2(mul2(factor, N.h), volume), difference), mul2(both(-1.0f), grad));
+            const float2 ratio = make_float2(quickDivide(r2.x, below.x), quickDivide(r2.y, below.y));
+            add(head, ratio);
+            if constexpr (BUDGET) diffusive = __fmaf_rn(head.y, ratio.y, __fmaf_rn(head.x, ratio.x, diffusive));
+        }
+    }
+    __device__ __forceinline__ void add(const float2 &a, const float2 &b)
+    {
+        if constexpr (COMP) {
+            addProduct(a.x, b.x, total.x, comp.x);
+            addProduct(a.y, b.y, total.y, comp.y);
+        } else {
+            total = fma2(a, b, total);
+        }
+    }
+    __device__ __forceinline__ float pairFactor(int j) const
+    {
+        const float deltaJ = __ldg(&F.eddy[j].y), sum = __fadd_rn(deltaI, deltaJ);
+        if (!(sum > 0.0f)) return 0.0f;
+        return __fmul_rn(__fmul_rn(2.0f, P.closureC0), __fdiv_rn(__fmul_rn(__fmul_rn(2.0f, deltaI), deltaJ), sum));
+    }
+    // A fluid-boundary pair, in float64: the distance by one Newton step from the float32 root (its small
+    // correction's divisor in float32), (dW/dr) / r.
+    template <int Q>
+    __device__ __forceinline__ void wallPair(const Neighbours &N, const CrossTaken &taken)
+    {
+        const double *dd = taken.dd[Q], *dv = taken.dv[Q];
+        double r2 = 0.0;
+        for (int a = 0; a < D; ++a) r2 = fma(dd[a], dd[a], r2);
+        const double rf = (double)(Q ? N.r.y : N.r.x);
+        const double rr = fma(fma(-rf, rf, r2), (double)(0.5f * (Q ? N.inverse.y : N.inverse.x)), rf);
+        const double weight = __dmul_rn((double)taken.mass[Q], kernelGradient64<K>(rr, N.k.of(Q)));
+        if (corrected) {
+            for (int a = 0; a < D; ++a) {
+                const double wv = __dmul_rn(weight, dv[a]);
+                for (int b = 0; b < D; ++b) cross[a * D + b] = fma(wv, dd[b], cross[a * D + b]);
             }
-            const float r2 = r * r;
-            const float head = factor * h * volumeIn<D>(B, X) * difference * (-grad), ratio = __fdividef(r2, r2 + k.soft);
-            if constexpr (COMP) addProduct(head, ratio, total, comp);
-            else total = __fmaf_rn(head, ratio, total);
-            if constexpr (BUDGET) diffusive = __fmaf_rn(head, ratio, diffusive);
+        } else {
+            double dot = __dmul_rn(dv[0], dd[0]);
+            for (int a = 1; a < D; ++a) dot = fma(dv[a], dd[a], dot);
+            cross[0] = fma(weight, dot, cross[0]);
         }
     }
 };
@@ -1130,16 +1201,14 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
     const int i = G.i;
     if (i >= P.n) return;
     float hs = signedLength<D>(F, i);
-    ContinuityVisit<D, K, BUDGET, COMP> visit{P, F, Smoothing<K, D>(P)};
-    visit.boundaryI = hs <= 0.0f;
-    visit.diffuses = P.diffusion != 0 && !visit.boundaryI;
-    visit.corrected = P.corrected && !visit.boundaryI;
+    ContinuityVisit<D, K, BUDGET, FINE, COMP> visit{P, F, Smoothing<K, D, FINE>(P, fabsf(hs))};
+    const bool boundary = hs <= 0.0f;
+    visit.diffuses = P.diffusion != 0 && !boundary;
+    visit.corrected = P.corrected && !boundary;
     velocityOf<D>(F, i, visit.vi);
     const float4 lowI = F.low[i];
     visit.vlI[0] = lowI.x; visit.vlI[1] = lowI.y; visit.vlI[2] = lowI.z;
     visit.devLoI = lowI.w;
-    visit.self = i;
-    visit.cross = 0.0;
     visit.devI = deviationOf<D>(F, i);
     visit.deltaI = P.closure && visit.diffuses ? F.eddy[i].y : 0.0f;
     if (visit.corrected) loadMatrix<D>(F.L0, F.L1, F.L2, i, visit.Li);
@@ -1148,22 +1217,38 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
         float4 g = F.gradRho[i];
         visit.gi[0] = g.x; visit.gi[1] = g.y; visit.gi[2] = g.z;
     }
-    visit.total = visit.comp = 0.0f;
-    visit.plainFluid = visit.plainWall = visit.continuity = visit.diffusive = 0.0f;
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, fabsf(hs), visit);
+    visit.total = visit.comp = both(0.0f);
+    visit.plainFluid = visit.continuity = visit.diffusive = 0.0f;
+    for (int q = 0; q < D * D; ++q) visit.cross[q] = 0.0;
+    const Row row = openRow<D, FINE>(P, F, i, G.t, fabsf(hs));
+    for (int a = 0; a < D; ++a) {
+        visit.x[a] = (double)row.pi[a] + (double)row.li[a];
+        visit.v[a] = (double)visit.vi[a] + (double)visit.vlI[a];
+    }
+    // the fluid pairs of a fluid row, then the fluid-boundary pairs of either
+    if (!boundary) sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, visit);
+    sumPairs<D, T, FINE, kCrossPair>(P, F, row, boundary, visit);
     float rate;
     if constexpr (COMP) rate = groupSumCompensated<T>(visit.total, visit.comp, G.mask);
     else rate = groupSum<T>(visit.total, G.mask);
+    double cross = visit.cross[0], plainCross = visit.cross[0];
+    if (visit.corrected) {
+        cross = plainCross = 0.0;
+        for (int a = 0; a < D; ++a) {
+            for (int b = 0; b < D; ++b) cross = fma((double)visit.Li[a][b], visit.cross[a * D + b], cross);
+            plainCross += visit.cross[a * D + a];
+        }
+    }
     // the fluid-boundary pairs' float64 sum joins before the one rounding to float32
-    rate = (float)((double)rate + groupSum<T>(visit.cross, G.mask));
+    cross = groupSum<T>(cross, G.mask);
+    rate = (float)((double)rate + cross);
     float parts[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if constexpr (BUDGET) {
-        const float plainFluid = groupSum<T>(visit.plainFluid, G.mask);
-        const float plainWall = groupSum<T>(visit.plainWall, G.mask);
-        const float continuity = groupSum<T>(visit.continuity, G.mask);
-        parts[0] = plainFluid;
-        parts[1] = plainWall;
-        parts[2] = visit.corrected ? continuity - plainFluid - plainWall : 0.0f;
+        // a fluid row's parts (a boundary row keeps none)
+        const float continuity = groupSum<T>(visit.continuity, G.mask) + (float)cross;
+        parts[0] = groupSum<T>(visit.plainFluid, G.mask);
+        parts[1] = (float)groupSum<T>(plainCross, G.mask);
+        parts[2] = visit.corrected ? continuity - parts[0] - parts[1] : 0.0f;
         parts[3] = groupSum<T>(visit.diffusive, G.mask);
     }
     if (G.t != 0) return;
@@ -1171,18 +1256,14 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
     if (mode == 0) return;
     double dt = ctl->dt;
     const double start = F.rho[i];
-    double rho = start + (double)rate * dt;
-    const double unfloored = rho;
-    bool fluid = hs > 0.0f;
-    if (P.densityFloor > 0.0 && fluid) rho = fmax(rho, P.densityFloor);
-    F.rho[i] = rho;
+    const bool fluid = hs > 0.0f;
+    const double unfloored = advanceDensity(P, F, i, rate, dt, fluid, ctl);
     if (BUDGET && fluid) {
         // each part of the rate over the secant slope of e, and the floor's change (src/pysurf/sphGpu.py:1111-1140)
         const double m = F.m[i], slope = elasticSlope(P, start, unfloored);
         for (int q = 0; q < 4; ++q) addEnergy(P, F, i, kContinuityFluid + q, m * slope * (double)parts[q] * dt);
-        addEnergy(P, F, i, kFloor, m * (elasticEnergy(P, rho) - elasticEnergy(P, unfloored)));
+        addEnergy(P, F, i, kFloor, m * (elasticEnergy(P, F.rho[i]) - elasticEnergy(P, unfloored)));
     }
-    if (!isfinite(rho)) atomicOr(&ctl->error, kErrNonFinite);
     if (mode == 2 && fluid) driftAndEnforce<D>(P, F, E, i, dt, nullptr, ctl);
 }
 
@@ -1190,23 +1271,22 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
 // Sweep X: XSPH over fluid pairs, with the densities the step has just advanced
 // ------------------------------------------------------------------------------------------
 
-template <int D, int K>
+template <int D, int K, bool FINE>
 struct XsphVisit {
+    static constexpr bool kCopied = false;
     static constexpr bool kSkipCoincident = false;
     static constexpr bool kKinetic = true;
-    const Frame &F; const float *densities;
-    Smoothing<K, D> S;
+    const float *densities;
+    Smoothing<K, D, FINE> S;
     float vi[3], rhoI, corr[3];
-    __device__ bool accept(bool fluidJ) const { return fluidJ; }
-    __device__ void operator()(int j, const float *, float r, float h, bool, int, const float4 &B, const float4 &Kj)
+    __device__ void operator()(int j, const float *, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
-        const KernelAt k = S.at(h);
-        float w = kernelValue<K>(r * k.invH, k);
-        float rhoJ = densities ? densities[j] : densityIn<D>(Kj);
-        float weight = massIn<D>(B) * w / (0.5f * (rhoI + rhoJ));
+        const float w = kernelValue<K>(__fmul_rn(r, k.invH), k);
+        const float rhoJ = densities ? densities[j] : densityIn<D>(R.K);
+        const float weight = __fdiv_rn(__fmul_rn(massIn<D>(R.B), w), __fmul_rn(0.5f, __fadd_rn(rhoI, rhoJ)));
         float vj[3];
-        velocityIn<D>(Kj, vj);
-        for (int a = 0; a < D; ++a) corr[a] += weight * (vj[a] - vi[a]);
+        velocityIn<D>(R.K, vj);
+        for (int a = 0; a < D; ++a) corr[a] = __fmaf_rn(weight, __fsub_rn(vj[a], vi[a]), corr[a]);
     }
 };
 
@@ -1227,11 +1307,11 @@ xsphKernel(Params P, Frame F, Control *ctl, Enforcement E, const float *densitie
         if (G.t == 0) F.vec[i] = make_float4(v[0], v[1], v[2], 0.0f);
         return;
     }
-    XsphVisit<D, K> visit{F, densities, Smoothing<K, D>(P)};
+    XsphVisit<D, K, FINE> visit{densities, Smoothing<K, D, FINE>(P, hs)};
     visit.vi[0] = v[0]; visit.vi[1] = v[1]; visit.vi[2] = v[2];
     visit.rhoI = densities ? densities[i] : densityOf<D>(F, i);
     visit.corr[0] = visit.corr[1] = visit.corr[2] = 0.0f;
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, visit);
+    sumPairs<D, T, FINE, kFluidPair>(P, F, openRow<D, FINE>(P, F, i, G.t, hs), true, visit);
     for (int a = 0; a < D; ++a) visit.corr[a] = groupSum<T>(visit.corr[a], G.mask);
     if (G.t != 0) return;
     float t[3];
@@ -1263,29 +1343,41 @@ __global__ void frameDensityKernel(Params P, Frame F, const Control *ctl)
 // grad C0, div r = -sum V_j r_ij . grad W_ij, grad rho from the deviations.
 template <int D, int K>
 struct ShiftFieldsVisit {
+    static constexpr bool kCopied = false;
+    static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
     static constexpr bool kKinetic = false;
-    const Params &P; const Frame &F;
-    Smoothing<K, D> S;
-    float devI, gradient[3], plain[3], densityGradient[3], total;
-    __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *d, float r, float h, bool, int, const float4 &B, const float4 &)
+    static constexpr bool kAuxRow = D == 3;
+    const Params &P;
+    Smoothing<K, D, false> S;
+    float devI;
+    float2 gradient[D], plain[D], densityGradient[D], total;    // over the lane's even and odd neighbours
+    struct Taken {
+        float volume[2];
+        float2 difference;
+    };
+    template <PairKind KIND>
+    __device__ __forceinline__ Taken take(const Neighbours &, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
-        const KernelAt k = S.at(h);
-        const float q = r * k.invH;
-        const float4 X = auxRow<D>(F, j);
-        const float volume = volumeIn<D>(B, X);
-        const float grad = kernelGradient<K>(q, k);         // (dW/dr) / r
-        const float ratio = kernelValue<K>(q, k) / P.spacingKernel, square = ratio * ratio;
-        const float weight = 1.0f + 0.2f * square * square;
-        const float difference = deviationIn<D>(B, X) - devI;
+        return Taken{{volumeIn<D>(R0.B, R0.X), volumeIn<D>(R1.B, R1.X)},
+                     make_float2(__fsub_rn(deviationIn<D>(R0.B, R0.X), devI), __fsub_rn(deviationIn<D>(R1.B, R1.X), devI))};
+    }
+    template <PairKind KIND>
+    __device__ __forceinline__ void finish(const Neighbours &N, const Taken &taken)
+    {
+        const float2 q = mul2(N.r, N.k.invH), grad = kernelGradient<K>(q, N.k);     // (dW/dr) / r
+        const float2 ratio = make_float2(__fdiv_rn(kernelValue<K>(q.x, N.k.of(0)), P.spacingKernel),
+                                         __fdiv_rn(kernelValue<K>(q.y, N.k.of(1)), P.spacingKernel));
+        const float2 square = mul2(ratio, ratio), weight = fma2(mul2(both(0.2f), square), square, both(1.0f));
+        const float2 scale = make_float2(N.live[0] ? __fmul_rn(taken.volume[0], grad.x) : 0.0f,
+                                         N.live[1] ? __fmul_rn(taken.volume[1], grad.y) : 0.0f);
         for (int a = 0; a < D; ++a) {
-            const float weighted = volume * grad * d[a];
-            plain[a] += weighted;
-            gradient[a] += weight * weighted;
-            densityGradient[a] += difference * weighted;
+            const float2 weighted = mul2(scale, N.d[a]);
+            plain[a] = add2(plain[a], weighted);
+            gradient[a] = fma2(weight, weighted, gradient[a]);
+            densityGradient[a] = fma2(taken.difference, weighted, densityGradient[a]);
         }
-        total -= volume * grad * r * r;
+        total = fma2(mul2(both(-1.0f), mul2(scale, N.r)), N.r, total);
     }
 };
 
@@ -1305,11 +1397,13 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftFieldsKernel
         F.shiftRhoGrad[i] = zero;
         return;
     }
-    ShiftFieldsVisit<D, K> visit{P, F, Smoothing<K, D>(P)};
+    ShiftFieldsVisit<D, K> visit{P, Smoothing<K, D, false>(P, hs)};
     visit.devI = deviationOf<D>(F, i);
-    for (int a = 0; a < 3; ++a) visit.gradient[a] = visit.plain[a] = visit.densityGradient[a] = 0.0f;
-    visit.total = 0.0f;
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, visit);
+    for (int a = 0; a < D; ++a) visit.gradient[a] = visit.plain[a] = visit.densityGradient[a] = both(0.0f);
+    visit.total = both(0.0f);
+    const Row row = openRow<D, FINE>(P, F, i, G.t, hs);
+    sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, visit);
+    sumPairs<D, T, FINE, kWallPair>(P, F, row, false, visit);
     float c[3] = {0.0f, 0.0f, 0.0f}, g[3] = {0.0f, 0.0f, 0.0f}, rg[3] = {0.0f, 0.0f, 0.0f};
     for (int a = 0; a < D; ++a) {
         c[a] = groupSum<T>(visit.plain[a], G.mask);
@@ -1329,25 +1423,24 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftFieldsKernel
 // kernel-weighted sum of their outward normals -grad C0 / |grad C0|.
 template <int D, int K>
 struct SurfaceVisit {
+    static constexpr bool kCopied = false;
     static constexpr bool kSkipCoincident = false;
     static constexpr bool kKinetic = false;
     const Params &P; const Frame &F;
-    Smoothing<K, D> S;
+    Smoothing<K, D, false> S;
     float normal[3];
     int vicinity;
-    __device__ bool accept(bool fluidJ) const { return fluidJ; }
-    __device__ void operator()(int j, const float *, float r, float h, bool, int, const float4 &, const float4 &)
+    __device__ void operator()(int j, const float *, float r, float, const KernelAt &k, const NeighbourRows &)
     {
         const float4 plainJ = __ldg(&F.shiftPlain[j]);
         if (!(plainJ.w < P.shiftThreshold)) return;
         vicinity = 1;
-        const float length = sqrtf(plainJ.x * plainJ.x + plainJ.y * plainJ.y + plainJ.z * plainJ.z);
+        const float length = sqrtf(__fmaf_rn(plainJ.z, plainJ.z, __fmaf_rn(plainJ.y, plainJ.y, __fmul_rn(plainJ.x, plainJ.x))));
         if (length > 0.0f) {
-            const KernelAt k = S.at(h);
-            const float w = kernelValue<K>(r * k.invH, k) / length;
-            normal[0] -= w * plainJ.x;
-            normal[1] -= w * plainJ.y;
-            normal[2] -= w * plainJ.z;
+            const float w = __fdiv_rn(kernelValue<K>(__fmul_rn(r, k.invH), k), length);
+            normal[0] = __fmaf_rn(-w, plainJ.x, normal[0]);
+            normal[1] = __fmaf_rn(-w, plainJ.y, normal[1]);
+            normal[2] = __fmaf_rn(-w, plainJ.z, normal[2]);
         }
     }
 };
@@ -1355,22 +1448,20 @@ struct SurfaceVisit {
 // The velocity at the shifted position: sum_j V_j (v_j - v_i) (grad W_ij . shift) over fluid pairs.
 template <int D, int K>
 struct ShiftedVelocityVisit {
+    static constexpr bool kCopied = false;
     static constexpr bool kSkipCoincident = true;
     static constexpr bool kKinetic = true;
-    const Params &P; const Frame &F;
-    Smoothing<K, D> S;
+    static constexpr bool kAuxRow = D == 3;
+    Smoothing<K, D, false> S;
     float vi[3], shift[3], change[3];
-    __device__ bool accept(bool fluidJ) const { return fluidJ; }
-    __device__ void operator()(int j, const float *d, float r, float h, bool, int, const float4 &B, const float4 &Kj)
+    __device__ void operator()(int, const float *d, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
-        const KernelAt k = S.at(h);
-        const float4 X = auxRow<D>(F, j);
-        float dot = 0.0f;
-        for (int a = 0; a < D; ++a) dot += d[a] * shift[a];
-        const float f = volumeIn<D>(B, X) * kernelGradient<K>(r * k.invH, k) * dot;
+        float dot = __fmul_rn(d[0], shift[0]);
+        for (int a = 1; a < D; ++a) dot = __fmaf_rn(d[a], shift[a], dot);
+        const float f = __fmul_rn(__fmul_rn(volumeIn<D>(R.B, R.X), kernelGradient<K>(__fmul_rn(r, k.invH), k)), dot);
         float vj[3];
-        velocityIn<D>(Kj, vj);
-        for (int a = 0; a < D; ++a) change[a] += f * (vj[a] - vi[a]);
+        velocityIn<D>(R.K, vj);
+        for (int a = 0; a < D; ++a) change[a] = __fmaf_rn(f, __fsub_rn(vj[a], vi[a]), change[a]);
     }
 };
 
@@ -1391,10 +1482,11 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftKernel(Param
         if (G.t == 0) { F.shift[i] = zero; F.shiftDv[i] = zero; }
         return;
     }
-    SurfaceVisit<D, K> surface{P, F, Smoothing<K, D>(P)};
+    SurfaceVisit<D, K> surface{P, F, Smoothing<K, D, false>(P, hs)};
     surface.normal[0] = surface.normal[1] = surface.normal[2] = 0.0f;
     surface.vicinity = 0;
-    forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, surface);
+    const Row row = openRow<D, FINE>(P, F, i, G.t, hs);
+    sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, surface);
     float normal[3];
     for (int a = 0; a < 3; ++a) normal[a] = groupSum<T>(surface.normal[a], G.mask);
     const bool vicinity = groupSum<T>((float)surface.vicinity, G.mask) > 0.0f;
@@ -1423,9 +1515,9 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftKernel(Param
     const float densityChange = shift[0] * rg.x + shift[1] * rg.y + shift[2] * rg.z;
     float change[3] = {0.0f, 0.0f, 0.0f};
     if (shift[0] != 0.0f || shift[1] != 0.0f || shift[2] != 0.0f) {
-        ShiftedVelocityVisit<D, K> velocity{P, F, Smoothing<K, D>(P)};
+        ShiftedVelocityVisit<D, K> velocity{Smoothing<K, D, false>(P, hs)};
         for (int a = 0; a < 3; ++a) { velocity.vi[a] = vi[a]; velocity.shift[a] = shift[a]; velocity.change[a] = 0.0f; }
-        forEachNeighbour<D, T, FINE>(P, F, i, G.t, hs, velocity);
+        sumPairs<D, T, FINE, kFluidPair>(P, F, row, true, velocity);
         for (int a = 0; a < D; ++a) change[a] = groupSum<T>(velocity.change[a], G.mask);
     }
     if (G.t != 0) return;
@@ -1482,37 +1574,44 @@ __global__ void shiftDriftKernel(Params P, Frame F, Control *ctl, Enforcement E,
 
 static inline int blocksFor(long long n, int block) { return (int)((n + block - 1) / block); }
 
-#ifndef SPH_LIST_LANES_2D
-#define SPH_LIST_LANES_2D 8
-#endif
-constexpr int kListLanes2 = SPH_LIST_LANES_2D;
-constexpr int kListLanes3 = 4;
+// The table kernel: in 3D a cell holds about 8 particles, and the cell batches build the table a quarter
+// faster than lanes a particle (19.8 against 14.4 ms a step on the 16-ppd ridge when both were built);
+// a 2D cell holds about 4, too few to pay for a batch's setup (0.149 against 0.112 ms on the 64-ppd
+// beach), so 2D keeps the lanes.  The table is the same whatever the batch or the lanes.
+template <int D, int SHARE>
+static void launchListAs(const LaunchArgs &A)
+{
+    cudaStream_t st = A.stream;
+    if constexpr (D == 3) {
+        const int grid = blocksFor((long long)blocksFor(A.P.n, SHARE) * 32, kBlock);
+        if (A.P.precise && !A.P.mixedH) cellListKernel<D, SHARE, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else if (A.P.precise) cellListKernel<D, SHARE, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else if (!A.P.mixedH) cellListKernel<D, SHARE, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else cellListKernel<D, SHARE, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+    } else {
+        const int grid = blocksFor((long long)A.P.n * SHARE, kBlock);
+        if (A.P.precise && !A.P.mixedH) listKernel<D, SHARE, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else if (A.P.precise) listKernel<D, SHARE, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else if (!A.P.mixedH) listKernel<D, SHARE, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        else listKernel<D, SHARE, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+    }
+}
 
-// The table kernel: lanes a slot (the 2D stencil's runs are longer), and its precision and
-// smoothing-length forms.
-// The table kernel a dimension takes: in 3D a cell holds about 8 particles, and the cell batches
-// build the table a quarter faster than lanes a particle (19.8 against 14.4 ms a step on the 16-ppd
-// ridge, 17.1 against 13.1 on the refined 12-ppd one); a 2D cell holds about 4, too few to pay for
-// a batch's setup (0.149 against 0.112 ms on the 64-ppd beach), so 2D keeps the lanes.
+// Particles too few to fill the chip take more of it each: 4 in place of 8 members a batch in 3D (below
+// 65,536 particles, 8,192 warps of 8; the 27,000-particle channel's table 0.322 -> 0.270 ms, while the
+// 760,000-particle ridge's goes from 3.17 to 3.65), 16 in place of 8 lanes a slot in 2D (below 24,576
+// particles; the 10,000-particle beach's table 0.0449 -> 0.0367 ms, the 114,000-particle one's 0.133 ->
+// 0.143).
 template <int D>
 static void launchList(const LaunchArgs &A)
 {
-    if (D == 3) {
-        const int grid = blocksFor((long long)blocksFor(A.P.n, kBatch) * 32, kBlock);
-        cudaStream_t st = A.stream;
-        if (A.P.precise && !A.P.mixedH) cellListKernel<D, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (A.P.precise) cellListKernel<D, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (!A.P.mixedH) cellListKernel<D, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else cellListKernel<D, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        return;
+    if constexpr (D == 3) {
+        if (A.P.n < 65536) launchListAs<D, 4>(A);
+        else launchListAs<D, 8>(A);
+    } else {
+        if (A.P.n < 24576) launchListAs<D, 16>(A);
+        else launchListAs<D, 8>(A);
     }
-    constexpr int L = D == 2 ? kListLanes2 : kListLanes3;
-    const int grid = blocksFor((long long)A.P.n * L, kBlock);
-    cudaStream_t st = A.stream;
-    if (A.P.precise && !A.P.mixedH) listKernel<D, L, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-    else if (A.P.precise) listKernel<D, L, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-    else if (!A.P.mixedH) listKernel<D, L, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-    else listKernel<D, L, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
 }
 
 template <int D, int K, int T, bool FINE>
@@ -1557,8 +1656,8 @@ static void launchT(const LaunchArgs &A, Stage stage)
 template <int D, int K>
 static void launchDK(const LaunchArgs &A, Stage stage)
 {
-    if (A.P.levels > 1) {
-        // the shifting sweeps never see two levels (shifting needs one smoothing length)
+    if (A.P.levels > 1 || A.P.mixedH) {
+        // the shifting sweeps never see differing lengths (shifting needs one smoothing length)
         if (A.threads >= 8) launchT<D, K, 8, true>(A, stage);
         else if (A.threads == 4) launchT<D, K, 4, true>(A, stage);
         else if (A.threads == 2) launchT<D, K, 2, true>(A, stage);
@@ -1571,13 +1670,15 @@ static void launchDK(const LaunchArgs &A, Stage stage)
     }
 }
 
-void launchStage(const LaunchArgs &A, Stage stage)
+// This file is compiled once a dimension (SPH_SWEEP_DIM 2 and 3), so the two halves build side by side.
+#if SPH_SWEEP_DIM == 2
+void launchStage2(const LaunchArgs &A, Stage stage)
+#else
+void launchStage3(const LaunchArgs &A, Stage stage)
+#endif
 {
-    const int D = A.P.dim, K = A.P.kind;
-    if (D == 2 && K == 0) launchDK<2, 0>(A, stage);
-    else if (D == 2 && K == 1) launchDK<2, 1>(A, stage);
-    else if (D == 3 && K == 0) launchDK<3, 0>(A, stage);
-    else launchDK<3, 1>(A, stage);
+    if (A.P.kind == 0) launchDK<SPH_SWEEP_DIM, 0>(A, stage);
+    else launchDK<SPH_SWEEP_DIM, 1>(A, stage);
 }
 
 }  // namespace sph

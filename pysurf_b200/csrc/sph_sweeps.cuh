@@ -8,17 +8,19 @@
 //
 // Each step the table kernel walks the cells once and records, per particle, the neighbours the
 // walk accepts, in the walk's order, in a table of 16-byte chunks: entries 4c .. 4c + 3 of particle
-// i form chunk c, stored at c * stride + i, so a lane takes four neighbours with one load and a
-// warp's loads of chunk c are contiguous.  The sweeps then read the table
+// i form chunk c, stored at c * stride + i, so the chunks c of a warp's particles are contiguous.  A
+// row holds the fluid neighbours from its front and the boundary neighbours from its back, so that a
+// sweep sums each kind in a loop of its own, without a test of each neighbour's kind.
+// The sweeps then read the table
 // instead of walking the cells: no candidate that fails the distance test is visited again, so
 // a warp's lanes stay busy.  A particle with more neighbours than its row holds walks the cells
-// instead.  Table and walk feed one loop body, the visitor called from one place, so a sweep
-// gives the same bits either way.
+// instead.  Table and walk hand the same pairs of neighbours to the same arithmetic, whose roundings
+// are explicit on every path that differs, so a sweep gives the same bits either way.
 //
-// T threads serve one particle: lane t of the group takes the particle's neighbours in chunks t,
-// t + T, t + 2T, ... (neighbour k, counted in the walk's order, is in chunk k / 4), and the group
-// sums its partial sums with a
-// butterfly of shuffles, which gives every lane the same bits (each level adds two values whose
+// T threads serve one particle: lane t of the group takes the particle's neighbours of a kind
+// k = t, t + T, t + 2T, ..., counted in the walk's order, so that the lanes read neighbouring slots' rows together
+// (the order runs along the grid's rows, where slots follow one another), and the group sums its
+// partial sums with a butterfly of shuffles, which gives every lane the same bits (each level adds two values whose
 // order does not matter).  T = 1 is the plain one-thread-per-particle sweep.
 //
 // A periodic y axis (3D) is searched a second time from the particle's image across the seam
@@ -108,6 +110,15 @@ __device__ __forceinline__ float groupSumCompensated(float s, float c, unsigned 
     return __fadd_rn(s, c);
 }
 
+// The same from a lane's two running sums (its even and its odd neighbours').
+template <int T>
+__device__ __forceinline__ float groupSumCompensated(const float2 &s, const float2 &c, unsigned mask)
+{
+    float sum, error;
+    twoSum(s.x, s.y, sum, error);
+    return groupSumCompensated<T>(sum, __fadd_rn(__fadd_rn(c.x, c.y), error), mask);
+}
+
 // The coarse test's squared distance between float32 points, and a pair's separation and squared
 // distance.  Each takes its roundings from explicit intrinsics, so that the table kernel and the
 // walk, compiled apart, reach the same decision on a pair at the edge of the support.  The support
@@ -150,13 +161,34 @@ __device__ __forceinline__ float separation2(const Params &P, const float pi[3],
     return r2;
 }
 
-// A pair's distance from its squared distance: the hardware reciprocal square root (about 2 ulp)
-// times r^2, 0 for a coincident pair.  The support is decided on r^2, so r only enters the kernel's
-// value and gradient, where its rounding is of the float32 terms' own size; continuity's and the
-// correction matrix's float64 parts take one Newton step from it to float64's digits.
-__device__ __forceinline__ float pairDistance(float r2)
+// Two neighbours' values side by side: Blackwell's packed float32 instructions take both in one issue
+// slot, each rounded as the single instruction rounds.
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add2(const float2 &a, const float2 &b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(const float2 &a, const float2 &b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(const float2 &a, const float2 &b, const float2 &c) { return __ffma2_rn(a, b, c); }
+
+// A pair's distance from its squared distance: r^2 times the hardware reciprocal square root (about 2
+// ulp), 0 for a coincident pair, and that reciprocal (finite always).  The support is decided on r^2,
+// so r only enters the kernel's value and gradient, where its rounding is of the float32 terms' own
+// size; continuity's and the correction matrix's float64 parts take one Newton step from it to
+// float64's digits.  The .ftz form skips the subnormal scaling of rsqrtf; the floor keeps its argument
+// normal, and a pair under it (r < 1e-15 m) is coincident to every kernel.
+constexpr float kLeastDistance2 = 1.0e-30f;
+__device__ __forceinline__ float inverseRoot(float r2)
 {
-    return r2 > 0.0f ? r2 * rsqrtf(r2) : 0.0f;
+    float inverse;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inverse) : "f"(fmaxf(r2, kLeastDistance2)));
+    return inverse;
+}
+
+// a / b to 2 ulp for a normal b up to 2^126: __fdividef without its subnormal scaling (a subnormal
+// counts as zero).
+__device__ __forceinline__ float quickDivide(float a, float b)
+{
+    float q;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+    return q;
 }
 
 // (2 h)^2, the support test's bound.
@@ -201,20 +233,12 @@ struct Origin {
     double shift64;
 };
 
-// The candidates of slot i, one at a time: its table row when the row holds them all, else the
-// cells of its searches.  Search s is of grid level s >> 1 (coarse, then fine when the particles
-// carry two levels of smoothing length) from origin s & 1 (the particle, then its periodic image
-// when it lies near the seam).
+// The candidates of a walk over the cells of slot i's searches, one at a time.  Search s is of grid
+// level s >> 1 (coarse, then fine when the particles carry two levels of smoothing length) from origin
+// s & 1 (the particle, then its periodic image when it lies near the seam).
 // FINE: the particles carry two levels of smoothing length (else only the coarse grid is searched).
 template <int D, bool FINE>
 struct Candidates {
-    // table
-    const int4 *column;
-    int stride, count, k, step;
-    int4 chunk;         // the entries still to visit of the current chunk, first in x
-    int4 ahead;         // this lane's next chunk, loaded while the current one's neighbours are summed
-    // walk
-    bool walking;
     int search, first, nx, ny, x0, x1, y0, y1, z1, zz, yy, j, end;
     const int *cellStart;
 
@@ -254,23 +278,6 @@ struct Candidates {
     __device__ __forceinline__ bool next(const Params &P, const Origin &O, const float pi[3], const float li[3],
                                          int &jOut, int &imageOut, int &levelOut)
     {
-        if (!walking) {
-            if (k >= count) return false;
-            if ((k & 3) == 0) {
-                // the table streams from DRAM: the lane's next chunk is requested a chunk ahead
-                chunk = ahead;
-                const int next = (k >> 2) + step;
-                if (4 * next < count) ahead = __ldg(column + (size_t)next * stride);
-            }
-            const int entry = chunk.x;
-            chunk.x = chunk.y; chunk.y = chunk.z; chunk.z = chunk.w;
-            // the chunk's last entry passes to this lane's next chunk
-            k = (k & 3) == 3 ? k + 1 + 4 * (step - 1) : k + 1;
-            jOut = entry & 0x7FFFFFFF;
-            imageOut = entry < 0 ? 1 : 0;
-            levelOut = 0;
-            return true;
-        }
         while (true) {
             if (++j < end) {
                 jOut = j;
@@ -295,50 +302,22 @@ struct Candidates {
     }
 };
 
-// Visit the neighbours of slot i.  Every neighbour j != i with r^2 < (2 h_ij)^2 (the table's
-// criterion) is counted in the walk's order; lane t of T takes those whose count k has k / 4 = t
-// mod T (the table's chunks t, t + T, ...).  Of those, the visitor gets (j, d, r, h_ij, fluidJ,
-// image, pb row of j, kin row of j when Visitor::kKinetic) when Visitor::accept(fluidJ), and
-// r >= 1e-12 where Visitor::kSkipCoincident.
-// useTable: false forces the walk (the table kernel itself).
-// A boundary particle's row holds its fluid neighbours only: every sweep that reads boundary rows
-// takes fluid neighbours alone (the wall pressure, continuity), except a visitor that says
-// kWholeBoundaryRows (the Shepard sum, whose boundary rows the host-step call returns), which walks
-// a boundary row's cells for all of them.
-template <class V, class = void>
-struct WholeBoundaryRows {
-    static constexpr bool value = false;
-};
-template <class V>
-struct WholeBoundaryRows<V, std::void_t<decltype(V::kWholeBoundaryRows)>> {
-    static constexpr bool value = V::kWholeBoundaryRows;
-};
-// Whether a sweep walks boundary rows at all (kBoundaryRows); the others run fluid rows only and
-// skip the row's kind at compile time.
-template <class V, class = void>
-struct BoundaryRows {
-    static constexpr bool value = false;
-};
-template <class V>
-struct BoundaryRows<V, std::void_t<decltype(V::kBoundaryRows)>> {
-    static constexpr bool value = V::kBoundaryRows;
-};
+// The pairs a sweep sums: of a fluid neighbour, of a boundary neighbour, or (continuity) of a fluid and
+// a boundary particle, whichever way round.
+enum PairKind { kFluidPair, kWallPair, kCrossPair };
 
-// Whether a sweep reading its particle's table row keeps the next neighbour's rows in flight while it
-// sums the current one (kPipelined): one more neighbour's loads in registers, the same visits in the
-// same order, so the same bits.
+// Whether a visitor takes two neighbours at a time (kPaired).
 template <class V, class = void>
-struct Pipelined {
+struct Paired {
     static constexpr bool value = false;
 };
 template <class V>
-struct Pipelined<V, std::void_t<decltype(V::kPipelined)>> {
-    static constexpr bool value = V::kPipelined;
+struct Paired<V, std::void_t<decltype(V::kPaired)>> {
+    static constexpr bool value = V::kPaired;
 };
 
 // Whether a visitor reads a neighbour's aux row (3D: P2, deviation, V) or remainder row (kAuxRow,
-// kLowRow): the walk loads them with the others, so the pipeline keeps them in flight too, and hands
-// them to the visitor in its rowX / rowLow.
+// kLowRow): they are loaded with the others, in flight as they are.
 template <class V, class = void>
 struct AuxRow {
     static constexpr bool value = false;
@@ -356,134 +335,263 @@ struct LowRow<V, std::void_t<decltype(V::kLowRow)>> {
     static constexpr bool value = V::kLowRow;
 };
 
-template <int D, class Visitor>
-__device__ __forceinline__ void loadExtra(const Frame &F, int j, float4 &X, float4 &L)
-{
-    if constexpr (AuxRow<Visitor>::value) X = auxRow<D>(F, j);
-    if constexpr (LowRow<Visitor>::value) L = __ldg(&F.low[j]);
-}
+// A neighbour's rows, as far as the visitor reads them.
+struct NeighbourRows {
+    float4 A, B, K, X, L;
+};
 
-// One table entry's visit: the separation from the rows already loaded, the support's r, the visitor.
-template <int D, class Visitor>
-__device__ __forceinline__ void visitEntry(const Params &P, const float pi[3], const float li[3], double shift64,
-                                           float hI, int j, int image, const float4 &A, const float4 &B,
-                                           const float4 &Kj, const float4 &X, const float4 &L, Visitor &visit)
+// A row's load, which stays where it is written: the compiler would otherwise move it down to its first
+// use, and the software pipeline of sumPairs() with it.
+__device__ __forceinline__ float4 loadEarly(const float4 *at)
 {
-    const float offset = image ? (float)shift64 : 0.0f;
-    float pj[3], lj[3], d[3];
-    pointIn<D>(A, pj);
-    const float hs = signedLengthIn<D>(A, B);
-    const bool fluidJ = hs > 0.0f;
-    if (!visit.accept(fluidJ)) return;
-    remainderIn<D>(A, B, lj);
-    const float r2 = separation2<D>(P, pi, li, pj, lj, offset, image, shift64, d);
-    const float h = P.mixedH ? 0.5f * (hI + fabsf(hs)) : P.hMax;
-    const float r = pairDistance(r2);
-    if (Visitor::kSkipCoincident && r < 1.0e-12f) return;
-    if constexpr (AuxRow<Visitor>::value) visit.rowX = X;
-    if constexpr (LowRow<Visitor>::value) visit.rowLow = L;
-    visit(j, d, r, h, fluidJ, image, B, Kj);
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
+    return v;
 }
 
 template <int D, class Visitor>
-__device__ __forceinline__ void loadRows(const Frame &F, int j, float4 &A, float4 &B, float4 &Kj)
+__device__ __forceinline__ void loadRows(const Frame &F, int j, NeighbourRows &R)
 {
-    A = __ldg(&F.pa[j]);
-    B = __ldg(&F.pb[j]);
-    Kj = Visitor::kKinetic ? __ldg(&F.kin[j]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    R.A = loadEarly(&F.pa[j]);
+    R.B = loadEarly(&F.pb[j]);
+    if constexpr (Visitor::kKinetic) R.K = loadEarly(&F.kin[j]);
+    if constexpr (AuxRow<Visitor>::value) R.X = loadEarly(&F.aux[j]);
+    if constexpr (LowRow<Visitor>::value) R.L = loadEarly(&F.low[j]);
 }
 
-template <int D, int T, bool FINE, class Visitor>
-__device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F, int i, int t, float hI,
-                                                 Visitor &visit, bool useTable = true)
+// Two neighbours of a particle as a paired visitor gets them: their slots, whether each counts and lies
+// across the seam; d = x_i - x_j, h_ij, and, for finish(), r and 1 / r and the kernel's constants at h_ij.
+struct Neighbours {
+    int j[2];
+    bool live[2];
+    int image[2];
+    float2 d[3], h, r, inverse;
+    KernelPair k;
+};
+
+// A particle's row as its sweep opens it: its slot, this lane, its length, point and remainder, the
+// periodic image's shift when it lies near the seam, its fluid and boundary neighbours in the table,
+// and whether the table lists them (else the sweep walks the cells).  A boundary particle's row holds
+// its fluid neighbours only: every sweep over boundary rows takes fluid neighbours alone, except the
+// Shepard sum, which walks a boundary row's cells for all of them (whole).
+struct Row {
+    int i, t;
+    float hI, pi[3], li[3], reach;
+    double shift64;
+    bool seam, listed;
+    int2 count;
+};
+
+// FINE: the smoothing lengths differ; else every length is P.hMax.
+template <int D, bool FINE>
+__device__ __forceinline__ Row openRow(const Params &P, const Frame &F, int i, int t, float hI, bool whole = false)
 {
-    const bool boundaryRow = BoundaryRows<Visitor>::value && signedLength<D>(F, i) <= 0.0f;
-    const bool wholeRow = WholeBoundaryRows<Visitor>::value && boundaryRow;
-    const bool fluidOnly = boundaryRow && !wholeRow;     // the row the table holds, in the walk too
-    float pi[3], li[3];
-    pointOf<D>(F, i, pi);
-    remainderOf<D>(F, i, li);
-    const float reach = P.mixedH ? hI + P.hMax : 2.0f * P.hMax;
-    const float limit = kCandidateMargin * reach * reach;
-    // the coarse test's bound for fine candidates: no fine neighbour lies past hI + fineMax
-    const float fineReach = hI + P.fineMax;
-    const float fineLimit = kCandidateMargin * fineReach * fineReach;
-    Origin O;
-    O.cell = 0;
+    Row O;
+    O.i = i;
+    O.t = t;
     O.hI = hI;
-    O.shift64 = 0.0;
+    pointOf<D>(F, i, O.pi);
+    remainderOf<D>(F, i, O.li);
+    O.reach = FINE ? hI + P.hMax : 2.0f * P.hMax;
     O.seam = false;
-    if (D == 3 && P.period > 0.0 && (pi[1] < reach || pi[1] > P.periodF - reach)) {
+    O.shift64 = 0.0;
+    if (D == 3 && P.period > 0.0 && (O.pi[1] < O.reach || O.pi[1] > P.periodF - O.reach)) {
         O.seam = true;
-        O.shift64 = pi[1] < 0.5f * P.periodF ? P.period : -P.period;
+        O.shift64 = O.pi[1] < 0.5f * P.periodF ? P.period : -P.period;
     }
-    const double shift64 = O.shift64;
+    O.count = P.listCap > 0 && !whole ? __ldg(&F.ncount[i]) : make_int2(0, 0);
+    O.listed = P.listCap > 0 && !whole && O.count.x + O.count.y <= P.listCap;
+    return O;
+}
 
-    Candidates<D, FINE> C;
-    const int count = useTable && P.listCap > 0 && !wholeRow ? __ldg(&F.ncount[i]) : 0;
-    C.walking = wholeRow || !(useTable && P.listCap > 0 && count <= P.listCap);
-    if (!C.walking) {
-        C.column = reinterpret_cast<const int4 *>(F.nbr) + i;
-        C.stride = P.listStride;
-        C.count = count;
-        C.k = 4 * t;
-        if (C.k < count) C.ahead = __ldg(C.column + (size_t)t * C.stride);
-        C.step = T;
+// Two neighbours' pairs go in two parts, so that the rows of the next two can load in between, into the
+// registers these two's rows leave: takeBoth() reads all it needs from the rows, finishBoth() sums.
+// A visitor with kPaired has a take<KIND>(N, R0, R1) that returns what its finish<KIND>(N, taken) adds,
+// the two neighbours together in packed float32; any other is called with each that counts in turn, from
+// its rows.
+// entry0, entry1: table entries (the slot, the top bit a pair across the seam); second: whether there is
+// an entry1 (else it repeats entry0, and does not count).  A neighbour at r < 1e-12 does not count where
+// Visitor::kSkipCoincident.
+struct BothRows {
+    NeighbourRows R0, R1;
+};
+template <int D, int PRECISE, bool FINE, PairKind KIND, class Visitor>
+__device__ __forceinline__ auto takeBoth(const Params &P, const Row &O, int entry0, int entry1, bool second,
+                                         const NeighbourRows &R0, const NeighbourRows &R1, Visitor &visit,
+                                         Neighbours &N)
+{
+    const int entries[2] = {entry0, entry1};
+    float d[2][3], r2[2], h[2];
+    for (int q = 0; q < 2; ++q) {
+        const NeighbourRows &R = q ? R1 : R0;
+        N.j[q] = entries[q] & 0x7FFFFFFF;
+        N.image[q] = D == 3 && entries[q] < 0 ? 1 : 0;
+        float pj[3], lj[3];
+        pointIn<D>(R.A, pj);
+        remainderIn<D>(R.A, R.B, lj);
+        r2[q] = separation2<D, PRECISE>(P, O.pi, O.li, pj, lj, N.image[q] ? (float)O.shift64 : 0.0f, N.image[q],
+                                        O.shift64, d[q]);
+        h[q] = FINE ? 0.5f * (O.hI + fabsf(signedLengthIn<D>(R.A, R.B))) : P.hMax;
+        N.live[q] = (q == 0 || second) && (!Visitor::kSkipCoincident || r2[q] >= 1.0e-24f);
+    }
+    for (int a = 0; a < 3; ++a) N.d[a] = make_float2(d[0][a], d[1][a]);
+    N.r = make_float2(r2[0], r2[1]);        // r^2 until finishBoth()
+    N.h = make_float2(h[0], h[1]);
+    if constexpr (Paired<Visitor>::value) return visit.template take<KIND>(N, R0, R1);
+    else return BothRows{R0, R1};
+}
+
+// What takeBoth() returns for a visitor.
+template <int D, bool FINE, PairKind KIND, class Visitor>
+using Taken = decltype(takeBoth<D, 1, FINE, KIND>(std::declval<const Params &>(), std::declval<const Row &>(), 0, 0, true,
+                                                  std::declval<const NeighbourRows &>(),
+                                                  std::declval<const NeighbourRows &>(), std::declval<Visitor &>(),
+                                                  std::declval<Neighbours &>()));
+
+template <PairKind KIND, class Visitor, class TakenValues>
+__device__ __forceinline__ void finishBoth(Neighbours &N, const TakenValues &taken, Visitor &visit)
+{
+    N.inverse = make_float2(inverseRoot(N.r.x), inverseRoot(N.r.y));
+    N.r = mul2(N.r, N.inverse);
+    N.k = visit.S.at(N.h);
+    if constexpr (Paired<Visitor>::value) {
+        visit.template finish<KIND>(N, taken);
     } else {
-        O.cell = F.cell[i];
-        C.cellStart = F.cellStart;
-        C.startSearch(P, O, pi, li, 0);
+        const float d0[3] = {N.d[0].x, N.d[1].x, N.d[2].x}, d1[3] = {N.d[0].y, N.d[1].y, N.d[2].y};
+        if (N.live[0]) visit(N.j[0], d0, N.r.x, N.h.x, N.k.of(0), taken.R0);
+        if (N.live[1]) visit(N.j[1], d1, N.r.y, N.h.y, N.k.of(1), taken.R1);
     }
+}
 
-    int counted = 0, j = 0, image = 0, level = 0;
-    if constexpr (Pipelined<Visitor>::value) {
-        if (!C.walking) {
-            // a software pipeline over the row: the next entry's rows load while this one is summed
-            float4 A, B, Kj, X, L;
-            bool more = C.next(P, O, pi, li, j, image, level);
-            if (more) { loadRows<D, Visitor>(F, j, A, B, Kj); loadExtra<D, Visitor>(F, j, X, L); }
-            while (more) {
-                int jn = 0, imagen = 0;
-                float4 An, Bn, Kn, Xn, Ln;
-                more = C.next(P, O, pi, li, jn, imagen, level);
-                if (more) { loadRows<D, Visitor>(F, jn, An, Bn, Kn); loadExtra<D, Visitor>(F, jn, Xn, Ln); }
-                visitEntry<D>(P, pi, li, shift64, hI, j, image, A, B, Kj, X, L, visit);
-                j = jn; image = imagen; A = An; B = Bn; Kj = Kn; X = Xn; L = Ln;
+template <int D, int PRECISE, bool FINE, PairKind KIND, class Visitor>
+__device__ __forceinline__ void visitBoth(const Params &P, const Row &O, int entry0, int entry1, bool second,
+                                          const NeighbourRows &R0, const NeighbourRows &R1, Visitor &visit)
+{
+    Neighbours N;
+    const auto taken = takeBoth<D, PRECISE, FINE, KIND>(P, O, entry0, entry1, second, R0, R1, visit, N);
+    finishBoth<KIND>(N, taken, visit);
+}
+
+// Visit the neighbours of one kind (fluid or boundary) of an open row, as pairs of KIND.  Every such
+// neighbour j != i with r^2 < (2 h_ij)^2 (the table's criterion) is counted in the walk's order; lane t
+// of T takes those whose count k has k = t mod T, two at a time.
+template <int D, int T, bool FINE, PairKind KIND, class Visitor>
+__device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const Row &O, bool fluid, Visitor &visit)
+{
+    if (O.listed) {
+        // the lane's entries: k = t, t + T, ... from the row's front, or from its back
+        const int count = fluid ? O.count.x : O.count.y;
+        const int *column = F.nbr + 4 * (size_t)O.i;
+        const long long stride = 4ll * P.listStride;
+        auto place = [&](int k) {
+            const int e = fluid ? k : P.listCap - 1 - k;
+            return column + (e >> 2) * stride + (e & 3);
+        };
+        auto entry = [&](const int *at) {
+            int value;
+                        asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(value) : "l"(at));
+            return value;
+        };
+        int left = count > O.t ? (count - O.t - 1) / T + 1 : 0;
+        if (P.precise) {
+            // A software pipeline over the lane's entries: the next two neighbours' rows load while two
+            // are summed, and the entries after them.  The T lanes of a particle read T neighbouring
+            // entries, and the particles of a warp lie side by side in each chunk, so a warp's load of
+            // one entry a lane is whole 128-byte lines; each line is read once, so it is kept out of L1,
+            // which the neighbours' rows need.  The first entries load without waiting for the count:
+            // whatever lies past it is not read as one.
+            int ring[4];
+            for (int q = 0; q < 4; ++q) ring[q] = O.t + q * T < P.listCap ? entry(place(O.t + q * T)) : 0;
+            if (left == 0) return;
+            // a chunk holds four entries, so with four lanes or more every entry a lane takes is the
+            // same distance on
+            const long long step = (fluid ? T : -T) * (stride / 4);
+            const int *ahead = place(min(O.t + 4 * T, P.listCap - 1));
+            int k = O.t;
+            NeighbourRows R0, R1;
+            if (left < 2) ring[1] = ring[0];
+            loadRows<D, Visitor>(F, ring[0] & 0x7FFFFFFF, R0);
+            loadRows<D, Visitor>(F, ring[1] & 0x7FFFFFFF, R1);
+            while (true) {
+                const int j0 = ring[0], j1 = ring[1];
+                Neighbours N;
+                // the rows' values that the sums need come first, or (kCopied) copies of the rows, so
+                // that the next rows load into the same registers meanwhile
+                BothRows C;
+                Taken<D, FINE, KIND, Visitor> taken;
+                if constexpr (Visitor::kCopied) C = BothRows{R0, R1};
+                else taken = takeBoth<D, 1, FINE, KIND>(P, O, j0, j1, left > 1, R0, R1, visit, N);
+                ring[0] = ring[2];
+                ring[1] = left == 3 ? ring[2] : ring[3];
+                if (left > 2) {
+                    loadRows<D, Visitor>(F, ring[0] & 0x7FFFFFFF, R0);
+                    loadRows<D, Visitor>(F, ring[1] & 0x7FFFFFFF, R1);
+                }
+                if (left > 4) ring[2] = entry(T >= 4 ? ahead : place(k + 4 * T));
+                if (left > 5) ring[3] = entry(T >= 4 ? ahead + step : place(k + 5 * T));
+                if constexpr (Visitor::kCopied)
+                    taken = takeBoth<D, 1, FINE, KIND>(P, O, j0, j1, left > 1, C.R0, C.R1, visit, N);
+                finishBoth<KIND>(N, taken, visit);
+                if (left <= 2) break;
+                left -= 2;
+                if (T >= 4) ahead += 2 * step;
+                else k += 2 * T;
             }
             return;
         }
-    }
-    while (C.next(P, O, pi, li, j, image, level)) {
-        const float offset = image ? (float)shift64 : 0.0f;     // the search's origin: particle or image
-        const float4 A = __ldg(&F.pa[j]);
-        float pj[3];
-        pointIn<D>(A, pj);
-        if (C.walking && (coarseDistance2<D>(pi, pj, offset) >= (FINE && level ? fineLimit : limit) || j == i)) continue;
-        const float4 B = __ldg(&F.pb[j]);
-        // the kinematic row too, with the others, when the visitor reads it
-        const float4 Kj = Visitor::kKinetic ? __ldg(&F.kin[j]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float hs = signedLengthIn<D>(A, B);
-        const bool fluidJ = hs > 0.0f;
-        if (C.walking && fluidOnly && !fluidJ) continue;     // not in the row: not counted either
-        // a lone lane may skip a rejected neighbour before its separation; a group counts every one
-        if ((T == 1 || !C.walking) && !visit.accept(fluidJ)) continue;
-        float lj[3];
-        remainderIn<D>(A, B, lj);
-        float d[3];
-        const float r2 = separation2<D>(P, pi, li, pj, lj, offset, image, shift64, d);
-        const float h = P.mixedH ? 0.5f * (hI + fabsf(hs)) : P.hMax;
-        if (C.walking) {
-            if (r2 >= support2(h)) continue;
-            if (T > 1) {
-                if ((counted++ >> 2) % T != t) continue;
-                if (!visit.accept(fluidJ)) continue;
-            }
+        // separations from the float32 points alone
+        for (int k = O.t; left > 0; left -= 2, k += 2 * T) {
+            const int j0 = entry(place(k)), j1 = left > 1 ? entry(place(k + T)) : j0;
+            NeighbourRows R0, R1;
+            loadRows<D, Visitor>(F, j0 & 0x7FFFFFFF, R0);
+            loadRows<D, Visitor>(F, j1 & 0x7FFFFFFF, R1);
+            visitBoth<D, 0, FINE, KIND>(P, O, j0, j1, left > 1, R0, R1, visit);
         }
-        const float r = pairDistance(r2);
-        if (Visitor::kSkipCoincident && r < 1.0e-12f) continue;
-        if constexpr (AuxRow<Visitor>::value) visit.rowX = auxRow<D>(F, j);
-        if constexpr (LowRow<Visitor>::value) visit.rowLow = __ldg(&F.low[j]);
-        visit(j, d, r, h, fluidJ, image, B, Kj);
+        return;
+    }
+
+    // the walk
+    const float limit = kCandidateMargin * O.reach * O.reach;
+    // the coarse test's bound for fine candidates: no fine neighbour lies past hI + fineMax
+    const float fineReach = O.hI + P.fineMax;
+    const float fineLimit = kCandidateMargin * fineReach * fineReach;
+    const Origin origin{F.cell[O.i], O.hI, O.seam, O.shift64};
+    Candidates<D, FINE> C;
+    C.cellStart = F.cellStart;
+    C.startSearch(P, origin, O.pi, O.li, 0);
+    int counted = 0, j = 0, image = 0, level = 0, held = 0;
+    bool holds = false, ended = false;
+    while (true) {
+        ended = !C.next(P, origin, O.pi, O.li, j, image, level);
+        if (!ended) {
+            const float offset = image ? (float)O.shift64 : 0.0f;   // the search's origin: particle or image
+            const float4 A = __ldg(&F.pa[j]);
+            float pj[3], lj[3], d[3];
+            pointIn<D>(A, pj);
+            if (coarseDistance2<D>(O.pi, pj, offset) >= (FINE && level ? fineLimit : limit) || j == O.i) continue;
+            const float4 B = __ldg(&F.pb[j]);
+            const float hs = signedLengthIn<D>(A, B);
+            if ((hs > 0.0f) != fluid) continue;     // the other kind
+            remainderIn<D>(A, B, lj);
+            const float r2 = separation2<D>(P, O.pi, O.li, pj, lj, offset, image, O.shift64, d);
+            if (r2 >= support2(FINE ? 0.5f * (O.hI + fabsf(hs)) : P.hMax)) continue;
+            if (T > 1 && counted++ % T != O.t) continue;
+        } else if (!holds) {
+            return;
+        }
+        const int entry = ended ? held : (image ? (j | (int)0x80000000) : j);
+        if (!ended && !holds) {
+            held = entry;
+            holds = true;
+            continue;
+        }
+        NeighbourRows R0, R1;
+        loadRows<D, Visitor>(F, held & 0x7FFFFFFF, R0);
+        loadRows<D, Visitor>(F, entry & 0x7FFFFFFF, R1);
+        visitBoth<D, -1, FINE, KIND>(P, O, held, entry, !ended, R0, R1, visit);
+        if (ended) return;
+        holds = false;
     }
 }
 

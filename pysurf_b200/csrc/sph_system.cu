@@ -146,7 +146,8 @@ struct SphSystem {
     // device memory
     MasterView master[2]{};
     float4 *pa = nullptr, *pb = nullptr, *kin = nullptr, *G[3] = {}, *L[3] = {}, *gradRho = nullptr, *acc = nullptr,
-           *vec = nullptr;
+           *vec = nullptr, *S0 = nullptr;
+    float2 *S1 = nullptr;
     float4 *aux = nullptr, *low = nullptr;
     float *pres = nullptr, *rate = nullptr, *scalar = nullptr;
     int *cell = nullptr, *cellStart = nullptr;
@@ -162,11 +163,14 @@ struct SphSystem {
     int *dRank = nullptr;
     Control *hCtl = nullptr;    // pinned
     // the neighbour table: listCap entries a slot (0: the sweeps walk the cells), stride capacity
-    int *nbr = nullptr, *ncount = nullptr, *dMaxCount = nullptr;
+    int *nbr = nullptr, *dMaxCount = nullptr;
+    int2 *ncount = nullptr;
+    unsigned *wallBits = nullptr;
     void *surface = nullptr;        // the breaking tracker's read scratch
     size_t surfaceBytes = 0;
     size_t nbrEntries = 0;
     int listCap = 0;
+    bool listTogether = false;  // the rows' order as built (Params::together)
     int tableMode = 1;          // 0 never build the table, 1 build it when it fits the budget
     bool listDirty = true;      // the table's size must be taken again before the next step
     int listSizedFor = -1;      // the particle count the table's size was taken for
@@ -198,18 +202,21 @@ struct SphSystem {
             cudaFree(M.rho); cudaFree(M.m); cudaFree(M.h); cudaFree(M.fluid); cudaFree(M.orig);
             M = MasterView{};
         }
-        void *ptrs[] = {pa, pb, kin, G[0], G[1], G[2], L[0], L[1], L[2], gradRho, acc, vec, aux, low, pres, rate,
+        void *ptrs[] = {pa, pb, kin, S0, S1, G[0], G[1], G[2], L[0], L[1], L[2], gradRho, acc, vec, aux, low, pres, rate,
                         scalar, cell, sortBuffers.slotCell, sortBuffers.slotWithin, sortBuffers.perm,
-                        sortBuffers.bucket, dStage, dStageU8, dRank, nbr, ncount, eddy, shiftGrad, shiftPlain,
+                        sortBuffers.bucket, dStage, dStageU8, dRank, nbr, ncount, wallBits, eddy, shiftGrad, shiftPlain,
                         shiftRhoGrad, shiftOut, shiftDv};
         for (void *p : ptrs) cudaFree(p);
         eddy = nullptr;
         shiftGrad = shiftPlain = shiftRhoGrad = shiftOut = shiftDv = nullptr;
-        nbr = ncount = nullptr;
+        nbr = nullptr;
+        ncount = nullptr;
+        wallBits = nullptr;
         nbrEntries = 0;
         listCap = 0;
         listDirty = true;
-        pa = pb = kin = gradRho = acc = vec = nullptr;
+        pa = pb = kin = gradRho = acc = vec = S0 = nullptr;
+        S1 = nullptr;
         for (int a = 0; a < 3; ++a) G[a] = L[a] = nullptr;
         aux = low = nullptr; pres = rate = scalar = nullptr; cell = nullptr;
         sortBuffers.slotCell = sortBuffers.slotWithin = sortBuffers.perm = nullptr;
@@ -274,6 +281,8 @@ struct SphSystem {
         TRY(deviceAlloc(&low, cap));
         TRY(deviceAlloc(&pres, cap));
         for (int a = 0; a < 3; ++a) { TRY(deviceAlloc(&G[a], cap)); TRY(deviceAlloc(&L[a], cap)); }
+        TRY(deviceAlloc(&S0, cap));
+        if (dim == 3) TRY(deviceAlloc(&S1, cap));
         TRY(deviceAlloc(&gradRho, cap));
         TRY(deviceAlloc(&acc, cap));
         TRY(deviceAlloc(&vec, cap));
@@ -293,6 +302,7 @@ struct SphSystem {
         TRY(deviceAlloc(&dStageU8, cap));
         TRY(deviceAlloc(&dRank, cap));
         TRY(deviceAlloc(&ncount, cap));
+        TRY(deviceAlloc(&wallBits, cap / 32 + 1));
         CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(float4) * cap, stream));
         CUDA_TRY(cudaMemsetAsync(kin, 0, sizeof(float4) * cap, stream));
         CUDA_TRY(cudaMemsetAsync(aux, 0, sizeof(float4) * cap, stream));
@@ -436,6 +446,13 @@ struct SphSystem {
         return setupLevels();
     }
 
+    // The classic scheme: XSPH over the plain sums at one smoothing length (sph_classic_sweeps.cu).
+    bool classic() const
+    {
+        return xsphEpsilon > 0.0 && !limited && !corrected && !closure && diffusionMode == 0 && !shifting && !compensated &&
+               !wallExtrapolated && !mixedH;
+    }
+
     // ---- parameters ----------------------------------------------------------------------------
 
     Params params() const
@@ -488,7 +505,9 @@ struct SphSystem {
         P.shiftDt = 0.0;
         P.wallExtrapolated = wallExtrapolated;
         P.xsphEpsilon = (float)xsphEpsilon;
-        P.listCap = listCap;
+        P.together = classic() ? 1 : 0;
+        // rows of the other order (an option changed since they were built) are not read
+        P.listCap = listTogether == classic() ? listCap : 0;
         P.listStride = capacity;
         P.budget = budget && energy ? 1 : 0;
         P.energyStride = energyCap;
@@ -502,11 +521,12 @@ struct SphSystem {
         F.pa = pa; F.pb = pb; F.kin = kin; F.aux = aux; F.low = low; F.pres = pres;
         F.cell = cell; F.cellStart = cellStart;
         F.G0 = G[0]; F.G1 = G[1]; F.G2 = G[2];
+        F.S0 = S0; F.S1 = S1;
         F.L0 = L[0]; F.L1 = L[1]; F.L2 = L[2];
         F.gradRho = gradRho; F.acc = acc; F.rate = rate; F.scalar = scalar; F.vec = vec; F.eddy = eddy;
         F.shiftGrad = shiftGrad; F.shiftPlain = shiftPlain; F.shiftRhoGrad = shiftRhoGrad; F.shift = shiftOut;
         F.shiftDv = shiftDv;
-        F.nbr = nbr; F.ncount = ncount;
+        F.nbr = nbr; F.ncount = ncount; F.wallBits = wallBits;
         F.energy = energy; F.parts = parts;
         const MasterView &M = master[cur];
         for (int a = 0; a < 3; ++a) { F.x[a] = M.x[a]; F.v[a] = M.v[a]; }
@@ -548,6 +568,7 @@ struct SphSystem {
         framed = true;
         cellsFresh = true;
         if (listCap > 0) {
+            listTogether = classic();
             LaunchArgs A = args(const_cast<Control *>(control));
             launchStage(A, Stage::List);
         }
@@ -570,6 +591,7 @@ struct SphSystem {
         CUDA_TRY(cudaMemsetAsync(dMaxCount, 0, sizeof(int), stream));
         const int keep = listCap;
         listCap = 0;    // count only
+        listTogether = classic();
         LaunchArgs A = args(nullptr);
         A.maxCount = dMaxCount;
         launchStage(A, Stage::List);
@@ -585,9 +607,10 @@ struct SphSystem {
             size_t freeBytes = 0, totalBytes = 0;
             cudaMemGetInfo(&freeBytes, &totalBytes);
             const size_t room = freeBytes / 4 * 3 / sizeof(int) / (size_t)std::max(capacity, 1);
-            if ((size_t)cap > room) cap = (int)(room & ~(size_t)7);
+            const bool capped = (size_t)cap > room;
+            if (capped) cap = (int)(room & ~(size_t)7);
             entries = (size_t)cap * (size_t)capacity;
-            if (cap < kMinTableRow || deviceAlloc(&nbr, entries) != SPH_OK) {
+            if ((capped && cap < kMinTableRow) || deviceAlloc(&nbr, entries) != SPH_OK) {
                 nbr = nullptr;
                 cap = 0;
                 cudaGetLastError();
@@ -1211,7 +1234,7 @@ int sph_velocity_gradients(SphSystem *sys, const double *velocities, const doubl
     if (!velocities || !densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, velocities, densities, nullptr));
     LaunchArgs A = sys->args(nullptr);
-    A.wantG = 1;
+    A.wantG = kWholeGradients;
     launchStage(A, Stage::Gradients);
     launchScatterMatrix(sys->n, sys->dim, A.F.orig, A.F, 0, sys->stage(SphSystem::kOutSlot), sys->stream);
     return finish(sys, out, (size_t)sys->n * sys->dim * sys->dim);

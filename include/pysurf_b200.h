@@ -185,6 +185,11 @@ int sph_count(const SphSystem *sys, int64_t *n);
  * takes it, and its fluid flag, in caller order; the caller keeps the fluid rows.  17 bytes a
  * particle in 3D cross the bus instead of a float64 pull's 48. */
 int sph_frame(SphSystem *sys, float *positions, float *speeds, uint8_t *is_fluid);
+/* The same frame of the fluid alone, its rows packed on the device in caller order: sph_fluid_frame
+ * packs them and returns how many there are, sph_fluid_frame_rows, the next call on the handle, copies
+ * them out (positions count x dim, speeds count). */
+int sph_fluid_frame(SphSystem *sys, int64_t *count);
+int sph_fluid_frame_rows(SphSystem *sys, float *positions, float *speeds, int64_t count);
 
 /* PairSums.setBoundary (src/pysurf/sphGpu.py:2121-2171), one call per kind. */
 int sph_clear_boundary(SphSystem *sys);

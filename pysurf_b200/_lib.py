@@ -65,6 +65,8 @@ SIGNATURES = {
     'sph_pull_device': [_h, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     'sph_count': [_h, _pi64],
     'sph_frame': [_h, _pf, _pf, _pu8],
+    'sph_fluid_frame': [_h, _pi64],
+    'sph_fluid_frame_rows': [_h, _pf, _pf, _i64],
     'sph_clear_boundary': [_h],
     'sph_set_boundary_container': [_h, _pd, _pd, _i],
     'sph_set_boundary_bed': [_h, _pd, _pd, _i64, _d, _i, _d, _i, _d, _d, _d],

@@ -139,6 +139,11 @@ void launchScatterFloat4(int n, int dim, const int *orig, const float4 *values, 
 void launchScatterFloat(int n, const int *orig, const float *values, double *out, cudaStream_t st);
 // Caller-order float32 positions (n x dim), float32 speeds and fluid flags of every particle.
 void launchFrame(int n, int dim, const MasterView &M, float *positions, float *speeds, uint8_t *fluid, cudaStream_t st);
+// The fluid's rows of that frame, packed in caller order: slotOf (n ints) and counts (frameTiles(n) + 1
+// ints) are scratch, counts[frameTiles(n)] the number of rows.
+int frameTiles(int n);
+void launchFluidFrame(int n, int dim, const MasterView &M, int *slotOf, int *counts, float *positions, float *speeds,
+                      cudaStream_t st);
 void launchScatterMatrix(int n, int dim, const int *orig, const Frame &F, int which, double *out, cudaStream_t st);
 void launchScatterPressure(int n, int dim, const int *orig, const Frame &F, double *out, cudaStream_t st);
 void launchNeighbourRows(const Params &P, const Frame &F, const int64_t *offsets, int *rows, long long *counts,

@@ -1381,6 +1381,40 @@ int sph_frame(SphSystem *sys, float *positions, float *speeds, uint8_t *is_fluid
     return SPH_OK;
 }
 
+// float32 rows in the output staging: positions, then speeds; the tiles' counts past them
+static float *framePositions(SphSystem *sys) { return reinterpret_cast<float *>(sys->stage(SphSystem::kOutSlot)); }
+static float *frameSpeeds(SphSystem *sys) { return reinterpret_cast<float *>(sys->stage(SphSystem::kOutSlot + 2)); }
+
+int sph_fluid_frame(SphSystem *sys, int64_t *count)
+{
+    CHECK_SYS(sys);
+    if (!count) return fail(SPH_ERR_INVALID, "null argument");
+    *count = 0;
+    if (!sys->resident) return fail(SPH_ERR_STATE, "no device state: call sph_push first");
+    if (sys->n == 0) return SPH_OK;
+    int *counts = reinterpret_cast<int *>(sys->stage(SphSystem::kOutSlot + 3)), rows = 0;
+    launchFluidFrame(sys->n, sys->dim, sys->master[sys->cur], sys->dRank, counts, framePositions(sys), frameSpeeds(sys),
+                     sys->stream);
+    CUDA_TRY(cudaGetLastError());
+    TRY(sys->download(&rows, counts + frameTiles(sys->n), sizeof(int)));
+    CUDA_TRY(cudaStreamSynchronize(sys->stream));
+    *count = rows;
+    return SPH_OK;
+}
+
+int sph_fluid_frame_rows(SphSystem *sys, float *positions, float *speeds, int64_t count)
+{
+    CHECK_SYS(sys);
+    if (count < 0 || count > sys->n) return fail(SPH_ERR_INVALID, "more rows than particles");
+    if (count == 0) return SPH_OK;
+    if (!positions || !speeds) return fail(SPH_ERR_INVALID, "null argument");
+    if (!sys->resident) return fail(SPH_ERR_STATE, "no device state: call sph_push first");
+    TRY(sys->download(positions, framePositions(sys), sizeof(float) * (size_t)count * sys->dim));
+    TRY(sys->download(speeds, frameSpeeds(sys), sizeof(float) * (size_t)count));
+    CUDA_TRY(cudaStreamSynchronize(sys->stream));
+    return SPH_OK;
+}
+
 int sph_count(const SphSystem *sys, int64_t *n)
 {
     if (!sys || !n) return fail(SPH_ERR_INVALID, "null argument");

@@ -125,3 +125,18 @@ def test_the_classic_schemes_rows(dim, threads):
     fresh.update(x, m, fluid)
     again = fresh.pairAccelerations(v, rho, C0 ** 2 * (rho - RHO0), C0, 0.05, 0.5, g)
     assert np.array_equal(again, runs[1]['limited'])
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+@pytest.mark.parametrize('n, walls', [(1, 0.0), (1, 1.0), (31, 0.5), (1023, 0.4), (1024, 0.4), (1025, 0.4), (2048, 1.0),
+                                      (2049, 0.0), (70001, 0.3)])
+def test_a_frame_is_the_fluids_rows(n, walls, dim):
+    # the device packs the fluid's rows in the caller's order: the pulled state's rows, rounded
+    from pysurf_b200.state import ParticleState
+    x, v, rho, m, fluid, h = cloud(dim, n, 2, walls=walls)
+    s = pairSums(dim, h, True)
+    s.push(ParticleState(x, v, np.zeros_like(x), rho, np.zeros(n), m, fluid))
+    positions, speeds = s.frame()
+    assert positions.dtype == np.float32 and speeds.dtype == np.float32
+    assert np.array_equal(positions, x[fluid].astype(np.float32))
+    assert np.array_equal(speeds, np.linalg.norm(v[fluid], axis=1).astype(np.float32))

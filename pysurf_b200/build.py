@@ -15,10 +15,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIBRARY = os.path.join(HERE, 'libpysurf_b200.so')
 OBJECTS = os.path.join(HERE, '_build')
-# each unit's source and definitions, compiled side by side; the sweeps once a dimension
-UNITS = [('csrc/sph_sweep_kernels.cu', ['-DSPH_SWEEP_DIM=3']), ('csrc/sph_sweep_kernels.cu', ['-DSPH_SWEEP_DIM=2']),
-         ('csrc/sph_classic_sweeps.cu', []), ('csrc/sph_kernels.cu', []), ('csrc/sph_system.cu', []), ('csrc/sph_noalloc.cu', []),
-         ('csrc/sph_surface.cu', []), ('csrc/sph_merge.cu', [])]
+# each unit's source and definitions, compiled side by side, the longest first; the sweeps once a dimension
+# and kernel
+UNITS = [('csrc/sph_sweep_kernels.cu', [f'-DSPH_SWEEP_DIM={dim}', f'-DSPH_SWEEP_KERNEL={kernel}'])
+         for dim in (3, 2) for kernel in (1, 0)]
+UNITS += [(f'csrc/{name}.cu', []) for name in ('sph_classic_sweeps', 'sph_kernels', 'sph_system', 'sph_noalloc',
+                                               'sph_surface', 'sph_merge')]
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC']
 

@@ -50,7 +50,7 @@ __device__ __forceinline__ float gradient(float q, const KernelAt &k)
 // Visits slot i's neighbours in the walk's order: of those counted (a boundary row's are its fluid
 // neighbours, unless `whole`), lane t of T takes those whose count k has k / 4 = t mod T, from the table's
 // row (all of them from its front; P.together) when it holds them, else from the cells.  The visitor gets
-// (j, d, r, image, pb and kin rows of j) when accept(fluidJ).
+// (j, d, r, whether j is fluid, whether the pair lies across the seam, j's rows) when accept(fluidJ).
 template <int D, int T, class Visitor>
 __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F, int i, int t, bool whole, Visitor &visit)
 {
@@ -90,13 +90,15 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
         float pj[3];
         pointIn<D>(A, pj);
         if (walking && (coarseDistance2<D>(pi, pj, offset) >= limit || j == i)) continue;
-        const float4 B = __ldg(&F.pb[j]);
-        const float4 Kj = Visitor::kKinetic ? __ldg(&F.kin[j]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const bool fluidJ = signedLengthIn<D>(A, B) > 0.0f;
+        NeighbourRows R;
+        R.A = A;
+        R.B = __ldg(&F.pb[j]);
+        if (Visitor::kKinetic || D == 2) R.K = __ldg(&F.kin[j]);
+        const bool fluidJ = signedLengthIn<D>(A, R.B) > 0.0f;
         if (walking && fluidOnly && !fluidJ) continue;     // not in the row: not counted either
         if ((T == 1 || !walking) && !visit.accept(fluidJ)) continue;
         float lj[3], d[3];
-        remainderIn<D>(A, B, lj);
+        remainderIn<D>(A, R.B, lj);
         const float r2 = separation2<D>(P, pi, li, pj, lj, offset, image, O.shift64, d);
         if (walking) {
             if (r2 >= support2(P.hMax)) continue;
@@ -107,7 +109,8 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
         }
         const float r = r2 > 0.0f ? r2 * rsqrtf(r2) : 0.0f;
         if (Visitor::kSkipCoincident && r < 1.0e-12f) continue;
-        visit(j, d, r, fluidJ, image, B, Kj);
+        if (D == 3) R.X = __ldg(&F.aux[j]);
+        visit(j, d, r, fluidJ, image, R);
     }
 }
 
@@ -119,12 +122,11 @@ struct ShepardVisit {
     KernelAt k;
     float num, den;
     __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *, float r, bool, int, const float4 &B, const float4 &)
+    __device__ void operator()(int j, const float *, float r, bool, int, const NeighbourRows &R)
     {
-        const float4 X = auxRow<D>(F, j);
         float w = value<K>(r * k.invH, k);
-        num += massIn<D>(B) * w;
-        den += volumeIn<D>(B, X) * w;
+        num += massIn<D>(R) * w;
+        den += volumeIn<D>(R) * w;
     }
 };
 
@@ -160,11 +162,11 @@ struct MomentumVisit {
     float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0
     float total[3], parts[BUDGET ? 4 : 1][3];
     __device__ bool accept(bool) const { return true; }
-    __device__ void operator()(int j, const float *d, float r, bool fluidJ, int, const float4 &B, const float4 &Kj)
+    __device__ void operator()(int j, const float *d, float r, bool fluidJ, int, const NeighbourRows &R)
     {
         const float h = P.hMax, q = r * k.invH;
         float vj[3];
-        velocityIn<D>(Kj, vj);
+        velocityIn<D>(R.K, vj);
         float rel[3] = {vi[0] - vj[0], vi[1] - vj[1], vi[2] - vj[2]};
         float approach = rel[0] * d[0] + rel[1] * d[1] + (D == 3 ? rel[2] * d[2] : 0.0f);
         float viscosity = 0.0f;
@@ -172,16 +174,16 @@ struct MomentumVisit {
             // -alpha c0 h (v_ij . r_ij) / ((r^2 + 0.01 h^2) (rho_i + rho_j) / 2); the denominator is
             // a positive normal float for any physical pair, which __fdividef takes to 2 ulp
             viscosity = __fdividef(viscosityScale * h * approach,
-                                   (r * r + k.soft) * (0.5f * (rhoI + densityIn<D>(Kj))));
+                                   (r * r + k.soft) * (0.5f * (rhoI + densityIn<D>(R))));
             if (!fluidJ) viscosity *= P.boundaryFactor;
         }
-        const float ratioJ = D == 2 ? Kj.w : auxRow<D>(F, j).x;
+        const float ratioJ = pressureRatioIn<D>(R);
         const float pressureTerm = __fadd_rn(own, ratioJ);
-        float coefficient = -__fadd_rn(pressureTerm, viscosity) * massIn<D>(B);
+        float coefficient = -__fadd_rn(pressureTerm, viscosity) * massIn<D>(R);
         float f = coefficient * gradient<K>(q, k);
         for (int a = 0; a < D; ++a) total[a] = __fmaf_rn(f, d[a], total[a]);
         if constexpr (BUDGET) {
-            const float grad = massIn<D>(B) * gradient<K>(q, k);
+            const float grad = massIn<D>(R) * gradient<K>(q, k);
             const float fp = -pressureTerm * grad, fv = -viscosity * grad;
             if (fluidJ) {
                 for (int a = 0; a < D; ++a) { parts[0][a] += fp * d[a]; parts[1][a] += fv * d[a]; }
@@ -242,19 +244,18 @@ struct ContinuityVisit {
     double cross;           // the fluid-boundary pairs' terms in float64
     float plainFluid, plainWall;    // BUDGET
     __device__ bool accept(bool fluidJ) const { return !(boundaryI && !fluidJ); }
-    __device__ void operator()(int j, const float *d, float r, bool fluidJ, int image, const float4 &B, const float4 &Kj)
+    __device__ void operator()(int j, const float *d, float r, bool fluidJ, int image, const NeighbourRows &R)
     {
         float vj[3];
-        velocityIn<D>(Kj, vj);
+        velocityIn<D>(R.K, vj);
         const float4 lowJ = __ldg(&F.low[j]);
         const float vlJ[3] = {lowJ.x, lowJ.y, lowJ.z};
         if (boundaryI == fluidJ) {
-            const float4 A = __ldg(&F.pa[j]);
             float pi[3], li[3], pj[3], lj[3];
             pointOf<D>(F, self, pi);
             remainderOf<D>(F, self, li);
-            pointIn<D>(A, pj);
-            remainderIn<D>(A, B, lj);
+            pointIn<D>(R.A, pj);
+            remainderIn<D>(R.A, R.B, lj);
             double dd[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
             for (int a = 0; a < D; ++a) {
                 dd[a] = ((double)pi[a] - (double)pj[a]) + ((double)li[a] - (double)lj[a]);
@@ -266,7 +267,7 @@ struct ContinuityVisit {
             double dot = 0.0;
             for (int a = 0; a < D; ++a)
                 dot = fma(((double)vi[a] + (double)vlI[a]) - ((double)vj[a] + (double)vlJ[a]), dd[a], dot);
-            const double term = (double)massIn<D>(B) * dot * grad;
+            const double term = (double)massIn<D>(R) * dot * grad;
             cross += term;
             if constexpr (BUDGET) {
                 if (fluidJ) plainFluid += (float)term;
@@ -280,7 +281,7 @@ struct ContinuityVisit {
             dv[a] = __fadd_rn(__fsub_rn(vi[a], vj[a]), __fsub_rn(vlI[a], vlJ[a]));
         float dot = 0.0f;
         for (int a = 0; a < D; ++a) dot += dv[a] * d[a];
-        const float massDot = massIn<D>(B) * dot;
+        const float massDot = massIn<D>(R) * dot;
         total = __fmaf_rn(massDot, grad, total);
         if constexpr (BUDGET) plainFluid = __fmaf_rn(massDot, grad, plainFluid);
     }
@@ -331,13 +332,13 @@ struct XsphVisit {
     KernelAt k;
     float vi[3], rhoI, corr[3];
     __device__ bool accept(bool fluidJ) const { return fluidJ; }
-    __device__ void operator()(int j, const float *, float r, bool, int, const float4 &B, const float4 &Kj)
+    __device__ void operator()(int j, const float *, float r, bool, int, const NeighbourRows &R)
     {
         float w = value<K>(r * k.invH, k);
-        float rhoJ = densities ? densities[j] : densityIn<D>(Kj);
-        float weight = massIn<D>(B) * w / (0.5f * (rhoI + rhoJ));
+        float rhoJ = densities ? densities[j] : densityIn<D>(R);
+        float weight = massIn<D>(R) * w / (0.5f * (rhoI + rhoJ));
         float vj[3];
-        velocityIn<D>(Kj, vj);
+        velocityIn<D>(R.K, vj);
         for (int a = 0; a < D; ++a) corr[a] += weight * (vj[a] - vi[a]);
     }
 };

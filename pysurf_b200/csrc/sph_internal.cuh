@@ -7,11 +7,14 @@
 //     m, h (float64), fluid (uint8), orig (int32: the caller's index of the slot)
 //   the sweeps' float32 frame, rebuilt from the master each step:
 //     pa   float4  2D (hx, hy, lx, ly)      3D (hx, hy, hz, hs)
-//     pb   float4  2D (m, hs, dev, V)       3D (lx, ly, lz, m)
-//     kin  float4  2D (vx, vy, rho, P2)     3D (vx, vy, vz, rho)
-//     aux  float4  3D (P2, dev, V, -)
-//     low  float4  (vlx, vly, vlz, devLo): the float32 remainders of the float64 velocity and deviation
+//     pb   float4  2D (m, hs, P2, rho)      3D (lx, ly, lz, V)
+//     kin  float4  2D (vx, vy, V, dev)      3D (vx, vy, vz, dev)
+//     aux  float4  3D (P2, rho, m, -)
+//     low  float4  (vlx, vly, 2D m, 3D vlz, devLo): the float32 remainders of the float64 velocity and
+//                  deviation
 //     pres float   the pressure p
+//   The rows lie so that each sweep reads few: gradients pa, kin (3D pb too); momentum pa, pb, kin (3D aux
+//   too); continuity pa, kin, low (3D pb and m alone).
 //   hi + lo is each float64 coordinate split into a float32 point and its float32 remainder, so a
 //   separation (hi_i - hi_j) + (lo_i - lo_j) keeps the float64 positions' digits without float64
 //   arithmetic (src/pysurf/sphGpu.py:227-242 states the same split).  hs is +h for a fluid
@@ -40,6 +43,7 @@ constexpr float kViscositySoftening = 0.01f;   // mu_ij's r^2 + 0.01 h^2 (src/py
 constexpr float kCloseDistance = 0.3f;      // limiter fade (src/pysurf/sphSolver.py:220-221)
 constexpr float kFoldWidth = 0.2f;
 constexpr float kCandidateMargin = 1.0001f; // on r^2, as the reference's coarse test (src/pysurf/sphGpu.py:99)
+
 
 // Error flags the device raises; the host reads them after each call that syncs.
 enum DeviceError : int {
@@ -406,46 +410,34 @@ template <int D> __device__ __forceinline__ float signedLength(const Frame &F, i
 template <> __device__ __forceinline__ float signedLength<2>(const Frame &F, int j) { return __ldg(&F.pb[j].y); }
 template <> __device__ __forceinline__ float signedLength<3>(const Frame &F, int j) { return __ldg(&F.pa[j].w); }
 
-template <int D> __device__ __forceinline__ float massOf(const Frame &F, int j);
-template <> __device__ __forceinline__ float massOf<2>(const Frame &F, int j) { return __ldg(&F.pb[j].x); }
-template <> __device__ __forceinline__ float massOf<3>(const Frame &F, int j) { return __ldg(&F.pb[j].w); }
-
+// A slot's own fields.
+template <int D> __device__ __forceinline__ float massOf(const Frame &F, int j)
+{ return D == 2 ? __ldg(&F.pb[j].x) : __ldg(&F.aux[j].z); }
 template <int D> __device__ __forceinline__ float pressureOf(const Frame &F, int j) { return __ldg(&F.pres[j]); }
-
 // p / rho^2
-template <int D> __device__ __forceinline__ float pressureRatioOf(const Frame &F, int j);
-template <> __device__ __forceinline__ float pressureRatioOf<2>(const Frame &F, int j) { return __ldg(&F.kin[j].w); }
-template <> __device__ __forceinline__ float pressureRatioOf<3>(const Frame &F, int j) { return __ldg(&F.aux[j].x); }
-
-template <int D> __device__ __forceinline__ float deviationOf(const Frame &F, int j);
-template <> __device__ __forceinline__ float deviationOf<2>(const Frame &F, int j) { return __ldg(&F.pb[j].z); }
-template <> __device__ __forceinline__ float deviationOf<3>(const Frame &F, int j) { return __ldg(&F.aux[j].y); }
-
+template <int D> __device__ __forceinline__ float pressureRatioOf(const Frame &F, int j)
+{ return D == 2 ? __ldg(&F.pb[j].z) : __ldg(&F.aux[j].x); }
+template <int D> __device__ __forceinline__ float deviationOf(const Frame &F, int j) { return __ldg(&F.kin[j].w); }
 // m / rho
-template <int D> __device__ __forceinline__ float volumeOf(const Frame &F, int j);
-template <> __device__ __forceinline__ float volumeOf<2>(const Frame &F, int j) { return __ldg(&F.pb[j].w); }
-template <> __device__ __forceinline__ float volumeOf<3>(const Frame &F, int j) { return __ldg(&F.aux[j].z); }
+template <int D> __device__ __forceinline__ float volumeOf(const Frame &F, int j)
+{ return D == 2 ? __ldg(&F.kin[j].z) : __ldg(&F.pb[j].w); }
+template <int D> __device__ __forceinline__ float densityOf(const Frame &F, int j)
+{ return D == 2 ? __ldg(&F.pb[j].w) : __ldg(&F.aux[j].y); }
 
-template <int D> __device__ __forceinline__ float densityOf(const Frame &F, int j);
-template <> __device__ __forceinline__ float densityOf<2>(const Frame &F, int j) { return __ldg(&F.kin[j].z); }
-template <> __device__ __forceinline__ float densityOf<3>(const Frame &F, int j) { return __ldg(&F.kin[j].w); }
-
-// A neighbour's values from its rows, each row loaded once a pair: pa (A), pb (B), kin (K) and, in
-// 3D, aux (X).
-template <int D> __device__ __forceinline__ float4 auxRow(const Frame &F, int j)
-{
-    return D == 3 ? __ldg(&F.aux[j]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-}
+// A neighbour's rows, and its fields from them: pa (A), pb (B), kin (K), aux (X, 3D), low (L), and its mass
+// where a sweep reads it apart from them.
+struct NeighbourRows {
+    float4 A, B, K, X, L;
+    float m;
+};
 template <int D> __device__ __forceinline__ float signedLengthIn(const float4 &A, const float4 &B)
 { return D == 2 ? B.y : A.w; }
-template <int D> __device__ __forceinline__ float massIn(const float4 &B) { return D == 2 ? B.x : B.w; }
-template <int D> __device__ __forceinline__ float volumeIn(const float4 &B, const float4 &X)
-{ return D == 2 ? B.w : X.z; }
-template <int D> __device__ __forceinline__ float deviationIn(const float4 &B, const float4 &X)
-{ return D == 2 ? B.z : X.y; }
-template <int D> __device__ __forceinline__ float densityIn(const float4 &K) { return D == 2 ? K.z : K.w; }
-template <int D> __device__ __forceinline__ float pressureRatioIn(const float4 &K, const float4 &X)
-{ return D == 2 ? K.w : X.x; }
+template <int D> __device__ __forceinline__ float massIn(const NeighbourRows &R) { return D == 2 ? R.B.x : R.X.z; }
+template <int D> __device__ __forceinline__ float volumeIn(const NeighbourRows &R) { return D == 2 ? R.K.z : R.B.w; }
+template <int D> __device__ __forceinline__ float deviationIn(const NeighbourRows &R) { return R.K.w; }
+template <int D> __device__ __forceinline__ float densityIn(const NeighbourRows &R) { return D == 2 ? R.B.w : R.X.y; }
+template <int D> __device__ __forceinline__ float pressureRatioIn(const NeighbourRows &R)
+{ return D == 2 ? R.B.z : R.X.x; }
 template <int D> __device__ __forceinline__ void pointIn(const float4 &A, float p[3])
 {
     p[0] = A.x; p[1] = A.y; p[2] = D == 3 ? A.z : 0.0f;
@@ -469,12 +461,13 @@ __device__ __forceinline__ void storeDensity(const Frame &F, int i, float m, dou
     const float volume = m / rho, ratio = p / (rho * rho);
     F.pres[i] = p;
     F.low[i].w = (float)(dev64 - (double)dev);
+    F.kin[i].w = dev;
     if (D == 2) {
-        F.kin[i].z = rho; F.kin[i].w = ratio;
-        F.pb[i].z = dev; F.pb[i].w = volume;
+        F.pb[i].z = ratio; F.pb[i].w = rho;
+        F.kin[i].z = volume;
     } else {
-        F.kin[i].w = rho;
-        F.aux[i] = make_float4(ratio, dev, volume, 0.0f);
+        F.pb[i].w = volume;
+        F.aux[i].x = ratio; F.aux[i].y = rho;
     }
 }
 

@@ -210,16 +210,16 @@ __global__ void gatherKernel(Params P, int n, const int *perm, MasterView from, 
         vl[a] = (float)(v[a] - (double)vf[a]);
     }
     F.pres[s] = p;
-    F.low[s] = make_float4(vl[0], vl[1], vl[2], (float)(dev64 - (double)dev));
+    F.low[s] = make_float4(vl[0], vl[1], P.dim == 2 ? m : vl[2], (float)(dev64 - (double)dev));
     if (P.dim == 2) {
         F.pa[s] = make_float4(hi[0], hi[1], lo[0], lo[1]);
-        F.pb[s] = make_float4(m, hs, dev, volume);
-        F.kin[s] = make_float4(vf[0], vf[1], rhoF, ratio);
+        F.pb[s] = make_float4(m, hs, ratio, rhoF);
+        F.kin[s] = make_float4(vf[0], vf[1], volume, dev);
     } else {
         F.pa[s] = make_float4(hi[0], hi[1], hi[2], hs);
-        F.pb[s] = make_float4(lo[0], lo[1], lo[2], m);
-        F.kin[s] = make_float4(vf[0], vf[1], vf[2], rhoF);
-        F.aux[s] = make_float4(ratio, dev, volume, 0.0f);
+        F.pb[s] = make_float4(lo[0], lo[1], lo[2], volume);
+        F.kin[s] = make_float4(vf[0], vf[1], vf[2], dev);
+        F.aux[s] = make_float4(ratio, rhoF, m, 0.0f);
     }
 }
 
@@ -247,29 +247,26 @@ __global__ void loadFieldsKernel(Params P, int n, const int *orig, const double 
     }
     float p = pressures ? (float)pressures[o] : F.pres[s];
     F.pres[s] = p;
+    float4 b = F.pb[s], x = F.aux[s];
+    float rho = P.dim == 2 ? b.w : x.y;
+    if (densities) {
+        const double dev = densities[o] - deviationReference;
+        rho = (float)densities[o];
+        k.w = (float)dev;
+        low.w = (float)(dev - (double)k.w);
+    }
+    const float m = P.dim == 2 ? b.x : x.z, volume = m / rho, ratio = p / (rho * rho);
     if (P.dim == 2) {
-        float4 b = F.pb[s];
-        if (densities) {
-            const double dev = densities[o] - deviationReference;
-            k.z = (float)densities[o];
-            b.z = (float)dev;
-            low.w = (float)(dev - (double)b.z);
-        }
-        b.w = b.x / k.z;
-        k.w = p / (k.z * k.z);
-        F.pb[s] = b;
+        b.z = ratio;
+        b.w = rho;
+        k.z = volume;
     } else {
-        float4 x = F.aux[s];
-        if (densities) {
-            const double dev = densities[o] - deviationReference;
-            k.w = (float)densities[o];
-            x.y = (float)dev;
-            low.w = (float)(dev - (double)x.y);
-        }
-        x.z = F.pb[s].w / k.w;
-        x.x = p / (k.w * k.w);
+        b.w = volume;
+        x.x = ratio;
+        x.y = rho;
         F.aux[s] = x;
     }
+    F.pb[s] = b;
     F.kin[s] = k;
     F.low[s] = low;
 }

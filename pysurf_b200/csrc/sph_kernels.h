@@ -52,10 +52,13 @@ struct LaunchArgs {
     int *maxCount;          // List: the largest neighbour count goes here (atomic max), when given
 };
 
-// The stages of a 2D and a 3D system (sph_sweep_kernels.cu), and of the classic scheme, where it has its
-// own (sph_classic_sweeps.cu; false where it has none).
-void launchStage2(const LaunchArgs &A, Stage stage);
-void launchStage3(const LaunchArgs &A, Stage stage);
+// The stages of a 2D or a 3D system with the cubic spline (0) or the Wendland kernel (1)
+// (sph_sweep_kernels.cu; the Wendland units build the table for both), and of the classic scheme, where it
+// has its own (sph_classic_sweeps.cu; false where it has none).
+void launchStage2_0(const LaunchArgs &A, Stage stage);
+void launchStage2_1(const LaunchArgs &A, Stage stage);
+void launchStage3_0(const LaunchArgs &A, Stage stage);
+void launchStage3_1(const LaunchArgs &A, Stage stage);
 bool launchClassicStage(const LaunchArgs &A, Stage stage);
 inline void launchStage(const LaunchArgs &A, Stage stage)
 {
@@ -64,8 +67,9 @@ inline void launchStage(const LaunchArgs &A, Stage stage)
         if (launchClassicStage(A, stage)) return;
         if (stage != Stage::List) B.P.listCap = 0;      // the paired sweeps' rows part the kinds: walk the cells
     }
-    if (A.P.dim == 2) launchStage2(B, stage);
-    else launchStage3(B, stage);
+    const bool wendland = A.P.kind == 1 || stage == Stage::List;
+    if (A.P.dim == 2) wendland ? launchStage2_1(B, stage) : launchStage2_0(B, stage);
+    else wendland ? launchStage3_1(B, stage) : launchStage3_0(B, stage);
 }
 
 // A merge of split particles (sph_merge.cu): the current master and the buffer it moves into, with

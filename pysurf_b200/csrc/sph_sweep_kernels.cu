@@ -232,9 +232,9 @@ struct alignas(16) BatchMember {
     int walls;          // its boundary neighbours so far
 };
 
-// No blocks-a-multiprocessor bound: at the compiler's default the kernel keeps about 24 warps an
-// SM with a few spills, faster than 85-116 registers and no spills at 3 to 6 blocks, or 64
-// registers at 8 (measured).
+// No blocks-a-multiprocessor bound: the compiler's own choice, 64 registers with a few spills at one
+// smoothing length, builds the 20-ppd ridge's table in 20.4 ms, against 22.1 to 23.8 at bounds of 7 to 9
+// blocks that spill none.
 template <int D, int kBatch, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
@@ -454,16 +454,15 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
 template <int D, int K, bool FINE>
 struct ShepardVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = true, kKinetic = D == 2, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = false;
-    static constexpr bool kAuxRow = D == 3;
     Smoothing<K, D, FINE> S;
     float num, den;
     __device__ void operator()(int, const float *, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
         const float w = kernelValue<K>(__fmul_rn(r, k.invH), k);
-        num = __fmaf_rn(massIn<D>(R.B), w, num);
-        den = __fmaf_rn(volumeIn<D>(R.B, R.X), w, den);
+        num = __fmaf_rn(massIn<D>(R), w, num);
+        den = __fmaf_rn(volumeIn<D>(R), w, den);
     }
 };
 
@@ -515,8 +514,8 @@ __global__ void applyShepardKernel(Params P, Frame F, const Control *ctl)
 template <int D, int K, bool FINE>
 struct WallVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = true, kKinetic = false, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = true;
     const Params &P; const Frame &F;
     Smoothing<K, D, FINE> S;
     float weight, total;
@@ -526,7 +525,7 @@ struct WallVisit {
         float gd = __fmaf_rn(P.g[1], d[1], __fmul_rn(P.g[0], d[0]));
         if (D == 3) gd = __fmaf_rn(P.g[2], d[2], gd);
         weight = __fadd_rn(weight, w);
-        total = __fmaf_rn(w, __fmaf_rn(densityIn<D>(R.K), gd, pressureOf<D>(F, j)), total);
+        total = __fmaf_rn(w, __fmaf_rn(densityIn<D>(R), gd, pressureOf<D>(F, j)), total);
     }
 };
 
@@ -558,7 +557,7 @@ wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
     // the density stays; the pressure and p / rho^2 take p_w
     const float rho = densityOf<D>(F, i), ratio = p / (rho * rho);
     F.pres[i] = p;
-    if (D == 2) F.kin[i].w = ratio;
+    if (D == 2) F.pb[i].z = ratio;
     else F.aux[i].x = ratio;
 }
 
@@ -572,19 +571,18 @@ wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
 template <int D>
 __device__ __forceinline__ constexpr int packed(int a, int b) { return a * D - a * (a - 1) / 2 + (b - a); }
 
-template <int D, int K, bool FINE>
+template <int D, int K, bool FINE, bool RHO>
 struct GradientVisit {
     static constexpr bool kCopied = D == 3 && !FINE;
+    static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kAuxRow = D == 3;
-    static constexpr bool kKinetic = true;
     Smoothing<K, D, FINE> S;
-    bool wantG, wantL, wantRho;
+    bool wantG, wantL;
     float vi[3], devI;
     // each lane's sums over its even and its odd neighbours: V (v_j - v_i) grad W, and M over the fluid
     // (its upper triangle, packed)
-    float2 jump[D][D], Mf[D * (D + 1) / 2], gsum[D];
+    float2 jump[D][D], Mf[D * (D + 1) / 2], gsum[RHO ? D : 1];   // gsum: RHO, the density gradient's sum
     double M[D * (D + 1) / 2];
     struct Taken {
         float volume[2];
@@ -594,14 +592,14 @@ struct GradientVisit {
     __device__ __forceinline__ Taken take(const Neighbours &, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
         Taken t;
-        t.volume[0] = volumeIn<D>(R0.B, R0.X);
-        t.volume[1] = volumeIn<D>(R1.B, R1.X);
+        t.volume[0] = volumeIn<D>(R0);
+        t.volume[1] = volumeIn<D>(R1);
         float vj0[3], vj1[3];
         velocityIn<D>(R0.K, vj0);
         velocityIn<D>(R1.K, vj1);
         if (KIND == kFluidPair)
             for (int a = 0; a < D; ++a) t.rel[a] = make_float2(__fsub_rn(vj0[a], vi[a]), __fsub_rn(vj1[a], vi[a]));
-        t.difference = make_float2(__fsub_rn(deviationIn<D>(R0.B, R0.X), devI), __fsub_rn(deviationIn<D>(R1.B, R1.X), devI));
+        t.difference = make_float2(__fsub_rn(deviationIn<D>(R0), devI), __fsub_rn(deviationIn<D>(R1), devI));
         return t;
     }
     template <PairKind KIND>
@@ -638,9 +636,9 @@ struct GradientVisit {
                 for (int b = a; b < D; ++b) Mf[packed<D>(a, b)] = fma2(wa, N.d[b], Mf[packed<D>(a, b)]);
             }
         }
-        if (wantRho) {
+        if (RHO) {
             const float2 t = mul2(w, taken.difference);
-            for (int a = 0; a < D; ++a) gsum[a] = fma2(t, N.d[a], gsum[a]);
+            for (int a = 0; a < D; ++a) gsum[RHO ? a : 0] = fma2(t, N.d[a], gsum[RHO ? a : 0]);
         }
     }
 };
@@ -652,9 +650,9 @@ __device__ __forceinline__ float groupSum(const float2 &value, unsigned mask)
     return groupSum<T>(__fadd_rn(value.x, value.y), mask);
 }
 
-template <int D, int K, int T, bool FINE>
+template <int D, int K, int T, bool FINE, bool RHO>
 __global__ void __launch_bounds__(kBlock, gradientMinBlocks<D>())
-gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int wantRho, float floorDet)
+gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, float floorDet)
 {
     if (ctl && !ctl->active) return;
     const Group<T> G = groupOf<T>();
@@ -667,14 +665,14 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
         float ident[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
         if (wantG == kWholeGradients) storeMatrix<D>(F.G0, F.G1, F.G2, i, zero);
         if (wantL) storeMatrix<D>(F.L0, F.L1, F.L2, i, ident);
-        if (wantRho) F.gradRho[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (RHO) F.gradRho[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
-    GradientVisit<D, K, FINE> visit{Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || wantRho != 0, wantRho != 0};
+    GradientVisit<D, K, FINE, RHO> visit{Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || RHO};
     velocityOf<D>(F, i, visit.vi);
     visit.devI = deviationOf<D>(F, i);
     for (int a = 0; a < D; ++a) {
-        visit.gsum[a] = both(0.0f);
+        visit.gsum[RHO ? a : 0] = both(0.0f);
         for (int b = 0; b < D; ++b) visit.jump[a][b] = both(0.0f);
     }
     for (int q = 0; q < D * (D + 1) / 2; ++q) { visit.M[q] = 0.0; visit.Mf[q] = both(0.0f); }
@@ -689,11 +687,11 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
         }
     }
     double M[3][3] = {{1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
-    if (wantL || wantRho)
+    if (wantL || RHO)
         for (int a = 0; a < D; ++a)
             for (int b = a; b < D; ++b) M[a][b] = M[b][a] = groupSum<T>(visit.M[packed<D>(a, b)], G.mask);
-    if (wantRho)
-        for (int a = 0; a < D; ++a) gsum[a] = groupSum<T>(visit.gsum[a], G.mask);
+    if (RHO)
+        for (int a = 0; a < D; ++a) gsum[a] = groupSum<T>(visit.gsum[RHO ? a : 0], G.mask);
     if (G.t != 0) return;
     if (wantG) {
         float Gm[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -711,7 +709,7 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
         if (wantG == kWholeGradients) storeMatrix<D>(F.G0, F.G1, F.G2, i, Gm);
         else storeSlopes<D>(F, i, Gm);
     }
-    if (wantL || wantRho) {
+    if (wantL || RHO) {
         // L = M^-1 in float64, rounded once
         float L[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
         if (determinant<D>(M) >= (double)floorDet) {
@@ -721,7 +719,7 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
                 for (int b = 0; b < D; ++b) L[a][b] = (float)inv[a][b];
         }
         if (wantL) storeMatrix<D>(F.L0, F.L1, F.L2, i, L);
-        if (wantRho) {
+        if (RHO) {
             float g[3] = {0.0f, 0.0f, 0.0f};
             for (int a = 0; a < D; ++a)
                 for (int b = 0; b < D; ++b) g[a] += L[a][b] * gsum[b];
@@ -737,13 +735,12 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, int 
 // BUDGET: the sum split for the energy budget too, into the pressure and the viscosity of fluid
 // and of boundary neighbours (src/pysurf/sphGpu.py:400-414).  COMP: the sum compensated (Dot2),
 // its running error in comp.
-template <int D, int K, bool BUDGET, bool FINE, bool COMP = false>
+template <int D, int K, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 struct MomentumVisit {
-    static constexpr bool kCopied = D == 2 || FINE;
+    static constexpr bool kCopied = false;
+    static constexpr bool kBody = true, kKinetic = true, kAux = true, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kAuxRow = D == 3;
-    static constexpr bool kKinetic = true;
     const Params &P; const Frame &F;
     Smoothing<K, D, FINE> S;
     float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0
@@ -774,13 +771,13 @@ struct MomentumVisit {
             if (t.plain.x < 0.0f) loadSlopes<D>(F, N.j[0], t.s0);
             if (t.plain.y < 0.0f) loadSlopes<D>(F, N.j[1], t.s1);
         }
-        t.rho[0] = densityIn<D>(R0.K);
-        t.rho[1] = densityIn<D>(R1.K);
+        t.rho[0] = densityIn<D>(R0);
+        t.rho[1] = densityIn<D>(R1);
         t.density = make_float2(__fadd_rn(rhoI, t.rho[0]), __fadd_rn(rhoI, t.rho[1]));
-        t.pressure = make_float2(__fadd_rn(own, pressureRatioIn<D>(R0.K, R0.X)),
-                                 __fadd_rn(own, pressureRatioIn<D>(R1.K, R1.X)));
-        t.mass[0] = massIn<D>(R0.B);
-        t.mass[1] = massIn<D>(R1.B);
+        t.pressure = make_float2(__fadd_rn(own, pressureRatioIn<D>(R0)),
+                                 __fadd_rn(own, pressureRatioIn<D>(R1)));
+        t.mass[0] = massIn<D>(R0);
+        t.mass[1] = massIn<D>(R1);
         return t;
     }
     template <PairKind KIND>
@@ -830,7 +827,7 @@ struct MomentumVisit {
         const float2 below = mul2(fma2(N.r, N.r, N.k.soft), mean);
         float2 viscosity = make_float2(quickDivide(above.x, below.x), quickDivide(above.y, below.y));
         if (KIND == kWallPair) viscosity = mul2(viscosity, both(P.boundaryFactor));
-        if (KIND == kFluidPair && P.closure) {
+        if (KIND == kFluidPair && CLOSURE && P.closure) {
             if (N.live[0])
                 viscosity.x = __fadd_rn(viscosity.x, closureTerm(N.j[0], N.h.x, N.r.x, plain.x, taken.rho[0]));
             if (N.live[1])
@@ -876,7 +873,7 @@ struct MomentumVisit {
 
 // maxima: fold the fluid maxima into ctl and take the time step (the device steps); 0 for the
 // host-step sums.
-template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP = false>
+template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 __global__ void __launch_bounds__(kBlock, BUDGET ? budgetMinBlocks<D>() : sweepMinBlocks<D>())
 momentumKernel(Params P, Frame F, Control *ctl, int maxima)
 {
@@ -889,12 +886,12 @@ momentumKernel(Params P, Frame F, Control *ctl, int maxima)
         if (hs <= 0.0f) {
             if (G.t == 0) F.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         } else {
-            MomentumVisit<D, K, BUDGET, FINE, COMP> visit{P, F, Smoothing<K, D, FINE>(P, hs)};
+            MomentumVisit<D, K, BUDGET, FINE, COMP, CLOSURE> visit{P, F, Smoothing<K, D, FINE>(P, hs)};
             velocityOf<D>(F, i, visit.vi);
             visit.rhoI = densityOf<D>(F, i);
             visit.own = pressureRatioOf<D>(F, i);
             visit.viscosityScale = -P.alpha * P.c0;
-            visit.alphaI = P.closure ? F.eddy[i].x : 0.0f;
+            visit.alphaI = CLOSURE && P.closure ? F.eddy[i].x : 0.0f;
             if (P.limited) loadSlopes<D>(F, i, visit.slopeI);
             for (int a = 0; a < D; ++a) visit.total[a] = both(0.0f);
             if constexpr (COMP) for (int a = 0; a < D; ++a) visit.comp[a] = both(0.0f);
@@ -1006,14 +1003,12 @@ __global__ void kickKernel(Params P, Frame F, Control *ctl)
 // and a boundary particle -- every pair of a boundary row, the wall's pairs of a fluid row -- take
 // their separation, distance, kernel gradient and term in float64, summed apart in float64 (cross).
 // Fluid pairs, whose velocity differences are small, keep float32 arithmetic.
-template <int D, int K, bool BUDGET, bool FINE, bool COMP = false>
+template <int D, int K, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 struct ContinuityVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = true, kMass = true;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kAuxRow = D == 3;
-    static constexpr bool kLowRow = true;
-    static constexpr bool kKinetic = true;
     const Params &P; const Frame &F;
     Smoothing<K, D, FINE> S;
     bool diffuses, corrected;
@@ -1054,7 +1049,7 @@ struct ContinuityVisit {
                     if (a == 1 && N.image[q]) t.dd[q][a] += x[1] < 0.5 * P.period ? P.period : -P.period;
                     t.dv[q][a] = v[a] - ((double)(q ? vj1[a] : vj0[a]) + (double)(q ? vl1[a] : vl0[a]));
                 }
-                t.mass[q] = massIn<D>(R.B);
+                t.mass[q] = R.m;
             }
             return t;
         } else {
@@ -1062,10 +1057,10 @@ struct ContinuityVisit {
             for (int a = 0; a < D; ++a)
                 t.dv[a] = add2(make_float2(__fsub_rn(vi[a], vj0[a]), __fsub_rn(vi[a], vj1[a])),
                                make_float2(__fsub_rn(vlI[a], vl0[a]), __fsub_rn(vlI[a], vl1[a])));
-            t.mass[0] = massIn<D>(R0.B);
-            t.mass[1] = massIn<D>(R1.B);
-            t.volume = make_float2(N.live[0] ? volumeIn<D>(R0.B, R0.X) : 0.0f, N.live[1] ? volumeIn<D>(R1.B, R1.X) : 0.0f);
-            t.devJ = make_float2(deviationIn<D>(R0.B, R0.X), deviationIn<D>(R1.B, R1.X));
+            t.mass[0] = R0.m;
+            t.mass[1] = R1.m;
+            t.volume = make_float2(N.live[0] ? volumeIn<D>(R0) : 0.0f, N.live[1] ? volumeIn<D>(R1) : 0.0f);
+            t.devJ = make_float2(deviationIn<D>(R0), deviationIn<D>(R1));
             // rho_j - rho_i from the float32 deviations and their remainders, so it keeps float64's
             // digits (the leading difference is exact for neighbours' nearly equal deviations)
             t.leading = make_float2(__fsub_rn(t.devJ.x, devI), __fsub_rn(t.devJ.y, devI));
@@ -1143,7 +1138,7 @@ struct ContinuityVisit {
             // 2 delta c0 h V_j (difference) (-(dW/dr) r) / (r^2 + 0.01 h^2), with (dW/dr) r = grad r^2;
             // with the closure, 2 delta c0 is 2 c0 times the harmonic mean of the two deltas
             float2 factor = both(P.diffusionFactor);
-            if (P.closure) factor = make_float2(pairFactor(N.j[0]), pairFactor(N.j[1]));
+            if (CLOSURE && P.closure) factor = make_float2(pairFactor(N.j[0]), pairFactor(N.j[1]));
             const float2 volume = taken.volume;
             const float2 r2 = mul2(N.r, N.r), below = add2(r2, N.k.soft);
             const float2 head = mul2(mul2(mul2(mul2(factor, N.h), volume), difference), mul2(both(-1.0f), grad));
@@ -1192,7 +1187,7 @@ struct ContinuityVisit {
 };
 
 // mode 0: the rate only; 1: advance the density; 2: advance, drift and enforce.
-template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP = false>
+template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 __global__ void __launch_bounds__(kBlock, BUDGET ? budgetMinBlocks<D>() : preciseMinBlocks<D>())
 continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
 {
@@ -1201,7 +1196,7 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
     const int i = G.i;
     if (i >= P.n) return;
     float hs = signedLength<D>(F, i);
-    ContinuityVisit<D, K, BUDGET, FINE, COMP> visit{P, F, Smoothing<K, D, FINE>(P, fabsf(hs))};
+    ContinuityVisit<D, K, BUDGET, FINE, COMP, CLOSURE> visit{P, F, Smoothing<K, D, FINE>(P, fabsf(hs))};
     const bool boundary = hs <= 0.0f;
     visit.diffuses = P.diffusion != 0 && !boundary;
     visit.corrected = P.corrected && !boundary;
@@ -1210,7 +1205,7 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
     visit.vlI[0] = lowI.x; visit.vlI[1] = lowI.y; visit.vlI[2] = lowI.z;
     visit.devLoI = lowI.w;
     visit.devI = deviationOf<D>(F, i);
-    visit.deltaI = P.closure && visit.diffuses ? F.eddy[i].y : 0.0f;
+    visit.deltaI = CLOSURE && P.closure && visit.diffuses ? F.eddy[i].y : 0.0f;
     if (visit.corrected) loadMatrix<D>(F.L0, F.L1, F.L2, i, visit.Li);
     visit.gi[0] = visit.gi[1] = visit.gi[2] = 0.0f;
     if (visit.diffuses && P.diffusion == 3) {
@@ -1274,16 +1269,16 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
 template <int D, int K, bool FINE>
 struct XsphVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = true, kKinetic = true, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = true;
     const float *densities;
     Smoothing<K, D, FINE> S;
     float vi[3], rhoI, corr[3];
     __device__ void operator()(int j, const float *, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
         const float w = kernelValue<K>(__fmul_rn(r, k.invH), k);
-        const float rhoJ = densities ? densities[j] : densityIn<D>(R.K);
-        const float weight = __fdiv_rn(__fmul_rn(massIn<D>(R.B), w), __fmul_rn(0.5f, __fadd_rn(rhoI, rhoJ)));
+        const float rhoJ = densities ? densities[j] : densityIn<D>(R);
+        const float weight = __fdiv_rn(__fmul_rn(massIn<D>(R), w), __fmul_rn(0.5f, __fadd_rn(rhoI, rhoJ)));
         float vj[3];
         velocityIn<D>(R.K, vj);
         for (int a = 0; a < D; ++a) corr[a] = __fmaf_rn(weight, __fsub_rn(vj[a], vi[a]), corr[a]);
@@ -1344,10 +1339,9 @@ __global__ void frameDensityKernel(Params P, Frame F, const Control *ctl)
 template <int D, int K>
 struct ShiftFieldsVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kKinetic = false;
-    static constexpr bool kAuxRow = D == 3;
     const Params &P;
     Smoothing<K, D, false> S;
     float devI;
@@ -1359,8 +1353,8 @@ struct ShiftFieldsVisit {
     template <PairKind KIND>
     __device__ __forceinline__ Taken take(const Neighbours &, const NeighbourRows &R0, const NeighbourRows &R1) const
     {
-        return Taken{{volumeIn<D>(R0.B, R0.X), volumeIn<D>(R1.B, R1.X)},
-                     make_float2(__fsub_rn(deviationIn<D>(R0.B, R0.X), devI), __fsub_rn(deviationIn<D>(R1.B, R1.X), devI))};
+        return Taken{{volumeIn<D>(R0), volumeIn<D>(R1)},
+                     make_float2(__fsub_rn(deviationIn<D>(R0), devI), __fsub_rn(deviationIn<D>(R1), devI))};
     }
     template <PairKind KIND>
     __device__ __forceinline__ void finish(const Neighbours &N, const Taken &taken)
@@ -1424,8 +1418,8 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftFieldsKernel
 template <int D, int K>
 struct SurfaceVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = false, kKinetic = false, kAux = false, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = false;
     const Params &P; const Frame &F;
     Smoothing<K, D, false> S;
     float normal[3];
@@ -1449,16 +1443,15 @@ struct SurfaceVisit {
 template <int D, int K>
 struct ShiftedVelocityVisit {
     static constexpr bool kCopied = false;
+    static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kKinetic = true;
-    static constexpr bool kAuxRow = D == 3;
     Smoothing<K, D, false> S;
     float vi[3], shift[3], change[3];
     __device__ void operator()(int, const float *d, float r, float, const KernelAt &k, const NeighbourRows &R)
     {
         float dot = __fmul_rn(d[0], shift[0]);
         for (int a = 1; a < D; ++a) dot = __fmaf_rn(d[a], shift[a], dot);
-        const float f = __fmul_rn(__fmul_rn(volumeIn<D>(R.B, R.X), kernelGradient<K>(__fmul_rn(r, k.invH), k)), dot);
+        const float f = __fmul_rn(__fmul_rn(volumeIn<D>(R), kernelGradient<K>(__fmul_rn(r, k.invH), k)), dot);
         float vj[3];
         velocityIn<D>(R.K, vj);
         for (int a = 0; a < D; ++a) change[a] = __fmaf_rn(f, __fsub_rn(vj[a], vi[a]), change[a]);
@@ -1614,6 +1607,31 @@ static void launchList(const LaunchArgs &A)
     }
 }
 
+// The plain sums are a form of their own, which carries none of the state of the closure, the budget (its
+// parts matter only where the step takes the maxima, or advances the density) or the compensated sums.
+template <int D, int K, int T, bool FINE>
+static void launchMomentum(const LaunchArgs &A, int grid)
+{
+    const Params &P = A.P;
+    const Frame &F = A.F;
+    cudaStream_t st = A.stream;
+    if (P.budget && A.maxima) momentumKernel<D, K, T, true, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
+    else if (P.compensated) momentumKernel<D, K, T, false, FINE, true, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
+    else if (P.closure) momentumKernel<D, K, T, false, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
+    else momentumKernel<D, K, T, false, FINE, false, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
+}
+template <int D, int K, int T, bool FINE>
+static void launchContinuity(const LaunchArgs &A, int grid)
+{
+    const Params &P = A.P;
+    const Frame &F = A.F;
+    cudaStream_t st = A.stream;
+    if (P.budget && A.flag != 0) continuityKernel<D, K, T, true, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
+    else if (P.compensated) continuityKernel<D, K, T, false, FINE, true, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
+    else if (P.closure) continuityKernel<D, K, T, false, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
+    else continuityKernel<D, K, T, false, FINE, false, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
+}
+
 template <int D, int K, int T, bool FINE>
 static void launchT(const LaunchArgs &A, Stage stage)
 {
@@ -1627,24 +1645,17 @@ static void launchT(const LaunchArgs &A, Stage stage)
     case Stage::ShepardApply: applyShepardKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
     case Stage::Wall: wallPressureKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.flag); break;
     case Stage::Gradients:
-        gradientKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.wantG, A.wantL, A.wantRho, A.floorDet);
+        if (A.wantRho) gradientKernel<D, K, T, FINE, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
+        else gradientKernel<D, K, T, FINE, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
         break;
-    case Stage::Momentum:
-        if (P.budget && A.maxima) momentumKernel<D, K, T, true, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-        else if (P.compensated)
-            momentumKernel<D, K, T, false, FINE, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-        else momentumKernel<D, K, T, false, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-        break;
+    case Stage::Momentum: launchMomentum<D, K, T, FINE>(A, grid); break;
     case Stage::Kick: kickKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::Continuity:
-        // the budget's parts matter only where the step advances the density
-        if (P.budget && A.flag != 0) continuityKernel<D, K, T, true, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-        else if (P.compensated)
-            continuityKernel<D, K, T, false, FINE, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-        else continuityKernel<D, K, T, false, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-        break;
+    case Stage::Continuity: launchContinuity<D, K, T, FINE>(A, grid); break;
     case Stage::Xsph: xsphKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.densities, A.flag); break;
-    case Stage::List: launchList<D>(A); break;
+    case Stage::List:
+        // the table does not depend on the kernel: one unit builds it for both
+        if constexpr (K == 1) launchList<D>(A);
+        break;
     case Stage::Closure: closureKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
     case Stage::ShiftFields: shiftFieldsKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl); break;
     case Stage::Shift: shiftKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl); break;
@@ -1670,15 +1681,13 @@ static void launchDK(const LaunchArgs &A, Stage stage)
     }
 }
 
-// This file is compiled once a dimension (SPH_SWEEP_DIM 2 and 3), so the two halves build side by side.
-#if SPH_SWEEP_DIM == 2
-void launchStage2(const LaunchArgs &A, Stage stage)
-#else
-void launchStage3(const LaunchArgs &A, Stage stage)
-#endif
+// This file is compiled once a dimension and kernel (SPH_SWEEP_DIM 2 and 3, SPH_SWEEP_KERNEL 0 and 1), so
+// that its units build side by side.
+#define SPH_JOIN2(a, b, c) a##b##_##c
+#define SPH_JOIN(a, b, c) SPH_JOIN2(a, b, c)
+void SPH_JOIN(launchStage, SPH_SWEEP_DIM, SPH_SWEEP_KERNEL)(const LaunchArgs &A, Stage stage)
 {
-    if (A.P.kind == 0) launchDK<SPH_SWEEP_DIM, 0>(A, stage);
-    else launchDK<SPH_SWEEP_DIM, 1>(A, stage);
+    launchDK<SPH_SWEEP_DIM, SPH_SWEEP_KERNEL>(A, stage);
 }
 
 }  // namespace sph

@@ -303,7 +303,8 @@ int sph_begin_steps(SphSystem *sys, double time, int64_t step, double last_dt, d
 int sph_enqueue_steps(SphSystem *sys, int64_t count);
 int sph_finish_steps(SphSystem *sys, double *time, int64_t *step, double *last_dt);
 
-/* Timing of the last sph_advance call (milliseconds, device events), and of each stage of the
+/* Timing of the last sph_advance call (milliseconds, device events), and, from its kernels' stamps of
+ * the device timer, of each stage of the
  * last step that ran (cells, filter, wall, gradients, momentum, kick, continuity: *count of them,
  * named by sph_stage_name), and the kernels one step launches. */
 int sph_last_advance_ms(const SphSystem *sys, double *ms);

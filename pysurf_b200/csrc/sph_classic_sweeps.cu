@@ -64,7 +64,7 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
         O.seam = true;
         O.shift64 = pi[1] < 0.5f * P.periodF ? P.period : -P.period;
     }
-    const int held = P.listCap > 0 && !(whole && boundaryRow) ? __ldg(&F.ncount[i]).x : P.listCap + 1;
+    const int held = P.listCap > 0 && !(whole && boundaryRow) ? fetch(&F.ncount[i]).x : P.listCap + 1;
     const bool walking = P.listCap == 0 || held > P.listCap;
     const int4 *column = reinterpret_cast<const int4 *>(F.nbr) + i;
     Candidates<D, false> C;
@@ -79,21 +79,21 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
             if (!C.next(P, O, pi, li, j, image, level)) return;
         } else {
             if (k >= held) return;
-            if ((k & 3) == 0) chunk = __ldg(column + (size_t)(k >> 2) * P.listStride);
+            if ((k & 3) == 0) chunk = fetch(column + (size_t)(k >> 2) * P.listStride);
             j = chunk.x & 0x7FFFFFFF;
             image = chunk.x < 0 ? 1 : 0;
             chunk.x = chunk.y; chunk.y = chunk.z; chunk.z = chunk.w;
             k = (k & 3) == 3 ? k + 1 + 4 * (T - 1) : k + 1;
         }
         const float offset = image ? (float)O.shift64 : 0.0f;     // the search's origin: particle or image
-        const float4 A = __ldg(&F.pa[j]);
+        const float4 A = fetch(&F.pa[j]);
         float pj[3];
         pointIn<D>(A, pj);
         if (walking && (coarseDistance2<D>(pi, pj, offset) >= limit || j == i)) continue;
         NeighbourRows R;
         R.A = A;
-        R.B = __ldg(&F.pb[j]);
-        if (Visitor::kKinetic || D == 2) R.K = __ldg(&F.kin[j]);
+        R.B = fetch(&F.pb[j]);
+        if (Visitor::kKinetic || D == 2) R.K = fetch(&F.kin[j]);
         const bool fluidJ = signedLengthIn<D>(A, R.B) > 0.0f;
         if (walking && fluidOnly && !fluidJ) continue;     // not in the row: not counted either
         if ((T == 1 || !walking) && !visit.accept(fluidJ)) continue;
@@ -109,7 +109,7 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
         }
         const float r = r2 > 0.0f ? r2 * rsqrtf(r2) : 0.0f;
         if (Visitor::kSkipCoincident && r < 1.0e-12f) continue;
-        if (D == 3) R.X = __ldg(&F.aux[j]);
+        if (D == 3) R.X = fetch(&F.aux[j]);
         visit(j, d, r, fluidJ, image, R);
     }
 }
@@ -133,6 +133,8 @@ struct ShepardVisit {
 template <int D, int K, int T>
 __global__ void __launch_bounds__(kBlock, 6) shepardKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
+    stampStages(const_cast<Control *>(ctl), P.stages);
     if (!filterDue(ctl)) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -197,7 +199,9 @@ struct MomentumVisit {
 template <int D, int K, int T, bool BUDGET>
 __global__ void __launch_bounds__(kBlock, BUDGET ? 4 : D == 2 ? 8 : 6) momentumKernel(Params P, Frame F, Control *ctl, int maxima)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(ctl, P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     double speed = 0.0, accel = 0.0;
@@ -248,7 +252,7 @@ struct ContinuityVisit {
     {
         float vj[3];
         velocityIn<D>(R.K, vj);
-        const float4 lowJ = __ldg(&F.low[j]);
+        const float4 lowJ = fetch(&F.low[j]);
         const float vlJ[3] = {lowJ.x, lowJ.y, lowJ.z};
         if (boundaryI == fluidJ) {
             float pi[3], li[3], pj[3], lj[3];
@@ -291,7 +295,9 @@ struct ContinuityVisit {
 template <int D, int K, int T, bool BUDGET>
 __global__ void __launch_bounds__(kBlock, BUDGET ? 4 : 5) continuityKernel(Params P, Frame F, Control *ctl, int mode)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(ctl, P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     if (i >= P.n) return;
@@ -347,6 +353,7 @@ template <int D, int K, int T>
 __global__ void __launch_bounds__(kBlock, D == 2 ? 8 : 6)
 xsphKernel(Params P, Frame F, Control *ctl, Enforcement E, const float *densities, int mode)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -378,17 +385,17 @@ static bool launchT(const LaunchArgs &A, Stage stage)
     const int grid = (int)(((long long)A.P.n * T + kBlock - 1) / kBlock);
     cudaStream_t st = A.stream;
     switch (stage) {
-    case Stage::ShepardSum: shepardKernel<D, K, T><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl); return true;
+    case Stage::ShepardSum: launchNext(shepardKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl); return true;
     case Stage::Momentum:
-        if (A.P.budget && A.maxima) momentumKernel<D, K, T, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxima);
-        else momentumKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxima);
+        if (A.P.budget && A.maxima) launchNext(momentumKernel<D, K, T, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxima);
+        else launchNext(momentumKernel<D, K, T, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxima);
         return true;
     case Stage::Continuity:
         // the budget's parts matter only where the step advances the density
-        if (A.P.budget && A.flag != 0) continuityKernel<D, K, T, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.flag);
-        else continuityKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.flag);
+        if (A.P.budget && A.flag != 0) launchNext(continuityKernel<D, K, T, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.flag);
+        else launchNext(continuityKernel<D, K, T, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.flag);
         return true;
-    case Stage::Xsph: xsphKernel<D, K, T><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.E, A.densities, A.flag); return true;
+    case Stage::Xsph: launchNext(xsphKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl, A.E, A.densities, A.flag); return true;
     default: return false;
     }
 }

@@ -44,6 +44,7 @@ constexpr float kCloseDistance = 0.3f;      // limiter fade (src/pysurf/sphSolve
 constexpr float kFoldWidth = 0.2f;
 constexpr float kCandidateMargin = 1.0001f; // on r^2, as the reference's coarse test (src/pysurf/sphGpu.py:99)
 
+constexpr int kStageCount = 7;              // a step's stages: cells, filter, wall, gradients, momentum, kick, continuity
 
 // Error flags the device raises; the host reads them after each call that syncs.
 enum DeviceError : int {
@@ -118,7 +119,24 @@ struct Params {
     int energyStride;
     // the momentum and continuity sums compensated (never with the budget: its sweeps keep plain sums)
     int compensated;
+    // the stages of a step that start with this launch, one bit each (Control::stamps); 0 outside a step
+    int stages;
 };
+
+// A step's kernels are launched to follow one another closely (launchNext): each starts here, waits for the
+// kernel before it to be complete, and lets the next be set up as soon as all its own blocks run.  It reads
+// and writes nothing before the wait.  The wait comes first, so that one kernel at most waits on the chip
+// beside the running one, whatever streams share it.
+__device__ __forceinline__ void awaitPrevious()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+// A load of what an earlier kernel of the step wrote: a plain one, since that kernel may still run when
+// this one's blocks are set up (awaitPrevious), which the read-only path does not allow for.
+template <class T>
+__device__ __forceinline__ T fetch(const T *at) { return *at; }
 
 // The float32 frame and the float64 master state, current buffers.
 struct Frame {
@@ -169,7 +187,20 @@ struct Control {
     // the maxima reduction's running values: the bits of non-negative doubles, which order as the
     // doubles do, so an integer atomicMax takes their maximum in any order; zero between steps
     unsigned long long vmaxBits, amaxBits;
+    // when each stage of the step started, and the step's end, in nanoseconds of the device's timer
+    unsigned long long stamps[kStageCount + 1];
 };
+
+// Notes the time as the start of the stages whose bits are set (a stage without a kernel starts with the
+// next one's).
+__device__ __forceinline__ void stampStages(Control *ctl, int stages)
+{
+    if (!stages || blockIdx.x != 0 || threadIdx.x != 0 || !ctl || !ctl->active) return;
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    for (int k = 0; k <= kStageCount; ++k)
+        if (stages >> k & 1) ctl->stamps[k] = now;
+}
 
 // ------------------------------------------------------------------------------------------
 // Kernels W and (dW/dr) / r: src/pysurf/sphKernels.py:108-648; src/pysurf/sphGpu.py:139-204.
@@ -407,22 +438,22 @@ __device__ __forceinline__ CellBox cellBox(const Params &P, int level, int ownCe
 
 // A particle's signed smoothing length (+h fluid, -h boundary).
 template <int D> __device__ __forceinline__ float signedLength(const Frame &F, int j);
-template <> __device__ __forceinline__ float signedLength<2>(const Frame &F, int j) { return __ldg(&F.pb[j].y); }
-template <> __device__ __forceinline__ float signedLength<3>(const Frame &F, int j) { return __ldg(&F.pa[j].w); }
+template <> __device__ __forceinline__ float signedLength<2>(const Frame &F, int j) { return fetch(&F.pb[j].y); }
+template <> __device__ __forceinline__ float signedLength<3>(const Frame &F, int j) { return fetch(&F.pa[j].w); }
 
 // A slot's own fields.
 template <int D> __device__ __forceinline__ float massOf(const Frame &F, int j)
-{ return D == 2 ? __ldg(&F.pb[j].x) : __ldg(&F.aux[j].z); }
-template <int D> __device__ __forceinline__ float pressureOf(const Frame &F, int j) { return __ldg(&F.pres[j]); }
+{ return D == 2 ? fetch(&F.pb[j].x) : fetch(&F.aux[j].z); }
+template <int D> __device__ __forceinline__ float pressureOf(const Frame &F, int j) { return fetch(&F.pres[j]); }
 // p / rho^2
 template <int D> __device__ __forceinline__ float pressureRatioOf(const Frame &F, int j)
-{ return D == 2 ? __ldg(&F.pb[j].z) : __ldg(&F.aux[j].x); }
-template <int D> __device__ __forceinline__ float deviationOf(const Frame &F, int j) { return __ldg(&F.kin[j].w); }
+{ return D == 2 ? fetch(&F.pb[j].z) : fetch(&F.aux[j].x); }
+template <int D> __device__ __forceinline__ float deviationOf(const Frame &F, int j) { return fetch(&F.kin[j].w); }
 // m / rho
 template <int D> __device__ __forceinline__ float volumeOf(const Frame &F, int j)
-{ return D == 2 ? __ldg(&F.kin[j].z) : __ldg(&F.pb[j].w); }
+{ return D == 2 ? fetch(&F.kin[j].z) : fetch(&F.pb[j].w); }
 template <int D> __device__ __forceinline__ float densityOf(const Frame &F, int j)
-{ return D == 2 ? __ldg(&F.pb[j].w) : __ldg(&F.aux[j].y); }
+{ return D == 2 ? fetch(&F.pb[j].w) : fetch(&F.aux[j].y); }
 
 // A neighbour's rows, and its fields from them: pa (A), pb (B), kin (K), aux (X, 3D), low (L), and its mass
 // where a sweep reads it apart from them.
@@ -474,7 +505,7 @@ __device__ __forceinline__ void storeDensity(const Frame &F, int i, float m, dou
 // Velocity (float32) of slot j.
 template <int D> __device__ __forceinline__ void velocityOf(const Frame &F, int j, float v[3])
 {
-    float4 k = __ldg(&F.kin[j]);
+    float4 k = fetch(&F.kin[j]);
     v[0] = k.x; v[1] = k.y; v[2] = D == 3 ? k.z : 0.0f;
 }
 
@@ -482,21 +513,21 @@ template <int D> __device__ __forceinline__ void velocityOf(const Frame &F, int 
 template <int D> __device__ __forceinline__ void pointOf(const Frame &F, int j, float p[3]);
 template <> __device__ __forceinline__ void pointOf<2>(const Frame &F, int j, float p[3])
 {
-    float4 a = __ldg(&F.pa[j]); p[0] = a.x; p[1] = a.y; p[2] = 0.0f;
+    float4 a = fetch(&F.pa[j]); p[0] = a.x; p[1] = a.y; p[2] = 0.0f;
 }
 template <> __device__ __forceinline__ void pointOf<3>(const Frame &F, int j, float p[3])
 {
-    float4 a = __ldg(&F.pa[j]); p[0] = a.x; p[1] = a.y; p[2] = a.z;
+    float4 a = fetch(&F.pa[j]); p[0] = a.x; p[1] = a.y; p[2] = a.z;
 }
 
 template <int D> __device__ __forceinline__ void remainderOf(const Frame &F, int j, float l[3]);
 template <> __device__ __forceinline__ void remainderOf<2>(const Frame &F, int j, float l[3])
 {
-    float4 a = __ldg(&F.pa[j]); l[0] = a.z; l[1] = a.w; l[2] = 0.0f;
+    float4 a = fetch(&F.pa[j]); l[0] = a.z; l[1] = a.w; l[2] = 0.0f;
 }
 template <> __device__ __forceinline__ void remainderOf<3>(const Frame &F, int j, float l[3])
 {
-    float4 b = __ldg(&F.pb[j]); l[0] = b.x; l[1] = b.y; l[2] = b.z;
+    float4 b = fetch(&F.pb[j]); l[0] = b.x; l[1] = b.y; l[2] = b.z;
 }
 
 // Matrix rows (dim x dim) packed in float4 rows.
@@ -505,13 +536,13 @@ template <int D> __device__ __forceinline__ void loadMatrix(const float4 *R0, co
 template <> __device__ __forceinline__ void loadMatrix<2>(const float4 *R0, const float4 *, const float4 *, int j,
                                                           float M[3][3])
 {
-    float4 a = __ldg(&R0[j]);
+    float4 a = fetch(&R0[j]);
     M[0][0] = a.x; M[0][1] = a.y; M[1][0] = a.z; M[1][1] = a.w;
 }
 template <> __device__ __forceinline__ void loadMatrix<3>(const float4 *R0, const float4 *R1, const float4 *R2, int j,
                                                           float M[3][3])
 {
-    float4 a = __ldg(&R0[j]), b = __ldg(&R1[j]), c = __ldg(&R2[j]);
+    float4 a = fetch(&R0[j]), b = fetch(&R1[j]), c = fetch(&R2[j]);
     M[0][0] = a.x; M[0][1] = a.y; M[0][2] = a.z;
     M[1][0] = b.x; M[1][1] = b.y; M[1][2] = b.z;
     M[2][0] = c.x; M[2][1] = c.y; M[2][2] = c.z;
@@ -534,10 +565,10 @@ template <> __device__ __forceinline__ void storeMatrix<3>(float4 *R0, float4 *R
 // The slopes' coefficients of slot j (Frame::S0, S1), in the order (0,0), (0,1), (0,2), (1,1), ...
 template <int D> __device__ __forceinline__ void loadSlopes(const Frame &F, int j, float s[6])
 {
-    const float4 a = __ldg(&F.S0[j]);
+    const float4 a = fetch(&F.S0[j]);
     s[0] = a.x; s[1] = a.y; s[2] = a.z;
     if (D == 3) {
-        const float2 b = __ldg(&F.S1[j]);
+        const float2 b = fetch(&F.S1[j]);
         s[3] = a.w; s[4] = b.x; s[5] = b.y;
     }
 }

@@ -39,8 +39,10 @@ namespace sph {
 // the square of a cell's count, as the sweeps' candidate tests over that cell already do.
 // A slot whose h is below P.fineBelow goes to the fine grid's cells, numbered after the coarse grid's.
 __global__ void cellCountKernel(Params P, int n, const double *x0, const double *x1, const double *x2,
-                                const double *h, int *slotCell, int *slotWithin, int *cellCount, const Control *ctl)
+                                const double *h, int *slotCell, int *slotWithin, int *cellCount, Control *ctl)
 {
+    awaitPrevious();
+    stampStages(ctl, P.stages);
     if (ctl && !ctl->active) return;
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -77,6 +79,7 @@ __device__ __forceinline__ int blockSumInt(int value, int *shared)
 __global__ void __launch_bounds__(kScanThreads)
 cellScanReduceKernel(const int *cellCount, int total, int *partials, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     __shared__ int shared[32];
     const int base = blockIdx.x * kScanTile;
@@ -93,6 +96,7 @@ cellScanReduceKernel(const int *cellCount, int total, int *partials, const Contr
 __global__ void __launch_bounds__(kScanThreads)
 cellScanApplyKernel(int *cellCount, int total, const int *partials, int *cellStart, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     __shared__ int shared[32];
     // the tiles before this one
@@ -138,6 +142,7 @@ cellScanApplyKernel(int *cellCount, int total, const int *partials, int *cellSta
 __global__ void cellPlaceKernel(int n, const int *slotCell, const int *slotWithin, const int *orig,
                                 const int *cellStart, int2 *bucket, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -148,6 +153,7 @@ __global__ void cellPlaceKernel(int n, const int *slotCell, const int *slotWithi
 __global__ void cellRankKernel(int n, const int2 *bucket, const int *slotCell, const int *cellStart, int *perm,
                                int *sortedCell, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -170,6 +176,7 @@ __global__ void cellRankKernel(int n, const int2 *bucket, const int *slotCell, c
 __global__ void gatherKernel(Params P, int n, const int *perm, MasterView from, MasterView to, Frame F,
                              const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned present = __ballot_sync(0xFFFFFFFFu, s < n);
@@ -273,6 +280,7 @@ __global__ void loadFieldsKernel(Params P, int n, const int *orig, const double 
 
 __global__ void refreshDensityKernel(int n, const double *rho, float *out)
 {
+    awaitPrevious();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (float)rho[i];
 }
@@ -338,7 +346,9 @@ __global__ void fluidEnergyKernel(Params P, Frame F, double *columns, long long 
 // count allows (src/pysurf/sphSolver.py:1980-1989).
 __global__ void stepEndKernel(Control *ctl)
 {
+    awaitPrevious();
     if (!ctl->active) return;
+    stampStages(ctl, 1 << kStageCount);
     ctl->time += ctl->dt;
     ctl->step += 1;
     ctl->active = ctl->time < ctl->untilTime && ctl->step < ctl->lastStep && ctl->error == 0;
@@ -616,23 +626,23 @@ static inline int blocksFor(long long n, int block) { return (int)((n + block - 
 int scanTiles(int total) { return blocksFor(total, kScanTile); }
 
 void launchCellSort(const Params &P, int n, const MasterView &M, const CellSortBuffers &B, int *cellStart,
-                    int *sortedCell, const Control *ctl, cudaStream_t st)
+                    int *sortedCell, Control *ctl, cudaStream_t st)
 {
     if (n == 0) return;
     const int total = P.cells + 1, tiles = scanTiles(total);
-    cellCountKernel<<<blocksFor(n, 256), 256, 0, st>>>(P, n, M.x[0], M.x[1], M.x[2], M.h, B.slotCell, B.slotWithin,
+    launchNext(cellCountKernel, blocksFor(n, 256), 256, st, P, n, M.x[0], M.x[1], M.x[2], M.h, B.slotCell, B.slotWithin,
                                                        B.cellCount, ctl);
-    cellScanReduceKernel<<<tiles, kScanThreads, 0, st>>>(B.cellCount, total, B.partials, ctl);
-    cellScanApplyKernel<<<tiles, kScanThreads, 0, st>>>(B.cellCount, total, B.partials, cellStart, ctl);
-    cellPlaceKernel<<<blocksFor(n, 256), 256, 0, st>>>(n, B.slotCell, B.slotWithin, M.orig, cellStart, B.bucket, ctl);
-    cellRankKernel<<<blocksFor(n, 256), 256, 0, st>>>(n, B.bucket, B.slotCell, cellStart, B.perm, sortedCell, ctl);
+    launchNext(cellScanReduceKernel, tiles, kScanThreads, st, B.cellCount, total, B.partials, ctl);
+    launchNext(cellScanApplyKernel, tiles, kScanThreads, st, B.cellCount, total, B.partials, cellStart, ctl);
+    launchNext(cellPlaceKernel, blocksFor(n, 256), 256, st, n, B.slotCell, B.slotWithin, M.orig, cellStart, B.bucket, ctl);
+    launchNext(cellRankKernel, blocksFor(n, 256), 256, st, n, B.bucket, B.slotCell, cellStart, B.perm, sortedCell, ctl);
 }
 
 void launchGather(const Params &P, int n, const int *perm, const MasterView &from, const MasterView &to,
                   const Frame &F, const Control *ctl, cudaStream_t st)
 {
     if (n == 0) return;
-    gatherKernel<<<blocksFor(n, 256), 256, 0, st>>>(P, n, perm, from, to, F, ctl);
+    launchNext(gatherKernel, blocksFor(n, 256), 256, st, P, n, perm, from, to, F, ctl);
 }
 
 void launchLoadFields(const Params &P, int n, const int *orig, const double *v, const double *rho, const double *p,
@@ -649,7 +659,7 @@ void launchLoadMaster(int n, int dim, const double *x, const double *v, const do
     loadMasterKernel<<<blocksFor(n, 256), 256, 0, st>>>(n, dim, x, v, rho, m, fluid, h, hDefault, M);
 }
 
-void launchStepEnd(Control *ctl, cudaStream_t st) { stepEndKernel<<<1, 1, 0, st>>>(ctl); }
+void launchStepEnd(Control *ctl, cudaStream_t st) { launchNext(stepEndKernel, 1, 1, st, ctl); }
 
 cudaError_t kernelAttributes(cudaFuncAttributes *attributes)
 {
@@ -677,7 +687,7 @@ void launchFluidEnergy(const Params &P, const Frame &F, double *columns, long lo
 void launchRefreshDensity(int n, const double *rho, float *out, cudaStream_t st)
 {
     if (n == 0) return;
-    refreshDensityKernel<<<blocksFor(n, 256), 256, 0, st>>>(n, rho, out);
+    launchNext(refreshDensityKernel, blocksFor(n, 256), 256, st, n, rho, out);
 }
 
 void launchPull(int n, int dim, const MasterView &M, const Frame &F, const float4 *acc, const PullRows &R,

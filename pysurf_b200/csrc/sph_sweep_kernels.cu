@@ -51,13 +51,13 @@ constexpr int gradientMinBlocks() { return D == 2 ? 5 : 3; }
 // word, so a run of a stencil row is a few words).
 __device__ __forceinline__ bool isFluid(const Frame &F, int j)
 {
-    return !(__ldg(&F.wallBits[j >> 5]) >> (j & 31) & 1);
+    return !(fetch(&F.wallBits[j >> 5]) >> (j & 31) & 1);
 }
 __device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
 {
     unsigned any = 0;
     for (int w = first >> 5; w <= (end - 1) >> 5; ++w) {
-        unsigned bits = __ldg(&F.wallBits[w]);
+        unsigned bits = fetch(&F.wallBits[w]);
         if (w == first >> 5) bits &= 0xFFFFFFFFu << (first & 31);
         if (w == (end - 1) >> 5) bits &= 0xFFFFFFFFu >> (31 - ((end - 1) & 31));
         any |= bits;
@@ -78,6 +78,7 @@ __device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
 template <int D, int L, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     const Group<L> G = groupOf<L>();
     const int i = G.i;
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
     const int t = G.t;
     const int shift = (threadIdx.x & 31) & ~(L - 1);
     const unsigned lower = (1u << t) - 1u;
-    const float4 Ai = __ldg(&F.pa[i]), Bi = __ldg(&F.pb[i]);
+    const float4 Ai = fetch(&F.pa[i]), Bi = fetch(&F.pb[i]);
     const float hI = fabsf(signedLengthIn<D>(Ai, Bi));
     // a boundary row holds its fluid neighbours only (Row says why)
     const bool fluidOnly = signedLengthIn<D>(Ai, Bi) <= 0.0f;
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
                 const int j = base + t;
                 bool accepted = false, fluidJ = true;
                 if (j < end && j != i) {
-                    const float4 A = __ldg(&F.pa[j]);
+                    const float4 A = fetch(&F.pa[j]);
                     float pj[3];
                     pointIn<D>(A, pj);
                     if (WALLED) fluidJ = isFluid(F, j);
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
                     if (PRECISE && !image && level == 0 && coarse < sure) {
                         accepted = true;
                     } else if (coarse < searchLimit) {
-                        const float4 B = (D == 3 && PRECISE) || MIXED ? __ldg(&F.pb[j]) : A;
+                        const float4 B = (D == 3 && PRECISE) || MIXED ? fetch(&F.pb[j]) : A;
                         float r2 = coarse;      // the float32 points' separation is the coarse one
                         if (PRECISE) {
                             float lj[3], d[3];
@@ -188,8 +189,8 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
                 }
                 if (!empty) {
                     const int row = box.first + (zz * box.ny + yy) * box.nx;
-                    runFirst = __ldg(&F.cellStart[row + xa]);
-                    runEnd = __ldg(&F.cellStart[row + xb + 1]);
+                    runFirst = fetch(&F.cellStart[row + xa]);
+                    runEnd = fetch(&F.cellStart[row + xb + 1]);
                     runWalls = runHasWalls(F, runFirst, runEnd);
                 }
             }
@@ -238,6 +239,7 @@ struct alignas(16) BatchMember {
 template <int D, int kBatch, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     __shared__ BatchMember members[kBlock / 32][kBatch];
     const int lane = threadIdx.x & 31;
@@ -252,21 +254,21 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
     bool starts = false;
     if (lane < kBatch && first + lane < last) {
         const int s = first + lane;
-        starts = (s - __ldg(&F.cellStart[F.cell[s]])) % kBatch == 0;
+        starts = (s - fetch(&F.cellStart[F.cell[s]])) % kBatch == 0;
     }
     unsigned pending = __ballot_sync(0xFFFFFFFFu, starts);
     while (pending) {
         const int b0 = first + __ffs(pending) - 1;
         pending &= pending - 1;
         const int ownCell = F.cell[b0];
-        const int count = min(kBatch, __ldg(&F.cellStart[ownCell + 1]) - b0);
+        const int count = min(kBatch, fetch(&F.cellStart[ownCell + 1]) - b0);
         // lane p < count sets up member p
         float hIp = 0.0f, pip[3] = {0, 0, 0}, lip[3] = {0, 0, 0};
         double shiftp = 0.0;
         bool seamp = false, wholeRow = false;
         if (lane < count) {
             const int i = b0 + lane;
-            const float4 Ai = __ldg(&F.pa[i]), Bi = __ldg(&F.pb[i]);
+            const float4 Ai = fetch(&F.pa[i]), Bi = fetch(&F.pb[i]);
             hIp = fabsf(signedLengthIn<D>(Ai, Bi));
             pointIn<D>(Ai, pip);
             remainderIn<D>(Ai, Bi, lip);
@@ -354,8 +356,8 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                             }
                         }
                         if (!empty) {
-                            a = __ldg(&F.cellStart[row + xa]);
-                            b = __ldg(&F.cellStart[row + xb + 1]);
+                            a = fetch(&F.cellStart[row + xa]);
+                            b = fetch(&F.cellStart[row + xb + 1]);
                         }
                     }
                     const int uA = __reduce_min_sync(0xFFFFFFFFu, a < b ? a : INT_MAX);
@@ -370,14 +372,14 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                         bool fluidJ = false;
                         unsigned offered = 0;       // the members this candidate is offered to
                         if (j < uB) {
-                            A = __ldg(&F.pa[j]);
+                            A = fetch(&F.pa[j]);
                             pointIn<D>(A, pj);
                             // the remainders with the point, although a candidate under `sure` needs
                             // none: loading them only for the precise test slowed the 3D table by 11%
-                            if ((D == 3 && PRECISE) || MIXED) B = __ldg(&F.pb[j]);
+                            if ((D == 3 && PRECISE) || MIXED) B = fetch(&F.pb[j]);
                             if (PRECISE) remainderIn<D>(A, D == 3 ? B : A, lj);
                             if (MIXED) hJ = fabsf(signedLengthIn<D>(A, B));
-                            fluidJ = D == 3 ? A.w > 0.0f : __ldg(&F.fluid[j]) != 0;
+                            fluidJ = D == 3 ? A.w > 0.0f : fetch(&F.fluid[j]) != 0;
                             offered = fluidJ ? 0xFFFFFFFFu : wholeRows;
                             if (j >= b0 && j < b0 + kBatch) offered &= ~(1u << (j - b0));      // not to itself
                         }
@@ -469,6 +471,8 @@ struct ShepardVisit {
 template <int D, int K, int T, bool FINE>
 __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shepardKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
+    stampStages(const_cast<Control *>(ctl), P.stages);
     if (!filterDue(ctl)) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -496,6 +500,7 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shepardKernel(Par
 template <int D>
 __global__ void applyShepardKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
     if (!filterDue(ctl)) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n || !F.fluid[i]) return;
@@ -535,7 +540,9 @@ template <int D, int K, int T, bool FINE>
 __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>())
 wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(const_cast<Control *>(ctl), P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     if (i >= P.n) return;
@@ -654,7 +661,9 @@ template <int D, int K, int T, bool FINE, bool RHO>
 __global__ void __launch_bounds__(kBlock, gradientMinBlocks<D>())
 gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, float floorDet)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(const_cast<Control *>(ctl), P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     if (i >= P.n) return;
@@ -864,7 +873,7 @@ struct MomentumVisit {
     // (r^2 rho_i rho_j) on every fluid pair, approaching or not (src/pysurf/sphGpu.py:388-396)
     __device__ __forceinline__ float closureTerm(int j, float h, float r, float plain, float rhoJ) const
     {
-        const float alphaJ = __ldg(&F.eddy[j].x), sum = __fadd_rn(alphaI, alphaJ);
+        const float alphaJ = fetch(&F.eddy[j].x), sum = __fadd_rn(alphaI, alphaJ);
         const float mean = sum > 0.0f ? __fdiv_rn(__fmul_rn(__fmul_rn(2.0f, alphaI), alphaJ), sum) : 0.0f;
         const float scale = __fmul_rn(__fmul_rn(__fmul_rn(__fadd_rn(__fdiv_rn(P.waterTerm, h), mean), P.c0), h), P.closureRho0);
         return __fdiv_rn(-__fmul_rn(scale, plain), __fmul_rn(__fmul_rn(__fmul_rn(r, r), rhoI), rhoJ));
@@ -877,7 +886,9 @@ template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 __global__ void __launch_bounds__(kBlock, BUDGET ? budgetMinBlocks<D>() : sweepMinBlocks<D>())
 momentumKernel(Params P, Frame F, Control *ctl, int maxima)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(ctl, P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     double speed = 0.0, accel = 0.0;
@@ -928,6 +939,7 @@ momentumKernel(Params P, Frame F, Control *ctl, int maxima)
 template <int D>
 __global__ void closureKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
@@ -953,7 +965,9 @@ __global__ void closureKernel(Params P, Frame F, const Control *ctl)
 template <int D>
 __global__ void kickKernel(Params P, Frame F, Control *ctl)
 {
+    awaitPrevious();
     if (!ctl->active) return;
+    stampStages(ctl, P.stages);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n || !F.fluid[i]) return;
     double dt = ctl->dt;
@@ -1128,7 +1142,7 @@ struct ContinuityVisit {
                 difference = add2(leading, remainder);
             }
             if (P.diffusion == 3) {
-                const float4 g0 = __ldg(&F.gradRho[N.j[0]]), g1 = __ldg(&F.gradRho[N.j[1]]);
+                const float4 g0 = fetch(&F.gradRho[N.j[0]]), g1 = fetch(&F.gradRho[N.j[1]]);
                 const float gj0[3] = {g0.x, g0.y, g0.z}, gj1[3] = {g1.x, g1.y, g1.z};
                 float2 t = both(0.0f);
                 for (int a = 0; a < D; ++a)
@@ -1158,7 +1172,7 @@ struct ContinuityVisit {
     }
     __device__ __forceinline__ float pairFactor(int j) const
     {
-        const float deltaJ = __ldg(&F.eddy[j].y), sum = __fadd_rn(deltaI, deltaJ);
+        const float deltaJ = fetch(&F.eddy[j].y), sum = __fadd_rn(deltaI, deltaJ);
         if (!(sum > 0.0f)) return 0.0f;
         return __fmul_rn(__fmul_rn(2.0f, P.closureC0), __fdiv_rn(__fmul_rn(__fmul_rn(2.0f, deltaI), deltaJ), sum));
     }
@@ -1191,7 +1205,9 @@ template <int D, int K, int T, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 __global__ void __launch_bounds__(kBlock, BUDGET ? budgetMinBlocks<D>() : preciseMinBlocks<D>())
 continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
+    stampStages(ctl, P.stages);
     const Group<T> G = groupOf<T>();
     const int i = G.i;
     if (i >= P.n) return;
@@ -1291,6 +1307,7 @@ template <int D, int K, int T, bool FINE>
 __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>())
 xsphKernel(Params P, Frame F, Control *ctl, Enforcement E, const float *densities, int mode)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -1328,6 +1345,7 @@ xsphKernel(Params P, Frame F, Control *ctl, Enforcement E, const float *densitie
 template <int D>
 __global__ void frameDensityKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
@@ -1378,6 +1396,7 @@ struct ShiftFieldsVisit {
 template <int D, int K, int T, bool FINE>
 __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftFieldsKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -1426,7 +1445,7 @@ struct SurfaceVisit {
     int vicinity;
     __device__ void operator()(int j, const float *, float r, float, const KernelAt &k, const NeighbourRows &)
     {
-        const float4 plainJ = __ldg(&F.shiftPlain[j]);
+        const float4 plainJ = fetch(&F.shiftPlain[j]);
         if (!(plainJ.w < P.shiftThreshold)) return;
         vicinity = 1;
         const float length = sqrtf(__fmaf_rn(plainJ.z, plainJ.z, __fmaf_rn(plainJ.y, plainJ.y, __fmul_rn(plainJ.x, plainJ.x))));
@@ -1465,6 +1484,7 @@ struct ShiftedVelocityVisit {
 template <int D, int K, int T, bool FINE>
 __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftKernel(Params P, Frame F, const Control *ctl)
 {
+    awaitPrevious();
     if (ctl && !ctl->active) return;
     const Group<T> G = groupOf<T>();
     const int i = G.i;
@@ -1523,6 +1543,7 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftKernel(Param
 template <int D>
 __global__ void shiftDriftKernel(Params P, Frame F, Control *ctl, Enforcement E, int useTransport)
 {
+    awaitPrevious();
     if (!ctl->active) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n || !F.fluid[i]) return;
@@ -1577,16 +1598,16 @@ static void launchListAs(const LaunchArgs &A)
     cudaStream_t st = A.stream;
     if constexpr (D == 3) {
         const int grid = blocksFor((long long)blocksFor(A.P.n, SHARE) * 32, kBlock);
-        if (A.P.precise && !A.P.mixedH) cellListKernel<D, SHARE, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (A.P.precise) cellListKernel<D, SHARE, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (!A.P.mixedH) cellListKernel<D, SHARE, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else cellListKernel<D, SHARE, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        if (A.P.precise && !A.P.mixedH) launchNext(cellListKernel<D, SHARE, true, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else if (A.P.precise) launchNext(cellListKernel<D, SHARE, true, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else if (!A.P.mixedH) launchNext(cellListKernel<D, SHARE, false, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else launchNext(cellListKernel<D, SHARE, false, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
     } else {
         const int grid = blocksFor((long long)A.P.n * SHARE, kBlock);
-        if (A.P.precise && !A.P.mixedH) listKernel<D, SHARE, true, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (A.P.precise) listKernel<D, SHARE, true, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else if (!A.P.mixedH) listKernel<D, SHARE, false, false><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
-        else listKernel<D, SHARE, false, true><<<grid, kBlock, 0, st>>>(A.P, A.F, A.ctl, A.maxCount);
+        if (A.P.precise && !A.P.mixedH) launchNext(listKernel<D, SHARE, true, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else if (A.P.precise) launchNext(listKernel<D, SHARE, true, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else if (!A.P.mixedH) launchNext(listKernel<D, SHARE, false, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
+        else launchNext(listKernel<D, SHARE, false, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxCount);
     }
 }
 
@@ -1615,10 +1636,10 @@ static void launchMomentum(const LaunchArgs &A, int grid)
     const Params &P = A.P;
     const Frame &F = A.F;
     cudaStream_t st = A.stream;
-    if (P.budget && A.maxima) momentumKernel<D, K, T, true, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-    else if (P.compensated) momentumKernel<D, K, T, false, FINE, true, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-    else if (P.closure) momentumKernel<D, K, T, false, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
-    else momentumKernel<D, K, T, false, FINE, false, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.maxima);
+    if (P.budget && A.maxima) launchNext(momentumKernel<D, K, T, true, FINE, false, true>, grid, kBlock, st, P, F, A.ctl, A.maxima);
+    else if (P.compensated) launchNext(momentumKernel<D, K, T, false, FINE, true, true>, grid, kBlock, st, P, F, A.ctl, A.maxima);
+    else if (P.closure) launchNext(momentumKernel<D, K, T, false, FINE, false, true>, grid, kBlock, st, P, F, A.ctl, A.maxima);
+    else launchNext(momentumKernel<D, K, T, false, FINE, false, false>, grid, kBlock, st, P, F, A.ctl, A.maxima);
 }
 template <int D, int K, int T, bool FINE>
 static void launchContinuity(const LaunchArgs &A, int grid)
@@ -1626,10 +1647,10 @@ static void launchContinuity(const LaunchArgs &A, int grid)
     const Params &P = A.P;
     const Frame &F = A.F;
     cudaStream_t st = A.stream;
-    if (P.budget && A.flag != 0) continuityKernel<D, K, T, true, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-    else if (P.compensated) continuityKernel<D, K, T, false, FINE, true, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-    else if (P.closure) continuityKernel<D, K, T, false, FINE, false, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
-    else continuityKernel<D, K, T, false, FINE, false, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag);
+    if (P.budget && A.flag != 0) launchNext(continuityKernel<D, K, T, true, FINE, false, true>, grid, kBlock, st, P, F, A.ctl, A.E, A.flag);
+    else if (P.compensated) launchNext(continuityKernel<D, K, T, false, FINE, true, true>, grid, kBlock, st, P, F, A.ctl, A.E, A.flag);
+    else if (P.closure) launchNext(continuityKernel<D, K, T, false, FINE, false, true>, grid, kBlock, st, P, F, A.ctl, A.E, A.flag);
+    else launchNext(continuityKernel<D, K, T, false, FINE, false, false>, grid, kBlock, st, P, F, A.ctl, A.E, A.flag);
 }
 
 template <int D, int K, int T, bool FINE>
@@ -1641,26 +1662,26 @@ static void launchT(const LaunchArgs &A, Stage stage)
     if (P.n == 0) return;
     cudaStream_t st = A.stream;
     switch (stage) {
-    case Stage::ShepardSum: shepardKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::ShepardApply: applyShepardKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::Wall: wallPressureKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.flag); break;
+    case Stage::ShepardSum: launchNext(shepardKernel<D, K, T, FINE>, grid, kBlock, st, P, F, A.ctl); break;
+    case Stage::ShepardApply: launchNext(applyShepardKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;
+    case Stage::Wall: launchNext(wallPressureKernel<D, K, T, FINE>, grid, kBlock, st, P, F, A.ctl, A.flag); break;
     case Stage::Gradients:
-        if (A.wantRho) gradientKernel<D, K, T, FINE, true><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
-        else gradientKernel<D, K, T, FINE, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
+        if (A.wantRho) launchNext(gradientKernel<D, K, T, FINE, true>, grid, kBlock, st, P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
+        else launchNext(gradientKernel<D, K, T, FINE, false>, grid, kBlock, st, P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
         break;
     case Stage::Momentum: launchMomentum<D, K, T, FINE>(A, grid); break;
-    case Stage::Kick: kickKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
+    case Stage::Kick: launchNext(kickKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;
     case Stage::Continuity: launchContinuity<D, K, T, FINE>(A, grid); break;
-    case Stage::Xsph: xsphKernel<D, K, T, FINE><<<grid, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.densities, A.flag); break;
+    case Stage::Xsph: launchNext(xsphKernel<D, K, T, FINE>, grid, kBlock, st, P, F, A.ctl, A.E, A.densities, A.flag); break;
     case Stage::List:
         // the table does not depend on the kernel: one unit builds it for both
         if constexpr (K == 1) launchList<D>(A);
         break;
-    case Stage::Closure: closureKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::ShiftFields: shiftFieldsKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::Shift: shiftKernel<D, K, T, false><<<grid, kBlock, 0, st>>>(P, F, A.ctl); break;
-    case Stage::ShiftDrift: shiftDriftKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl, A.E, A.flag); break;
-    case Stage::FrameDensity: frameDensityKernel<D><<<pointwise, kBlock, 0, st>>>(P, F, A.ctl); break;
+    case Stage::Closure: launchNext(closureKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;
+    case Stage::ShiftFields: launchNext(shiftFieldsKernel<D, K, T, false>, grid, kBlock, st, P, F, A.ctl); break;
+    case Stage::Shift: launchNext(shiftKernel<D, K, T, false>, grid, kBlock, st, P, F, A.ctl); break;
+    case Stage::ShiftDrift: launchNext(shiftDriftKernel<D>, pointwise, kBlock, st, P, F, A.ctl, A.E, A.flag); break;
+    case Stage::FrameDensity: launchNext(frameDensityKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;
     }
 }
 

@@ -245,8 +245,8 @@ struct Candidates {
     __device__ __forceinline__ void startRow()
     {
         const int row = first + (zz * ny + yy) * nx;
-        j = __ldg(&cellStart[row + x0]) - 1;
-        end = __ldg(&cellStart[row + x1 + 1]);
+        j = fetch(&cellStart[row + x0]) - 1;
+        end = fetch(&cellStart[row + x1 + 1]);
     }
 
     // Starts search s when it applies (its level is present, its image is wanted); false if not.
@@ -321,7 +321,7 @@ struct Paired<V, std::void_t<decltype(V::kPaired)>> {
 __device__ __forceinline__ float4 loadEarly(const float4 *at)
 {
     float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
     return v;
 }
@@ -339,7 +339,7 @@ __device__ __forceinline__ void loadRows(const Frame &F, int j, NeighbourRows &R
     if constexpr (Visitor::kLow) R.L = loadEarly(&F.low[j]);
     if constexpr (Visitor::kMass && D == 2) R.m = R.L.z;
     if constexpr (Visitor::kMass && D == 3)
-        asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(R.m) : "l"(&F.aux[j].z));
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(R.m) : "l"(&F.aux[j].z));
 }
 
 // Two neighbours of a particle as a paired visitor gets them: their slots, whether each counts and lies
@@ -382,7 +382,7 @@ __device__ __forceinline__ Row openRow(const Params &P, const Frame &F, int i, i
         O.seam = true;
         O.shift64 = O.pi[1] < 0.5f * P.periodF ? P.period : -P.period;
     }
-    O.count = P.listCap > 0 && !whole ? __ldg(&F.ncount[i]) : make_int2(0, 0);
+    O.count = P.listCap > 0 && !whole ? fetch(&F.ncount[i]) : make_int2(0, 0);
     O.listed = P.listCap > 0 && !whole && O.count.x + O.count.y <= P.listCap;
     return O;
 }
@@ -472,7 +472,7 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
         };
         auto entry = [&](const int *at) {
             int value;
-                        asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(value) : "l"(at));
+                        asm volatile("ld.global.L1::no_allocate.b32 %0, [%1];" : "=r"(value) : "l"(at));
             return value;
         };
         int left = count > O.t ? (count - O.t - 1) / T + 1 : 0;
@@ -552,11 +552,11 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
         ended = !C.next(P, origin, O.pi, O.li, j, image, level);
         if (!ended) {
             const float offset = image ? (float)O.shift64 : 0.0f;   // the search's origin: particle or image
-            const float4 A = __ldg(&F.pa[j]);
+            const float4 A = fetch(&F.pa[j]);
             float pj[3], lj[3], d[3];
             pointIn<D>(A, pj);
             if (coarseDistance2<D>(O.pi, pj, offset) >= (FINE && level ? fineLimit : limit) || j == O.i) continue;
-            const float4 B = __ldg(&F.pb[j]);
+            const float4 B = fetch(&F.pb[j]);
             const float hs = signedLengthIn<D>(A, B);
             if ((hs > 0.0f) != fluid) continue;     // the other kind
             remainderIn<D>(A, B, lj);

@@ -9,8 +9,8 @@
 // A device-resident step is captured once into a CUDA graph, twice over: a step moves the master
 // to the other buffer, so one graph starts from each.  Runs of steps replay them alternately;
 // each step's time step is taken on the device from its own maxima, and the host reads the clock
-// back only when it must decide whether to launch more.  Events between the stages of each graph
-// time every stage of the last step (sph_stage_times).
+// back only when it must decide whether to launch more.  The kernels that begin a step's stages note the
+// device's time (Control::stamps), for sph_stage_times.
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -26,8 +26,6 @@
 using namespace sph;
 
 namespace {
-
-constexpr int kStageCount = 7;      // cells, filter, wall, gradients, momentum, kick, continuity
 
 thread_local std::string lastError;
 
@@ -180,11 +178,9 @@ struct SphSystem {
     cudaStream_t stream = nullptr;
     bool ownStream = false;
     cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // one step from master buffer 0, one from buffer 1
-    cudaEvent_t stageEvents[2][kStageCount + 1] = {};
     bool graphDirty = true;
     bool graphFilter = false;
     int graphNodes = 0;
-    int lastGraph = 0;
     int beginCur = 0;
     long long beginStep = 0;
     long long enqueued = 0;
@@ -553,10 +549,12 @@ struct SphSystem {
     // Sort the master by (cell, caller index), permute it into the other buffer, and build the
     // frame and the cell list.
     // control: the device clock that gates the step (null: always runs).
-    void rebuild(const Control *control = nullptr)
+    // stages: the stages of a step that begin with it (Params::stages).
+    void rebuild(Control *control = nullptr, int stages = 0)
     {
         if (n == 0) return;
         Params P = params();
+        P.stages = stages;
         launchCellSort(P, n, master[cur], sortBuffers, cellStart, cell, control, stream);
         int next = 1 - cur;
         Frame F = frame();
@@ -569,7 +567,7 @@ struct SphSystem {
         cellsFresh = true;
         if (listCap > 0) {
             listTogether = classic();
-            LaunchArgs A = args(const_cast<Control *>(control));
+            LaunchArgs A = args(control);
             launchStage(A, Stage::List);
         }
     }
@@ -721,9 +719,6 @@ int sph_create(int dimensions, double smoothing_length, const double *domain_min
     if (status == SPH_OK && (cudaEventCreate(&s->evStart) != cudaSuccess || cudaEventCreate(&s->evStop) != cudaSuccess ||
                              cudaEventCreateWithFlags(&s->uploaded, cudaEventDisableTiming) != cudaSuccess))
         status = SPH_ERR_CUDA;
-    for (int b = 0; b < 2 && status == SPH_OK; ++b)
-        for (int k = 0; k <= kStageCount && status == SPH_OK; ++k)
-            if (cudaEventCreate(&s->stageEvents[b][k]) != cudaSuccess) status = SPH_ERR_CUDA;
     if (status == SPH_OK) status = s->setupGrid();
     if (status != SPH_OK) {
         sph_destroy(s);
@@ -743,8 +738,6 @@ int sph_destroy(SphSystem *sys)
     if (sys->stream) cudaStreamSynchronize(sys->stream);
     for (int b = 0; b < 2; ++b) {
         if (sys->graphs[b]) cudaGraphExecDestroy(sys->graphs[b]);
-        for (int k = 0; k <= kStageCount; ++k)
-            if (sys->stageEvents[b][k]) cudaEventDestroy(sys->stageEvents[b][k]);
     }
     sys->freeArrays();
     cudaFree(sys->energy);
@@ -1573,60 +1566,61 @@ int sph_enforce_boundary(SphSystem *sys)
     return SPH_OK;
 }
 
-// The stages a step's events bracket, in order (sph_stage_times reports them in this order).
+// A step's stages, in order (sph_stage_times reports them in this order).
 static const char *const kStageNames[kStageCount] = {"cells", "filter", "wall", "gradients", "momentum", "kick",
                                                       "continuity"};
 
-// Records the event of stage k when a set of events is given (inside a captured step graph).
-static void mark(SphSystem *sys, cudaEvent_t *events, int k)
-{
-    if (events) cudaEventRecordWithFlags(events[k], sys->stream, cudaEventRecordExternal);
-}
-
 // The first half of a step: cell list, optional filter, wall pressure, gradients, momentum.
 // filter: the Shepard stage is enqueued (the device decides each step whether it is due).
-static void enqueueRates(SphSystem *sys, bool filter, cudaEvent_t *events = nullptr)
+static void enqueueRates(SphSystem *sys, bool filter)
 {
-    mark(sys, events, 0);
-    sys->rebuild(sys->ctl);
-    mark(sys, events, 1);
+    sys->rebuild(sys->ctl, 1 << 0);
     LaunchArgs A = sys->args(sys->ctl);
+    int begins = 1 << 1;        // the stages that begin with the next launch
+    auto launch = [&](Stage stage) {
+        A.P.stages = begins;
+        launchStage(A, stage);
+        A.P.stages = begins = 0;
+    };
     if (filter) {
-        launchStage(A, Stage::ShepardSum);
-        launchStage(A, Stage::ShepardApply);
+        launch(Stage::ShepardSum);
+        launch(Stage::ShepardApply);
     }
-    mark(sys, events, 2);
+    begins |= 1 << 2;
     if (sys->wallExtrapolated) {
         A.flag = 1;
-        launchStage(A, Stage::Wall);
+        launch(Stage::Wall);
     }
-    mark(sys, events, 3);
+    begins |= 1 << 3;
     bool wantL = sys->corrected || sys->diffusionMode == 3;
     if (sys->limited || sys->closure || wantL) {
         A.wantG = sys->limited || sys->closure;
         A.wantL = wantL;
         A.wantRho = sys->diffusionMode == 3;
-        launchStage(A, Stage::Gradients);
+        launch(Stage::Gradients);
         A.wantG = A.wantL = A.wantRho = 0;
     }
     // the closure's coefficients, from this step's starting velocities (the diffusion reuses them)
     if (sys->closure) launchStage(A, Stage::Closure);
-    mark(sys, events, 4);
-    launchStage(A, Stage::Momentum);
-    mark(sys, events, 5);
+    begins |= 1 << 4;
+    launch(Stage::Momentum);
 }
 
 // The second half: kick, continuity with the density update, XSPH, drift and enforcement.
-static void enqueueIntegrate(SphSystem *sys, cudaEvent_t *events = nullptr)
+static void enqueueIntegrate(SphSystem *sys)
 {
     LaunchArgs A = sys->args(sys->ctl);
+    A.P.stages = 1 << 5;
     launchStage(A, Stage::Kick);
-    mark(sys, events, 6);
+    A.P.stages = 1 << 6;
+    // the density update; with neither shifting nor XSPH to come, the drift and the enforcement too
+    const bool drifts = !sys->shifting && !(sys->xsphEpsilon > 0.0);
+    A.flag = drifts ? 2 : 1;
+    launchStage(A, Stage::Continuity);
+    A.P.stages = 0;
     if (sys->shifting) {
-        // the density update, then the shift from the step's starting geometry, the updated
-        // densities and the kicked velocities, then one drift (src/pysurf/sphSolver.py:1760-1785)
-        A.flag = 1;
-        launchStage(A, Stage::Continuity);
+        // the shift from the step's starting geometry, the updated densities and the kicked velocities,
+        // then one drift (src/pysurf/sphSolver.py:1760-1785)
         int useTransport = 0;
         if (sys->xsphEpsilon > 0.0) {
             launchRefreshDensity(sys->n, A.F.rho, sys->scalar, sys->stream);
@@ -1640,18 +1634,12 @@ static void enqueueIntegrate(SphSystem *sys, cudaEvent_t *events = nullptr)
         launchStage(A, Stage::Shift);
         A.flag = useTransport;
         launchStage(A, Stage::ShiftDrift);
-    } else if (sys->xsphEpsilon > 0.0) {
-        A.flag = 1;
-        launchStage(A, Stage::Continuity);
+    } else if (!drifts) {
         launchRefreshDensity(sys->n, A.F.rho, sys->scalar, sys->stream);
         A.flag = 2;
         A.densities = sys->scalar;
         launchStage(A, Stage::Xsph);
-    } else {
-        A.flag = 2;
-        launchStage(A, Stage::Continuity);
     }
-    mark(sys, events, 7);
 }
 
 int sph_resident_rates(SphSystem *sys, int filter_density, double *max_speed, double *max_acceleration)
@@ -1703,7 +1691,7 @@ int sph_resident_integrate(SphSystem *sys, double time_step)
 }
 
 // Two single-step graphs, one from each master buffer (a step moves the master to the other
-// buffer), each with events between its stages.
+// buffer).
 static int captureSteps(SphSystem *sys, bool filter)
 {
     for (int b = 0; b < 2; ++b) {
@@ -1714,8 +1702,8 @@ static int captureSteps(SphSystem *sys, bool filter)
         sys->cur = b;
         cudaGraph_t g;
         CUDA_TRY(cudaStreamBeginCapture(sys->stream, cudaStreamCaptureModeThreadLocal));
-        enqueueRates(sys, filter, sys->stageEvents[b]);
-        enqueueIntegrate(sys, sys->stageEvents[b]);
+        enqueueRates(sys, filter);
+        enqueueIntegrate(sys);
         launchStepEnd(sys->ctl, sys->stream);
         cudaError_t err = cudaStreamEndCapture(sys->stream, &g);
         if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(err));
@@ -1780,7 +1768,6 @@ int sph_enqueue_steps(SphSystem *sys, int64_t count)
     if (!sys->graphs[0]) return fail(SPH_ERR_STATE, "call sph_begin_steps first");
     for (int64_t k = 0; k < count; ++k) {
         CUDA_TRY(cudaGraphLaunch(sys->graphs[sys->cur], sys->stream));
-        sys->lastGraph = sys->cur;
         sys->cur ^= 1;
         ++sys->enqueued;
     }
@@ -1859,13 +1846,10 @@ int sph_stage_times(SphSystem *sys, double *ms, int64_t capacity, int64_t *count
     *count = kStageCount;
     if (!ms || capacity < kStageCount) return ms ? fail(SPH_ERR_CAPACITY, "need one entry per stage") : SPH_OK;
     if (!sys->graphs[0] || sys->enqueued == 0) return fail(SPH_ERR_STATE, "no step has run since sph_begin_steps");
+    Control &c = *sys->hCtl;
+    CUDA_TRY(cudaMemcpyAsync(c.stamps, sys->ctl->stamps, sizeof(c.stamps), cudaMemcpyDeviceToHost, sys->stream));
     CUDA_TRY(cudaStreamSynchronize(sys->stream));
-    cudaEvent_t *events = sys->stageEvents[sys->lastGraph];
-    for (int k = 0; k < kStageCount; ++k) {
-        float t = 0.0f;
-        CUDA_TRY(cudaEventElapsedTime(&t, events[k], events[k + 1]));
-        ms[k] = t;
-    }
+    for (int k = 0; k < kStageCount; ++k) ms[k] = 1e-6 * (double)(c.stamps[k + 1] - c.stamps[k]);
     return SPH_OK;
 }
 
@@ -1880,8 +1864,7 @@ int sph_step_launches(SphSystem *sys, int64_t *kernels)
     if (!kernels) return fail(SPH_ERR_INVALID, "null argument");
     *kernels = 0;
     if (!sys->graphs[0]) return fail(SPH_ERR_STATE, "call sph_begin_steps first");
-    // the graph's nodes less its event records (kStageCount + 1 of them)
-    *kernels = sys->graphNodes - (kStageCount + 1);
+    *kernels = sys->graphNodes;
     return SPH_OK;
 }
 

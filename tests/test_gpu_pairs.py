@@ -140,3 +140,32 @@ def test_a_frame_is_the_fluids_rows(n, walls, dim):
     assert positions.dtype == np.float32 and speeds.dtype == np.float32
     assert np.array_equal(positions, x[fluid].astype(np.float32))
     assert np.array_equal(speeds, np.linalg.norm(v[fluid], axis=1).astype(np.float32))
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+@pytest.mark.parametrize('epsilon, filterInterval', [(0.0, 0), (0.5, 0), (0.0, 1)])
+def test_the_stages_of_a_step_follow_one_another(dim, epsilon, filterInterval):
+    # the stamps are of one clock and in order, a stage without a kernel takes no time, and the stages of a
+    # step fit in the time the host waits for it
+    import time
+    from pysurf_b200.state import ContainerBoundary, ParticleState
+    x, v, rho, m, fluid, h = cloud(dim, 2000, 4, ratio=1.3)
+    s = pairSums(dim, h, True)
+    g = np.zeros(dim)
+    g[-1] = -9.81
+    s.setPhysics(RHO0, C0, 0.1, 0.0, g, epsilon, 0.0)
+    state = ParticleState(x, 0.01 * v, np.zeros_like(x), rho, np.zeros(len(x)), m, fluid)
+    s.push(state)
+    s.setBoundary(ContainerBoundary(np.zeros(dim), np.ones(dim), h), state)
+    s.beginSteps(0.0, 0, math.inf, 1 << 30, h, 0.2, 1.0, filterInterval)
+    s.enqueueSteps(3)
+    s.finishSteps()
+    for _ in range(3):
+        start = time.perf_counter()
+        s.enqueueSteps(1)
+        s.finishSteps()
+        span = 1e3 * (time.perf_counter() - start)
+        stages = dict(zip(s.stageNames(), s.stageTimes()))
+        assert all(ms >= 0.0 for ms in stages.values()) and 0.0 < sum(stages.values()) <= span
+        assert stages['cells'] > 0.0 and stages['momentum'] > 0.0 and stages['continuity'] > 0.0
+        assert (stages['filter'] > 0.0) == (filterInterval > 0)

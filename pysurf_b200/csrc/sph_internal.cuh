@@ -63,6 +63,7 @@ struct Params {
     // grid: cell c = (cz * ny + cy) * nx + cx, x fastest; coordinates clamped onto the grid
     double origin[3];
     double cellWidth;
+    double perCell, perFine;    // 1 / cellWidth and 1 / fineWidth, for what needs no cell's exact bound
     int nc[3];
     int ncs;                // cells per support: the stencil is +-ncs cells
     int precise;            // separations from point + remainder (1) or the float32 points alone (0)
@@ -413,10 +414,10 @@ __device__ __forceinline__ CellBox cellBox(const Params &P, int level, int ownCe
     const double width = fine ? P.fineWidth : P.cellWidth;
     const double *origin = fine ? P.fineOrigin : P.origin;
     if (single || (ownCell >= P.fineFirst) == fine) {
-        const int local = ownCell - B.first;
-        B.cx = local % B.nx;
-        B.cy = (local / B.nx) % B.ny;
-        B.cz = local / (B.nx * B.ny);
+        const int local = ownCell - B.first, row = local / B.nx;
+        B.cx = local - row * B.nx;
+        B.cz = dim == 3 ? row / B.ny : 0;
+        B.cy = row - B.cz * B.ny;
         if (image) B.cy = cellCoordinate(pos[1], origin[1], width, B.ny);
     } else {
         B.cx = cellCoordinate(pos[0], origin[0], width, B.nx);

@@ -75,8 +75,13 @@ __device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
 // searches its whole stencil).  The reach carries slack over the coarse test's bound, so every
 // candidate the coarse test passes stays: the accepted neighbours and their order are those of the
 // whole stencil.  PRECISE: separations from point and remainder; MIXED: smoothing lengths differ.
+//
+// Bound by the instructions it issues (74-79% of the issue slots): eight lanes repeat a slot's set-up for its
+// about 150 candidates, so that has no division (the cell's place by one integer quotient, the reach by the
+// grid's reciprocal width), and 2D has no search of an image.  Sort and table on the 122,000-particle beach
+// 0.114 -> 0.107 ms; 0.106 at 11 blocks an SM (40 registers, no spill) in place of 10.
 template <int D, int L, bool PRECISE, bool MIXED>
-__global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
+__global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
     awaitPrevious();
     if (ctl && !ctl->active) return;
@@ -85,7 +90,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
     if (i >= P.n) return;           // a group's lanes share i, so groups leave whole
     const int t = G.t;
     const int shift = (threadIdx.x & 31) & ~(L - 1);
-    const unsigned lower = (1u << t) - 1u;
+    const unsigned lower = G.mask & ((1u << (threadIdx.x & 31)) - 1u);
     const float4 Ai = fetch(&F.pa[i]), Bi = fetch(&F.pb[i]);
     const float hI = fabsf(signedLengthIn<D>(Ai, Bi));
     // a boundary row holds its fluid neighbours only (Row says why)
@@ -108,23 +113,22 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
     int *column = F.nbr + 4 * (size_t)i;
     int count = 0, wallCount = 0;
     // search s: grid level s >> 1 (coarse, fine), origin s & 1 (the particle, its periodic image)
-    for (int search = 0; search < (MIXED ? 4 : 2); ++search) {
-        const int level = MIXED ? search >> 1 : 0, image = search & 1;
+    for (int search = 0; search < (MIXED ? 4 : 2); search += D == 2 ? 2 : 1) {
+        const int level = MIXED ? search >> 1 : 0, image = D == 3 ? search & 1 : 0;
         if (level >= P.levels || (image && !seam)) continue;
         const double pos[3] = {(double)pi[0] + (double)li[0], (double)pi[1] + (double)li[1] + (image ? shift64 : 0.0),
                                D == 3 ? (double)pi[2] + (double)li[2] : 0.0};
         const CellBox box = cellBox(P, level, ownCell, pos, image != 0, D, searchCells(P, level, hI), !MIXED);
         const float searchLimit = level ? fineLimit : limit;
-        const double width = level ? P.fineWidth : P.cellWidth;
+        const double perWidth = level ? P.perFine : P.perCell;
         const double *origin = level ? P.fineOrigin : P.origin;
         // the particle's place in the centre cell, in cell widths, and the reach in cell widths with slack
-        const float invW = (float)(1.0 / width);
-        const float fx = (float)(((double)pi[0] - origin[0]) / width) - (float)box.cx;
-        const float fz = D == 3 ? (float)(((double)pi[2] - origin[2]) / width) - (float)box.cz : 0.5f;
-        const float R = (1.001f * sqrtf(searchLimit) + 5.0e-7f * (fabsf(pi[0]) + fabsf(pi[1]) + fabsf(pi[2]))) * invW +
-                        1.0e-3f;
+        const float fx = (float)(((double)pi[0] - origin[0]) * perWidth - box.cx);
+        const float fz = D == 3 ? (float)(((double)pi[2] - origin[2]) * perWidth - box.cz) : 0.5f;
+        const float R = (1.001f * sqrtf(searchLimit) + 5.0e-7f * (fabsf(pi[0]) + fabsf(pi[1]) + fabsf(pi[2]))) *
+                            (float)perWidth + 1.0e-3f;
         const float offset = image ? (float)shift64 : 0.0f;
-        const float fy = (float)(((double)pi[1] + (image ? shift64 : 0.0) - origin[1]) / width) - (float)box.cy;
+        const float fy = (float)(((double)pi[1] + (image ? shift64 : 0.0) - origin[1]) * perWidth - box.cy);
         const bool trim = SPH_LIST_TRIM && fx >= 0.0f && fx < 1.0f && fy >= 0.0f && fy < 1.0f && fz >= 0.0f &&
                           fz < 1.0f;
         // one run of candidates, L at a time; WALLED: it holds boundary slots
@@ -153,10 +157,9 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
                         accepted = r2 < bound;
                     }
                 }
-                const unsigned all = (L >= 32 ? 0u : 1u << L) - 1u;
                 const bool front = !WALLED || fluidJ || P.together;
-                const unsigned bits = (__ballot_sync(G.mask, accepted) >> shift) & all;
-                const unsigned walls = WALLED ? (__ballot_sync(G.mask, accepted && !front) >> shift) & all : 0u;
+                const unsigned bits = __ballot_sync(G.mask, accepted) & G.mask;
+                const unsigned walls = WALLED ? __ballot_sync(G.mask, accepted && !front) & G.mask : 0u;
                 if (accepted) {
                     const int k = front ? count + __popc(bits & ~walls & lower) : wallCount + __popc(walls & lower);
                     if (k < P.listCap) {
@@ -169,12 +172,13 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 10 : 1) listKernel(
             }
         };
         // lane t takes the run of every L-th stencil row, trimmed; the group then walks the rows in order
-        const int across = box.y1 - box.y0 + 1, rows = across * (box.z1 - box.z0 + 1);
+        const int across = box.y1 - box.y0 + 1, rows = D == 3 ? across * (box.z1 - box.z0 + 1) : across;
         for (int block = 0; block < rows; block += L) {
             int runFirst = 0, runEnd = 0;
             bool runWalls = false;
             if (block + t < rows) {
-                const int zz = box.z0 + (D == 3 ? (block + t) / across : 0), yy = box.y0 + (block + t) % across;
+                const int zz = D == 3 ? box.z0 + (block + t) / across : 0;
+                const int yy = box.y0 + (D == 3 ? (block + t) % across : block + t);
                 int xa = box.x0, xb = box.x1;
                 bool empty = false;
                 if (trim) {
@@ -314,14 +318,19 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                                            (double)pip[1] + (double)lip[1] + (image ? shiftp : 0.0),
                                            D == 3 ? (double)pip[2] + (double)lip[2] : 0.0};
                     box = cellBox(P, level, ownCell, pos, image != 0, D, searchCells(P, level, hIp), !MIXED);
-                    const double width = level ? P.fineWidth : P.cellWidth;
+                    const double width = level ? P.fineWidth : P.cellWidth, perWidth = level ? P.perFine : P.perCell;
                     const double *origin = level ? P.fineOrigin : P.origin;
-                    const float invW = (float)(1.0 / width);
-                    fx = (float)(((double)pip[0] - origin[0]) / width) - (float)box.cx;
-                    fz = D == 3 ? (float)(((double)pip[2] - origin[2]) / width) - (float)box.cz : 0.5f;
-                    fy = (float)(((double)pip[1] + (image ? shiftp : 0.0) - origin[1]) / width) - (float)box.cy;
-                    R = (1.001f * sqrtf(lim) + 5.0e-7f * (fabsf(pip[0]) + fabsf(pip[1]) + fabsf(pip[2]))) * invW +
-                        1.0e-3f;
+                    // A place in a cell, by the reciprocal where lengths differ (the refined 11-ppd ridge's
+                    // table 9.34 -> 8.55 ms).  With one length the compiler fits the division's form in 64
+                    // registers and the reciprocal's in 72 (the 10-ppd ridge's table 3.15 ms against 3.31).
+                    auto placed = [&](double x, int cell) {
+                        return MIXED ? (float)(x * perWidth - cell) : (float)(x / width) - (float)cell;
+                    };
+                    fx = placed((double)pip[0] - origin[0], box.cx);
+                    fz = D == 3 ? placed((double)pip[2] - origin[2], box.cz) : 0.5f;
+                    fy = placed((double)pip[1] + (image ? shiftp : 0.0) - origin[1], box.cy);
+                    R = (1.001f * sqrtf(lim) + 5.0e-7f * (fabsf(pip[0]) + fabsf(pip[1]) + fabsf(pip[2]))) *
+                            (MIXED ? (float)perWidth : (float)(1.0 / width)) + 1.0e-3f;
                     trim = SPH_LIST_TRIM && fx >= 0.0f && fx < 1.0f && fy >= 0.0f && fy < 1.0f && fz >= 0.0f &&
                            fz < 1.0f;
                 }

@@ -462,11 +462,13 @@ struct SphSystem {
         P.sigmaUnit = (float)sigmaUnit(kind, dim);
         for (int a = 0; a < 3; ++a) { P.origin[a] = origin[a]; P.nc[a] = nc[a]; }
         P.cellWidth = cellWidth;
+        P.perCell = 1.0 / cellWidth;
         P.ncs = ncs;
         P.precise = precise;
         P.levels = levels;
         for (int a = 0; a < 3; ++a) { P.fineOrigin[a] = fineOrigin[a]; P.fineNc[a] = fineNc[a]; }
         P.fineWidth = fineWidth;
+        P.perFine = fineWidth > 0.0 ? 1.0 / fineWidth : 0.0;
         P.fineFirst = numCells;
         P.cells = numCells + fineCells;
         P.fineMax = (float)fineMax;

@@ -78,7 +78,7 @@ __device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
 //
 // Bound by the instructions it issues (74-79% of the issue slots): eight lanes repeat a slot's set-up for its
 // about 150 candidates, so that has no division (the cell's place by one integer quotient, the reach by the
-// grid's reciprocal width), and 2D has no search of an image.  Sort and table on the 122,000-particle beach
+// grid's reciprocal width), and 2D has no search of an image.  Sort and table on the 114,000-particle beach
 // 0.114 -> 0.107 ms; 0.106 at 11 blocks an SM (40 registers, no spill) in place of 10.
 template <int D, int L, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(Params P, Frame F, const Control *ctl, int *maxCount)
@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(
         const float R = (1.001f * sqrtf(searchLimit) + 5.0e-7f * (fabsf(pi[0]) + fabsf(pi[1]) + fabsf(pi[2]))) *
                             (float)perWidth + 1.0e-3f;
         const float offset = image ? (float)shift64 : 0.0f;
+        const float at[3] = {pi[0], image ? __fadd_rn(pi[1], offset) : pi[1], pi[2]};     // the search's origin
         const float fy = (float)(((double)pi[1] + (image ? shift64 : 0.0) - origin[1]) * perWidth - box.cy);
         const bool trim = SPH_LIST_TRIM && fx >= 0.0f && fx < 1.0f && fy >= 0.0f && fy < 1.0f && fz >= 0.0f &&
                           fz < 1.0f;
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(
                     float pj[3];
                     pointIn<D>(A, pj);
                     if (WALLED) fluidJ = isFluid(F, j);
-                    const float coarse = !WALLED || fluidJ || !fluidOnly ? coarseDistance2<D>(pi, pj, offset) : searchLimit;
+                    const float coarse = !WALLED || fluidJ || !fluidOnly ? coarseDistance2<D>(at, pj) : searchLimit;
                     if (PRECISE && !image && level == 0 && coarse < sure) {
                         accepted = true;
                     } else if (coarse < searchLimit) {
@@ -233,13 +234,17 @@ struct alignas(16) BatchMember {
     float4 rest;        // the remainder; w: this search's coarse limit
     float4 bounds;      // the limit on the coarse grid, on the fine grid, the sure bound, hI
     double shift64;     // the periodic image's shift (0 when it is not searched)
-    float offset;       // the shift as float32
+    float y;            // point.y before the image's shift, which it takes with one length
     int walls;          // its boundary neighbours so far
 };
 
+// Bound by the instructions it issues, most of them a member's test of a candidate.  So a member's point is
+// kept as the search sees it (moved across the seam already), and a candidate surely inside or outside the
+// support leaves the test without a load of the member's other rows: the 760,000-particle ridge's sort and
+// table 3.15 -> 2.86 ms, the refined 11-ppd ridge's 8.55 -> 8.20, the 27,000-particle channel's 0.278 ->
+// 0.263.  Two members' distances at a time in packed float32 took 96 registers and 3.7 ms.
 // No blocks-a-multiprocessor bound: the compiler's own choice, 64 registers with a few spills at one
-// smoothing length, builds the 20-ppd ridge's table in 20.4 ms, against 22.1 to 23.8 at bounds of 7 to 9
-// blocks that spill none.
+// smoothing length, against 3.28 ms at 8 blocks and 4.57 at 1 (118 registers, no spill).
 template <int D, int kBatch, bool PRECISE, bool MIXED>
 __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, const Control *ctl, int *maxCount)
 {
@@ -252,6 +257,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
     const int first = warp * kBatch;
     if (first >= P.n) return;               // whole warps leave together
     const int last = min(first + kBatch, P.n);
+    const float oneReach = 2.0f * P.hMax, oneLimit = kCandidateMargin * oneReach * oneReach;
     const unsigned lower = (1u << lane) - 1u;
     const float support = MIXED ? 0.0f : support2(P.hMax);
     // the batches that start in this warp's slots
@@ -290,7 +296,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
             m.bounds = make_float4(kCandidateMargin * reach * reach, kCandidateMargin * fineReach * fineReach,
                                    PRECISE ? sureBound(P, support, hIp, pip) : 0.0f, hIp);
             m.shift64 = shiftp;
-            m.offset = (float)shiftp;
+            m.y = pip[1];
         }
         const bool anySeam = __any_sync(0xFFFFFFFFu, seamp);
         // the members that take boundary neighbours: a boundary member's row holds fluid neighbours only
@@ -313,6 +319,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                 const float lim = level ? bounds.y : bounds.x;
                 mine[lane].point.w = PRECISE && !image && level == 0 ? bounds.z : 0.0f;
                 mine[lane].rest.w = lim;
+                if (!MIXED && image) mine[lane].point.y = __fadd_rn(pip[1], (float)shiftp);
                 if (takes) {
                     const double pos[3] = {(double)pip[0] + (double)lip[0],
                                            (double)pip[1] + (double)lip[1] + (image ? shiftp : 0.0),
@@ -378,7 +385,7 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                         const int j = base + lane;
                         float4 A = make_float4(0, 0, 0, 0), B = A;
                         float pj[3] = {0, 0, 0}, lj[3] = {0, 0, 0}, hJ = 0.0f;
-                        bool fluidJ = false;
+                        bool fluidJ = true;
                         unsigned offered = 0;       // the members this candidate is offered to
                         if (j < uB) {
                             A = fetch(&F.pa[j]);
@@ -400,26 +407,25 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
                             if (!(takers >> p & 1)) continue;       // the whole warp
                             const float4 point = mine[p].point;
                             const float mp[3] = {point.x, point.y, point.z};
-                            const float offset = image ? mine[p].offset : 0.0f;
-                            const float coarse = coarseDistance2<D>(mp, pj, offset);
-                            bool accepted = false;
-                            if (offered >> p & 1) {
-                                if (PRECISE && coarse < point.w) {
-                                    accepted = true;
-                                } else {
-                                    const float4 rest = mine[p].rest;
-                                    if (coarse < rest.w) {
-                                        float r2 = coarse;
-                                        if (PRECISE) {
-                                            const float ml[3] = {rest.x, rest.y, rest.z};
-                                            float d[3];
-                                            r2 = separation2<D, 1>(P, mp, ml, pj, lj, offset, image,
-                                                                   image ? mine[p].shift64 : 0.0, d);
-                                        }
-                                        const float bound =
-                                            MIXED ? support2(0.5f * (mine[p].bounds.w + hJ)) : support;
-                                        accepted = r2 < bound;
+                            const float coarse = MIXED ? coarseDistance2<D>(mp, pj, image ? (float)mine[p].shift64 : 0.0f)
+                                                       : coarseDistance2<D>(mp, pj);
+                            const bool offer = offered >> p & 1;
+                            bool accepted = PRECISE && offer && coarse < point.w;
+                            // With one length the search's limit is every member's, so that the whole warp
+                            // passes over this but for a candidate near the edge of the support.
+                            if (offer && !accepted && (MIXED || coarse < oneLimit)) {
+                                const float4 rest = mine[p].rest;
+                                if (!MIXED || coarse < rest.w) {
+                                    float r2 = coarse;
+                                    if (PRECISE) {
+                                        const float own[3] = {point.x, !MIXED && image ? mine[p].y : point.y, point.z};
+                                        const float ml[3] = {rest.x, rest.y, rest.z};
+                                        float d[3];
+                                        r2 = separation2<D, 1>(P, own, ml, pj, lj, 0.0f, image,
+                                                               image ? mine[p].shift64 : 0.0, d);
                                     }
+                                    const float bound = MIXED ? support2(0.5f * (mine[p].bounds.w + hJ)) : support;
+                                    accepted = r2 < bound;
                                 }
                             }
                             const unsigned bits = __ballot_sync(0xFFFFFFFFu, accepted);

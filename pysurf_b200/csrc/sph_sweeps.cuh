@@ -125,15 +125,22 @@ __device__ __forceinline__ float groupSumCompensated(const float2 &s, const floa
 // test is r^2 < (2 h)^2, so a rejected candidate takes no square root; it parts from the
 // reference's r < 2 h only where the two roundings straddle 2 h, where W and grad W vanish.
 template <int D>
-__device__ __forceinline__ float coarseDistance2(const float pi[3], const float pj[3], float offset)
+__device__ __forceinline__ float coarseDistance2(const float pi[3], const float pj[3])
 {
-    const float cx = __fsub_rn(pi[0], pj[0]), cy = __fsub_rn(__fadd_rn(pi[1], offset), pj[1]);
+    const float cx = __fsub_rn(pi[0], pj[0]), cy = __fsub_rn(pi[1], pj[1]);
     float r2 = __fadd_rn(__fmul_rn(cx, cx), __fmul_rn(cy, cy));
     if (D == 3) {
         const float cz = __fsub_rn(pi[2], pj[2]);
         r2 = __fadd_rn(r2, __fmul_rn(cz, cz));
     }
     return r2;
+}
+// From pi moved by offset across the periodic seam.
+template <int D>
+__device__ __forceinline__ float coarseDistance2(const float pi[3], const float pj[3], float offset)
+{
+    const float at[3] = {pi[0], __fadd_rn(pi[1], offset), pi[2]};
+    return coarseDistance2<D>(at, pj);
 }
 
 // d = x_i - x_j from the points and remainders (image: across the periodic seam, in float64); r^2.

@@ -87,6 +87,18 @@ def test_mixed_lengths(dim):
     sameBits(*(sums(pairSums(dim, h, table), x, v, rho, m, fluid, lengths) for table in (False, True)))
 
 
+@pytest.mark.parametrize('precision', ['float64', 'float32'])
+@pytest.mark.parametrize('mixed', [False, True])
+@pytest.mark.parametrize('n', [700, 1201])
+def test_the_table_across_the_seam(n, mixed, precision):
+    # the table moves a batch's points across the seam (one length) or each distance (mixed): both searches
+    # of a periodic axis, on one grid level and on two, find the walk's neighbours
+    x, v, rho, m, fluid, h = cloud(3, n, n, ratio=1.7)
+    lengths = np.where(np.random.default_rng(5).uniform(size=n) < 0.5, h, 0.5 * h) if mixed else None
+    sameBits(*(sums(pairSums(3, h, table, period=1.0, precision=precision), x, v, rho, m, fluid, lengths)
+               for table in (False, True)))
+
+
 @pytest.mark.parametrize('dim, n', [(2, 24575), (2, 24576), (3, 65535), (3, 65536)])
 def test_the_tables_lanes_and_batches(dim, n):
     # either side of the sizes at which the table kernel takes other lanes (2D) or batches (3D)

@@ -169,6 +169,7 @@ struct SphSystem {
     size_t nbrEntries = 0;
     int listCap = 0;
     bool listTogether = false;  // the rows' order as built (Params::together)
+    bool graphTogether = false; // the rows' order the captured steps build
     int tableMode = 1;          // 0 never build the table, 1 build it when it fits the budget
     bool listDirty = true;      // the table's size must be taken again before the next step
     int listSizedFor = -1;      // the particle count the table's size was taken for
@@ -733,14 +734,20 @@ int sph_create(int dimensions, double smoothing_length, const double *domain_min
     return SPH_OK;
 }
 
+static void destroyGraphs(SphSystem *sys)
+{
+    for (int b = 0; b < 2; ++b) {
+        if (sys->graphs[b]) cudaGraphExecDestroy(sys->graphs[b]);
+        sys->graphs[b] = nullptr;
+    }
+}
+
 int sph_destroy(SphSystem *sys)
 {
     if (!sys) return SPH_OK;
     cudaSetDevice(sys->device);
     if (sys->stream) cudaStreamSynchronize(sys->stream);
-    for (int b = 0; b < 2; ++b) {
-        if (sys->graphs[b]) cudaGraphExecDestroy(sys->graphs[b]);
-    }
+    destroyGraphs(sys);
     sys->freeArrays();
     cudaFree(sys->energy);
     cudaFree(sys->parts);
@@ -1692,33 +1699,47 @@ int sph_resident_integrate(SphSystem *sys, double time_step)
     return SPH_OK;
 }
 
+// Captures and instantiates the step from master buffer `buffer`.
+static int captureStep(SphSystem *sys, int buffer, bool filter)
+{
+    sys->cur = buffer;
+    cudaGraph_t g;
+    CUDA_TRY(cudaStreamBeginCapture(sys->stream, cudaStreamCaptureModeThreadLocal));
+    enqueueRates(sys, filter);
+    enqueueIntegrate(sys);
+    launchStepEnd(sys->ctl, sys->stream);
+    cudaError_t err = cudaStreamEndCapture(sys->stream, &g);
+    if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(err));
+    err = cudaGraphInstantiate(&sys->graphs[buffer], g, 0);
+    if (err == cudaSuccess) {
+        size_t nodes = 0;
+        cudaGraphGetNodes(g, nullptr, &nodes);
+        sys->graphNodes = (int)nodes;
+    }
+    cudaGraphDestroy(g);
+    if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(err));
+    return SPH_OK;
+}
+
 // Two single-step graphs, one from each master buffer (a step moves the master to the other
-// buffer).
+// buffer).  Capturing runs nothing, so what the handle notes of work done (the buffer, the frame, the
+// cells, the rows' order) stays as it was; sph_finish_steps notes it once a step has run.
 static int captureSteps(SphSystem *sys, bool filter)
 {
-    for (int b = 0; b < 2; ++b) {
-        if (sys->graphs[b]) { cudaGraphExecDestroy(sys->graphs[b]); sys->graphs[b] = nullptr; }
+    destroyGraphs(sys);
+    const int cur = sys->cur;
+    const bool framed = sys->framed, cellsFresh = sys->cellsFresh, listTogether = sys->listTogether;
+    int status = SPH_OK;
+    for (int b = 0; b < 2 && status == SPH_OK; ++b) status = captureStep(sys, b, filter);
+    sys->cur = cur;
+    sys->framed = framed;
+    sys->cellsFresh = cellsFresh;
+    sys->listTogether = listTogether;
+    if (status != SPH_OK) {
+        destroyGraphs(sys);
+        return status;
     }
-    const int keep = sys->cur;
-    for (int b = 0; b < 2; ++b) {
-        sys->cur = b;
-        cudaGraph_t g;
-        CUDA_TRY(cudaStreamBeginCapture(sys->stream, cudaStreamCaptureModeThreadLocal));
-        enqueueRates(sys, filter);
-        enqueueIntegrate(sys);
-        launchStepEnd(sys->ctl, sys->stream);
-        cudaError_t err = cudaStreamEndCapture(sys->stream, &g);
-        if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(err));
-        err = cudaGraphInstantiate(&sys->graphs[b], g, 0);
-        if (err == cudaSuccess) {
-            size_t nodes = 0;
-            cudaGraphGetNodes(g, nullptr, &nodes);
-            sys->graphNodes = (int)nodes;
-        }
-        cudaGraphDestroy(g);
-        if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(err));
-    }
-    sys->cur = keep;
+    sys->graphTogether = sys->classic();
     sys->graphFilter = filter;
     sys->graphDirty = false;
     return SPH_OK;
@@ -1787,6 +1808,10 @@ int sph_finish_steps(SphSystem *sys, double *time, int64_t *step, double *last_d
         const Control &c = *sys->hCtl;
         sys->cur = sys->beginCur ^ (int)((c.step - sys->beginStep) & 1);
         sys->cellsFresh = false;
+        if (c.step != sys->beginStep) {
+            sys->framed = true;
+            sys->listTogether = sys->graphTogether;
+        }
     }
     const Control &c = *sys->hCtl;
     if (time) *time = c.time;

@@ -1,0 +1,76 @@
+"""What a handle holds after the calls that set a step up without running it, and after those that drive
+steps from the host: the neighbour table's order, the frame and the stage stamps stay those of work done."""
+import math
+
+import numpy as np
+import pytest
+
+from test_gpu_pairs import C0, RHO0, cloud, pairSums
+
+pytestmark = pytest.mark.gpu
+
+
+def steppedHandle(dim, table, limited, threads=4):
+    """A handle with half its cloud boundary and XSPH on, at rest but for a small noise, pushed; its state."""
+    from pysurf_b200.state import ContainerBoundary, ParticleState
+    x, v, rho, m, fluid, h = cloud(dim, 500, 17 + dim, walls=0.5, ratio=1.6)
+    s = pairSums(dim, h, table, threads, kernel='cubicSpline', diffusion='none', corrected=False, limited=limited)
+    g = np.zeros(dim)
+    g[-1] = -9.81
+    s.setPhysics(RHO0, C0, 0.1, 0.0, g, 0.5, 0.0)
+    state = ParticleState(x.copy(), 0.01 * v, np.zeros_like(x), rho.copy(), np.zeros(len(x)), m, fluid)
+    s.push(state)
+    s.setBoundary(ContainerBoundary(np.zeros(dim), np.ones(dim), h), state)
+    return s, state, h
+
+
+def hostSums(s, state, dim):
+    g = np.zeros(dim)
+    g[-1] = -9.81
+    v, rho = state.velocities, state.densities
+    p = C0 ** 2 * (rho - RHO0)
+    return {'acceleration': s.pairAccelerations(v, rho, p, C0, 0.05, 0.5, g), 'rate': s.continuityRate(v, rho),
+            'wall': s.wallPressure(rho, p, g, RHO0, C0), 'shepard': s.shepardDensity(rho),
+            'xsph': s.xsphVelocity(v, rho, 0.5)}
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+@pytest.mark.parametrize('limited', [False, True])
+@pytest.mark.parametrize('stepless', ['advance', 'beginSteps', 'none'])
+def test_a_step_that_is_only_set_up_leaves_the_rows_as_they_are(dim, limited, stepless):
+    # rows built in one scheme's order, the scheme turned over, a run that is already over: the host sums
+    # after it read the rows in the order they were built in, whatever the captured step would build
+    runs = []
+    for table in (False, True):
+        s, state, h = steppedHandle(dim, table, limited)
+        s.residentRates(False)
+        s.setViscosityLimiter(not limited)
+        if stepless == 'advance':
+            assert s.advance(1.0, 7, 1.0, 1 << 40, h, 0.2, 1.0)[:2] == (1.0, 7)
+        elif stepless == 'beginSteps':
+            s.beginSteps(1.0, 7, 1.0, 1 << 40, h, 0.2, 1.0)
+        runs.append(hostSums(s, state, dim))
+    for name in runs[0]:
+        assert np.array_equal(runs[0][name], runs[1][name]), name
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+def test_every_span_leaves_the_pressures_of_its_last_step(dim):
+    # the frame a step leaves is in the master's order whether or not the span captured its graph: the
+    # second span of a handle pulls the pressures that the host-driven step has too
+    pulled = []
+    for drive in ('device', 'host'):
+        s, state, h = steppedHandle(dim, True, True)
+        for _ in range(2):
+            s.push(state)
+            if drive == 'device':
+                _, _, dt = s.advance(0.0, 0, math.inf, 1, h, 0.2, 1.0)
+            else:
+                s.residentRates(False)
+                s.residentIntegrate(dt)
+            out = state.copy()
+            s.pull(out)
+            pulled.append(out)
+    for other in pulled[1:]:
+        for name in ('positions', 'velocities', 'densities', 'pressures', 'accelerations'):
+            assert np.array_equal(getattr(pulled[0], name), getattr(other, name)), name

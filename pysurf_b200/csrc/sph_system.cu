@@ -1581,13 +1581,15 @@ static const char *const kStageNames[kStageCount] = {"cells", "filter", "wall", 
 
 // The first half of a step: cell list, optional filter, wall pressure, gradients, momentum.
 // filter: the Shepard stage is enqueued (the device decides each step whether it is due).
-static void enqueueRates(SphSystem *sys, bool filter)
+// stamped: the stages note their start (Control::stamps).  Only the device loop's steps do, which have an
+// end to note too; the stamps of its last step outlive steps that the host drives.
+static void enqueueRates(SphSystem *sys, bool filter, bool stamped)
 {
-    sys->rebuild(sys->ctl, 1 << 0);
+    sys->rebuild(sys->ctl, stamped ? 1 << 0 : 0);
     LaunchArgs A = sys->args(sys->ctl);
     int begins = 1 << 1;        // the stages that begin with the next launch
     auto launch = [&](Stage stage) {
-        A.P.stages = begins;
+        A.P.stages = stamped ? begins : 0;
         launchStage(A, stage);
         A.P.stages = begins = 0;
     };
@@ -1616,12 +1618,12 @@ static void enqueueRates(SphSystem *sys, bool filter)
 }
 
 // The second half: kick, continuity with the density update, XSPH, drift and enforcement.
-static void enqueueIntegrate(SphSystem *sys)
+static void enqueueIntegrate(SphSystem *sys, bool stamped)
 {
     LaunchArgs A = sys->args(sys->ctl);
-    A.P.stages = 1 << 5;
+    A.P.stages = stamped ? 1 << 5 : 0;
     launchStage(A, Stage::Kick);
-    A.P.stages = 1 << 6;
+    A.P.stages = stamped ? 1 << 6 : 0;
     // the density update; with neither shifting nor XSPH to come, the drift and the enforcement too
     const bool drifts = !sys->shifting && !(sys->xsphEpsilon > 0.0);
     A.flag = drifts ? 2 : 1;
@@ -1672,7 +1674,7 @@ int sph_resident_rates(SphSystem *sys, int filter_density, double *max_speed, do
     }
     if (sys->listDirty) TRY(sys->sizeList());
     TRY(sys->writeControl());
-    enqueueRates(sys, filter_density != 0);
+    enqueueRates(sys, filter_density != 0, false);
     CUDA_TRY(cudaGetLastError());
     TRY(sys->readError());
     if (max_speed) *max_speed = sys->hCtl->vmax;
@@ -1692,7 +1694,7 @@ int sph_resident_integrate(SphSystem *sys, double time_step)
     c.dt = time_step;
     c.error = 0;
     TRY(sys->writeControl());
-    enqueueIntegrate(sys);
+    enqueueIntegrate(sys, false);
     CUDA_TRY(cudaGetLastError());
     TRY(sys->readError());
     sys->cellsFresh = false;
@@ -1705,8 +1707,8 @@ static int captureStep(SphSystem *sys, int buffer, bool filter)
     sys->cur = buffer;
     cudaGraph_t g;
     CUDA_TRY(cudaStreamBeginCapture(sys->stream, cudaStreamCaptureModeThreadLocal));
-    enqueueRates(sys, filter);
-    enqueueIntegrate(sys);
+    enqueueRates(sys, filter, true);
+    enqueueIntegrate(sys, true);
     launchStepEnd(sys->ctl, sys->stream);
     cudaError_t err = cudaStreamEndCapture(sys->stream, &g);
     if (err != cudaSuccess) return fail(SPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(err));

@@ -74,3 +74,20 @@ def test_every_span_leaves_the_pressures_of_its_last_step(dim):
     for other in pulled[1:]:
         for name in ('positions', 'velocities', 'densities', 'pressures', 'accelerations'):
             assert np.array_equal(getattr(pulled[0], name), getattr(other, name)), name
+
+
+@pytest.mark.parametrize('filterInterval', [0, 1])
+@pytest.mark.parametrize('halves', [1, 2])
+def test_stage_times_are_of_one_step(filterInterval, halves):
+    # stage times are the device loop's last step's: the halves of a step that the host drives after it
+    # change none of them
+    s, state, h = steppedHandle(2, True, True)
+    time, step, dt = s.advance(0.0, 0, math.inf, 2, h, 0.2, 1.0, filterInterval)
+    before = s.stageTimes()
+    assert all(0.0 <= ms < 1e3 for ms in before) and sum(before) > 0.0
+    s.residentRates(filterInterval > 0)
+    if halves == 2:
+        s.residentIntegrate(dt)
+    assert s.stageTimes() == before
+    s.advance(time, step, math.inf, step + 1, h, 0.2, 1.0, filterInterval, dt)
+    assert all(0.0 <= ms < 1e3 for ms in s.stageTimes())

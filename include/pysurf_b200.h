@@ -186,8 +186,9 @@ int sph_count(const SphSystem *sys, int64_t *n);
  * particle in 3D cross the bus instead of a float64 pull's 48. */
 int sph_frame(SphSystem *sys, float *positions, float *speeds, uint8_t *is_fluid);
 /* The same frame of the fluid alone, its rows packed on the device in caller order: sph_fluid_frame
- * packs them and returns how many there are, sph_fluid_frame_rows, the next call on the handle, copies
- * them out (positions count x dim, speeds count). */
+ * packs them and returns how many there are, sph_fluid_frame_rows copies the first `count` of them out
+ * (positions count x dim, speeds count).  The rows wait in memory that other calls use too: once one has,
+ * sph_fluid_frame_rows fails with SPH_ERR_STATE. */
 int sph_fluid_frame(SphSystem *sys, int64_t *count);
 int sph_fluid_frame_rows(SphSystem *sys, float *positions, float *speeds, int64_t count);
 

@@ -157,6 +157,7 @@ struct SphSystem {
     static constexpr int kStageSlots = 14;
     static constexpr int kOutSlot = 5;
     double *dStage = nullptr;
+    int64_t packedRows = -1;    // the rows sph_fluid_frame left in the output staging; -1 once it is used again
     uint8_t *dStageU8 = nullptr;
     int *dRank = nullptr;
     Control *hCtl = nullptr;    // pinned
@@ -219,6 +220,7 @@ struct SphSystem {
         sortBuffers.slotCell = sortBuffers.slotWithin = sortBuffers.perm = nullptr;
         sortBuffers.bucket = nullptr;
         dStage = nullptr; dStageU8 = nullptr; dRank = nullptr;
+        packedRows = -1;
         capacity = 0;
         return SPH_OK;
     }
@@ -648,7 +650,14 @@ struct SphSystem {
         return SPH_OK;
     }
 
-    double *stage(int slot) const { return dStage + (size_t)slot * capacity; }
+    double *stage(int slot)
+    {
+        packedRows = -1;
+        return staged(slot);
+    }
+
+    // The same to read what a call before left there.
+    double *staged(int slot) const { return dStage + (size_t)slot * capacity; }
 
     int readError()
     {
@@ -1384,8 +1393,8 @@ int sph_frame(SphSystem *sys, float *positions, float *speeds, uint8_t *is_fluid
 }
 
 // float32 rows in the output staging: positions, then speeds; the tiles' counts past them
-static float *framePositions(SphSystem *sys) { return reinterpret_cast<float *>(sys->stage(SphSystem::kOutSlot)); }
-static float *frameSpeeds(SphSystem *sys) { return reinterpret_cast<float *>(sys->stage(SphSystem::kOutSlot + 2)); }
+static float *framePositions(SphSystem *sys) { return reinterpret_cast<float *>(sys->staged(SphSystem::kOutSlot)); }
+static float *frameSpeeds(SphSystem *sys) { return reinterpret_cast<float *>(sys->staged(SphSystem::kOutSlot + 2)); }
 
 int sph_fluid_frame(SphSystem *sys, int64_t *count)
 {
@@ -1400,7 +1409,7 @@ int sph_fluid_frame(SphSystem *sys, int64_t *count)
     CUDA_TRY(cudaGetLastError());
     TRY(sys->download(&rows, counts + frameTiles(sys->n), sizeof(int)));
     CUDA_TRY(cudaStreamSynchronize(sys->stream));
-    *count = rows;
+    *count = sys->packedRows = rows;
     return SPH_OK;
 }
 
@@ -1411,6 +1420,8 @@ int sph_fluid_frame_rows(SphSystem *sys, float *positions, float *speeds, int64_
     if (count == 0) return SPH_OK;
     if (!positions || !speeds) return fail(SPH_ERR_INVALID, "null argument");
     if (!sys->resident) return fail(SPH_ERR_STATE, "no device state: call sph_push first");
+    if (sys->packedRows < 0) return fail(SPH_ERR_STATE, "no frame is packed: call sph_fluid_frame first");
+    if (count > sys->packedRows) return fail(SPH_ERR_INVALID, "more rows than the packed frame has");
     TRY(sys->download(positions, framePositions(sys), sizeof(float) * (size_t)count * sys->dim));
     TRY(sys->download(speeds, frameSpeeds(sys), sizeof(float) * (size_t)count));
     CUDA_TRY(cudaStreamSynchronize(sys->stream));

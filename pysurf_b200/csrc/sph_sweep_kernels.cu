@@ -637,10 +637,7 @@ struct GradientVisit {
                     dd[a] = (double)(q ? N.d[a].y : N.d[a].x);
                     r2 = fma(dd[a], dd[a], r2);
                 }
-                // the root by one Newton step from float32's: r + (r2 - r^2) / (2 r), the small correction's
-                // divisor in float32
-                const double rf = (double)(q ? N.r.y : N.r.x);
-                const double rr = fma(fma(-rf, rf, r2), (double)(0.5f * (q ? N.inverse.y : N.inverse.x)), rf);
+                const double rr = preciseRoot(r2, q ? N.inverse.y : N.inverse.x);
                 const double w64 = (double)volume[q] * kernelGradient64<K>(rr, N.k.of(q));
                 for (int a = 0; a < D; ++a) {
                     const double wa = -w64 * dd[a];
@@ -1192,16 +1189,14 @@ struct ContinuityVisit {
         if (!(sum > 0.0f)) return 0.0f;
         return __fmul_rn(__fmul_rn(2.0f, P.closureC0), __fdiv_rn(__fmul_rn(__fmul_rn(2.0f, deltaI), deltaJ), sum));
     }
-    // A fluid-boundary pair, in float64: the distance by one Newton step from the float32 root (its small
-    // correction's divisor in float32), (dW/dr) / r.
+    // A fluid-boundary pair, in float64.
     template <int Q>
     __device__ __forceinline__ void wallPair(const Neighbours &N, const CrossTaken &taken)
     {
         const double *dd = taken.dd[Q], *dv = taken.dv[Q];
         double r2 = 0.0;
         for (int a = 0; a < D; ++a) r2 = fma(dd[a], dd[a], r2);
-        const double rf = (double)(Q ? N.r.y : N.r.x);
-        const double rr = fma(fma(-rf, rf, r2), (double)(0.5f * (Q ? N.inverse.y : N.inverse.x)), rf);
+        const double rr = preciseRoot(r2, Q ? N.inverse.y : N.inverse.x);
         const double weight = __dmul_rn((double)taken.mass[Q], kernelGradient64<K>(rr, N.k.of(Q)));
         if (corrected) {
             for (int a = 0; a < D; ++a) {

@@ -178,8 +178,7 @@ __device__ __forceinline__ float2 fma2(const float2 &a, const float2 &b, const f
 // A pair's distance from its squared distance: r^2 times the hardware reciprocal square root (about 2
 // ulp), 0 for a coincident pair, and that reciprocal (finite always).  The support is decided on r^2,
 // so r only enters the kernel's value and gradient, where its rounding is of the float32 terms' own
-// size; continuity's and the correction matrix's float64 parts take one Newton step from it to
-// float64's digits.  The .ftz form skips the subnormal scaling of rsqrtf; the floor keeps its argument
+// size; continuity's and the correction matrix's float64 parts take preciseRoot() from it.  The .ftz form skips the subnormal scaling of rsqrtf; the floor keeps its argument
 // normal, and a pair under it (r < 1e-15 m) is coincident to every kernel.
 constexpr float kLeastDistance2 = 1.0e-30f;
 __device__ __forceinline__ float inverseRoot(float r2)
@@ -187,6 +186,17 @@ __device__ __forceinline__ float inverseRoot(float r2)
     float inverse;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inverse) : "f"(fmaxf(r2, kLeastDistance2)));
     return inverse;
+}
+
+// A distance in float64 from its square, by way of y, the float32 reciprocal root of the square's float32
+// value: with e = 1 - r2 y^2, about 5e-7, r = r2 y (1 - e)^(-1/2) = r2 y (1 + e / 2 + 3 e^2 / 8 + ...), and
+// the next term, 5 e^3 / 16, lies below float64's rounding.  One Newton step scaled by y in float32 left up
+// to 6e-14 and, for its conversions, took longer: the 64-ppd beach's gradients 0.0607 -> 0.0576 ms, the
+// 10-ppd ridge's continuity 2.57 -> 2.52 (a division in place of y: 3.00).
+__device__ __forceinline__ double preciseRoot(double r2, float inverse)
+{
+    const double y = (double)inverse, near = __dmul_rn(r2, y), e = fma(-near, y, 1.0);
+    return fma(__dmul_rn(near, e), fma(0.375, e, 0.5), near);
 }
 
 // a / b to 2 ulp for a normal b up to 2^126: __fdividef without its subnormal scaling (a subnormal

@@ -1,0 +1,62 @@
+"""What a pair's arithmetic keeps: float64's digits where a sum is taken in float64, and every bit of a
+float32 quotient whose terms are small."""
+from decimal import Decimal, getcontext
+
+import numpy as np
+import pytest
+
+from test_gpu_pairs import C0, RHO0, cloud, pairSums
+
+pytestmark = pytest.mark.gpu
+
+getcontext().prec = 60
+
+
+def exactRoot(value):
+    return Decimal(value).sqrt()
+
+
+@pytest.mark.parametrize('threads', [1, 4])
+@pytest.mark.parametrize('dim', [2, 3])
+def test_a_wall_pairs_distance_has_float64s_digits(dim, threads):
+    # A fluid particle between two boundary particles whose terms cancel to about 1e-12 of either: the rate
+    # is what is left, so an error of a term's distance shows in it.  h and every coordinate are exact in
+    # binary, the velocities in 40 bits, and the rest is worked out in 60 digits.  Each term's roundings:
+    # 2 of the root, which (1 - q / 2)^3 magnifies by at most 4.5 at q <= 1.2, and 5 of the products, each
+    # 1.1e-16; two terms, 3e-15 in all.
+    rng = np.random.default_rng(dim)
+    h = 2.0 ** -6
+    places = np.stack(np.meshgrid(*[np.arange(24 if dim == 2 else 8)] * dim, indexing='ij'), -1).reshape(-1, dim)
+    centres = (places + 1) * (8 * h)
+    n = len(centres)
+
+    def offsets():
+        direction = rng.normal(size=(n, dim))
+        direction[:, 0] = np.sign(direction[:, 0]) * (np.abs(direction[:, 0]) + 0.5)     # well along x
+        direction /= np.linalg.norm(direction, axis=1)[:, None]
+        return np.round(direction * (h * rng.uniform(0.3, 1.2, (n, 1))) * 2.0 ** 36) / 2.0 ** 36
+
+    first, second = offsets(), offsets()
+    speed, left, size = np.empty(n), np.empty(n), np.empty(n)
+    for k in range(n):
+        terms = []
+        for d in (first[k], second[k]):
+            r = exactRoot(sum(Decimal(float(a)) ** 2 for a in d))
+            terms.append((1 - r / (2 * Decimal(h))) ** 3 * Decimal(float(d[0])))
+        s = float(-terms[0] / terms[1])
+        speed[k] = np.round(s * 2.0 ** (39 - np.floor(np.log2(abs(s))))) / 2.0 ** (39 - np.floor(np.log2(abs(s))))
+        left[k] = float(terms[0] + Decimal(speed[k]) * terms[1])
+        size[k] = abs(float(terms[0]))
+    x = np.concatenate([centres, centres - first, centres - second])
+    v = np.zeros_like(x)
+    v[n:2 * n, 0] = -1.0            # v_i - v_j along x: 1 and `speed`
+    v[2 * n:, 0] = -speed
+    fluid = np.arange(len(x)) < n
+    from pysurf_b200.sphGpu import PairSums
+    sums = PairSums(dim, h, np.zeros(dim), x.max(axis=0) + 8 * h, kernelType='wendlandC2')
+    sums.setSweepOptions(True, threads)
+    sums.update(x, np.ones(len(x)), fluid)
+    rate = sums.continuityRate(v)[:n]
+    scale = -5.0 * sums.sigmaUnit / h ** dim / h ** 2       # (dW/dr) / r = scale (1 - q / 2)^3
+    assert np.median(np.abs(left) / size) > 1e-13           # there is something left to be found
+    assert np.max(np.abs(rate / scale - left) / size) < 4e-15

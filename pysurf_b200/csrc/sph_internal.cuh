@@ -148,7 +148,8 @@ struct Frame {
     const int *cellStart;   // lower bound of each cell in the sorted order, numCells + 1 entries
     float4 *G0, *G1, *G2;   // velocity gradient rows (2D: G0 = (G00, G01, G10, G11))
     // the slopes' coefficients, r . G r = sum over a <= b of them times r_a r_b: G_aa, and G_ab + G_ba.
-    // 2D: S0 = (G00, G01 + G10, G11, -); 3D: S0 = (00, 01 + 10, 02 + 20, 11), S1 = (12 + 21, 22)
+    // 2D: S0 = (G00, G01 + G10, G11, -); 3D: S0 = (00, 01 + 10, 02 + 20, 11), S1 = (12 + 21, 22);
+    // each times kSlopeScale
     float4 *S0;
     float2 *S1;
     float4 *L0, *L1, *L2;   // correction matrix rows, same packing
@@ -563,6 +564,11 @@ template <> __device__ __forceinline__ void storeMatrix<3>(float4 *R0, float4 *R
     R2[j] = make_float4(M[2][0], M[2][1], M[2][2], 0.0f);
 }
 
+// The slopes' coefficients are kept times 2^24, so that the limiter's products of two slopes stay normal
+// floats down to slopes of 1e-26 m^2 / s (the tail of a wave has some of 1e-19, whose plain product is
+// subnormal or zero); they overflow past 5e11.  A power of two changes no other bit.
+constexpr float kSlopeScale = 16777216.0f;
+
 // The slopes' coefficients of slot j (Frame::S0, S1), in the order (0,0), (0,1), (0,2), (1,1), ...
 template <int D> __device__ __forceinline__ void loadSlopes(const Frame &F, int j, float s[6])
 {
@@ -575,11 +581,12 @@ template <int D> __device__ __forceinline__ void loadSlopes(const Frame &F, int 
 }
 template <int D> __device__ __forceinline__ void storeSlopes(const Frame &F, int j, const float G[3][3])
 {
+    constexpr float s = kSlopeScale;
     if (D == 2) {
-        F.S0[j] = make_float4(G[0][0], G[0][1] + G[1][0], G[1][1], 0.0f);
+        F.S0[j] = make_float4(s * G[0][0], s * (G[0][1] + G[1][0]), s * G[1][1], 0.0f);
     } else {
-        F.S0[j] = make_float4(G[0][0], G[0][1] + G[1][0], G[0][2] + G[2][0], G[1][1]);
-        F.S1[j] = make_float2(G[1][2] + G[2][1], G[2][2]);
+        F.S0[j] = make_float4(s * G[0][0], s * (G[0][1] + G[1][0]), s * (G[0][2] + G[2][0]), s * G[1][1]);
+        F.S1[j] = make_float2(s * (G[1][2] + G[2][1]), s * G[2][2]);
     }
 }
 

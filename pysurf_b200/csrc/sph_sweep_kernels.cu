@@ -16,6 +16,7 @@
 //
 // Each sweep is templated on the dimension D, the kernel K (0 cubic spline, 1 Wendland C2) and
 // the threads per particle T.  Sums are float32 in a fixed order, no atomics on them.
+#include <cfloat>
 #include <climits>
 #include <math.h>
 
@@ -754,6 +755,10 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, floa
 // Sweep C: accelerations, fluid maxima, time step
 // ------------------------------------------------------------------------------------------
 
+// What the viscosity is multiplied by until it joins the pressure, so that quickDivide, which takes and
+// leaves no subnormal, loses none.
+constexpr float kViscosityScale = 4294967296.0f;
+
 // BUDGET: the sum split for the energy budget too, into the pressure and the viscosity of fluid
 // and of boundary neighbours (src/pysurf/sphGpu.py:400-414).  COMP: the sum compensated (Dot2),
 // its running error in comp.
@@ -765,7 +770,7 @@ struct MomentumVisit {
     static constexpr bool kSkipCoincident = true;
     const Params &P; const Frame &F;
     Smoothing<K, D, FINE> S;
-    float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0
+    float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0 kViscosityScale
     float alphaI;                               // closure: this particle's eddy alpha
     float slopeI[6];                            // r . G_i r's coefficients (Frame::S0, S1)
     float2 total[D];                            // minus the sum, over the lane's even and odd neighbours
@@ -822,13 +827,14 @@ struct MomentumVisit {
                         slopeI2 = fma2(both(slopeI[c]), dd, slopeI2);
                         slopeJ = make_float2(__fmaf_rn(s0[c], dd.x, slopeJ.x), __fmaf_rn(s1[c], dd.y, slopeJ.y));
                     }
-                // 4 R / (1 + R)^2 at R = slopeI / slopeJ, as 4 slopeI slopeJ / (slopeI + slopeJ)^2
+                // 4 R / (1 + R)^2 at R = slopeI / slopeJ, as 4 slopeI slopeJ / (slopeI + slopeJ)^2, which is
+                // never less than what stands above it; 0 where that has no normal float
                 const float2 sum = add2(slopeI2, slopeJ), product = mul2(slopeI2, slopeJ);
                 const float2 four = mul2(both(4.0f), product), square = mul2(sum, sum);
                 // the fast division takes 8% off the momentum sweep; its range limit (a denominator
-                // past 2^126) lies far beyond any pair's slopes
-                float2 limiter = make_float2(product.x > 0.0f ? fminf(1.0f, quickDivide(four.x, square.x)) : 0.0f,
-                                             product.y > 0.0f ? fminf(1.0f, quickDivide(four.y, square.y)) : 0.0f);
+                // past 2^126) lies far beyond any pair's slopes, and the scale keeps both sides normal
+                float2 limiter = make_float2(four.x >= FLT_MIN ? fminf(1.0f, quickDivide(four.x, square.x)) : 0.0f,
+                                             four.y >= FLT_MIN ? fminf(1.0f, quickDivide(four.y, square.y)) : 0.0f);
                 if (q.x < kCloseDistance || q.y < kCloseDistance) {
                     const float fade0 = (q.x - kCloseDistance) * (1.0f / kFoldWidth);
                     const float fade1 = (q.y - kCloseDistance) * (1.0f / kFoldWidth);
@@ -836,26 +842,32 @@ struct MomentumVisit {
                     if (q.y < kCloseDistance) limiter.y = __fmul_rn(limiter.y, expf(-__fmul_rn(fade1, fade1)));
                 }
                 // (v_ij - (phi / 2) (G_i + G_j) r) . r = v_ij . r - (phi / 2) (r . G_i r + r . G_j r)
-                const float2 limited = fma2(mul2(both(-0.5f), limiter), sum, plain);
+                const float2 limited = fma2(mul2(both(-0.5f / kSlopeScale), limiter), sum, plain);
                 if (limit0) approach.x = limited.x;
                 if (limit1) approach.y = limited.y;
             }
         }
-        // -alpha c0 h (v_ij . r_ij) / ((r^2 + 0.01 h^2) (rho_i + rho_j) / 2) where the pair approaches; the
-        // denominator is a positive normal float for any physical pair
+        // -alpha c0 h (v_ij . r_ij) / ((r^2 + 0.01 h^2) (rho_i + rho_j) / 2) where the pair approaches, times
+        // kViscosityScale; the denominator is a positive normal float for any physical pair
         const float2 closing = make_float2(fminf(approach.x, 0.0f), fminf(approach.y, 0.0f));
         const float2 above = mul2(mul2(both(viscosityScale), N.h), closing);
         const float2 mean = mul2(both(0.5f), taken.density);
         const float2 below = mul2(fma2(N.r, N.r, N.k.soft), mean);
         float2 viscosity = make_float2(quickDivide(above.x, below.x), quickDivide(above.y, below.y));
         if (KIND == kWallPair) viscosity = mul2(viscosity, both(P.boundaryFactor));
+        const float2 pressure = taken.pressure;
+        float2 stress;
         if (KIND == kFluidPair && CLOSURE && P.closure) {
+            viscosity = mul2(viscosity, both(1.0f / kViscosityScale));
             if (N.live[0])
                 viscosity.x = __fadd_rn(viscosity.x, closureTerm(N.j[0], N.h.x, N.r.x, plain.x, taken.rho[0]));
             if (N.live[1])
                 viscosity.y = __fadd_rn(viscosity.y, closureTerm(N.j[1], N.h.y, N.r.y, plain.y, taken.rho[1]));
+            stress = add2(pressure, viscosity);
+        } else {
+            stress = fma2(viscosity, both(1.0f / kViscosityScale), pressure);
+            if (BUDGET) viscosity = mul2(viscosity, both(1.0f / kViscosityScale));
         }
-        const float2 pressure = taken.pressure, stress = add2(pressure, viscosity);
         const float m0 = taken.mass[0], m1 = taken.mass[1];
         const float2 f = mul2(make_float2(N.live[0] ? __fmul_rn(stress.x, m0) : 0.0f,
                                           N.live[1] ? __fmul_rn(stress.y, m1) : 0.0f), grad);
@@ -914,7 +926,7 @@ momentumKernel(Params P, Frame F, Control *ctl, int maxima)
             velocityOf<D>(F, i, visit.vi);
             visit.rhoI = densityOf<D>(F, i);
             visit.own = pressureRatioOf<D>(F, i);
-            visit.viscosityScale = -P.alpha * P.c0;
+            visit.viscosityScale = -P.alpha * P.c0 * kViscosityScale;
             visit.alphaI = CLOSURE && P.closure ? F.eddy[i].x : 0.0f;
             if (P.limited) loadSlopes<D>(F, i, visit.slopeI);
             for (int a = 0; a < D; ++a) visit.total[a] = both(0.0f);
@@ -966,7 +978,8 @@ __global__ void closureKernel(Params P, Frame F, const Control *ctl)
     float sum = 0.0f;
     for (int a = 0; a < D; ++a)
         for (int b = 0; b < D; ++b) {
-            const float e = a == b ? slopes[packed<D>(a, a)] : 0.5f * slopes[packed<D>(min(a, b), max(a, b))];
+            const float scaled = a == b ? slopes[packed<D>(a, a)] : 0.5f * slopes[packed<D>(min(a, b), max(a, b))];
+            const float e = scaled * (1.0f / kSlopeScale);
             sum += e * e;
         }
     const float scale = hs * sqrtf(2.0f * sum) / P.closureC0;
@@ -1150,7 +1163,7 @@ struct ContinuityVisit {
                 const float2 slope = mul2(both(P.hydrostaticSlope), N.d[D - 1]);
                 const float2 back = mul2(mul2(slope, e), sum);
                 difference = add2(add2(fma2(both(-P.hydrostaticSlope), N.d[D - 1], leading), remainder),
-                                  make_float2(quickDivide(back.x, fifth.x), quickDivide(back.y, fifth.y)));
+                                  make_float2(__fdividef(back.x, fifth.x), __fdividef(back.y, fifth.y)));
             } else {
                 difference = add2(leading, remainder);
             }

@@ -199,8 +199,10 @@ __device__ __forceinline__ double preciseRoot(double r2, float inverse)
     return fma(__dmul_rn(near, e), fma(0.375, e, 0.5), near);
 }
 
-// a / b to 2 ulp for a normal b up to 2^126: __fdividef without its subnormal scaling (a subnormal
-// counts as zero).
+// a / b to 2 ulp for a normal b up to 2^126: __fdividef without its subnormal scaling.  A subnormal, taken or
+// given, counts as zero, so it stands only where none can matter: the limiter's and the viscosity's quotients
+// are of scaled values (kSlopeScale, kViscosityScale), and the diffusion's r^2 / (r^2 + 0.01 h^2) has r above
+// 1e-12.  With __fdividef at these the ridges' steps take 0.5% longer.
 __device__ __forceinline__ float quickDivide(float a, float b)
 {
     float q;

@@ -60,3 +60,35 @@ def test_a_wall_pairs_distance_has_float64s_digits(dim, threads):
     scale = -5.0 * sums.sigmaUnit / h ** dim / h ** 2       # (dW/dr) / r = scale (1 - q / 2)^3
     assert np.median(np.abs(left) / size) > 1e-13           # there is something left to be found
     assert np.max(np.abs(rate / scale - left) / size) < 4e-15
+
+
+@pytest.mark.parametrize('kernel', ['wendlandC2', 'cubicSpline'])
+@pytest.mark.parametrize('dim', [2, 3])
+@pytest.mark.parametrize('power', [40, 60, 70])
+def test_the_limited_viscosity_scales_with_the_velocities(dim, power, kernel):
+    # Without pressure and gravity the limited viscosity is of degree one in the velocities, so velocities
+    # scaled by a power of two scale every acceleration by it, bit for bit, down to slopes of 1e-22 whose
+    # squares have no float32: the tail of a wave is such a flow.
+    x, v, rho, m, fluid, h = cloud(dim, 900, 31, ratio=2.0)
+    rho = np.full(len(x), RHO0)
+    s = pairSums(dim, h, True, kernel=kernel)
+    s.update(x, m, fluid)
+    zero = np.zeros(len(x))
+    whole = s.pairAccelerations(v, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
+    small = s.pairAccelerations(v * 2.0 ** -power, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
+    assert np.abs(whole).max() > 0.0 and np.array_equal(small, whole * 2.0 ** -power)
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+def test_the_smallest_viscosity_is_not_lost(dim):
+    # The same without the limiter at 2^-118, where the viscosity's numerator, alpha c0 h (v_ij . r_ij), has
+    # no normal float32.  A product v d is off by half the least float32, 2^-150, three of them against the
+    # largest v_ij . r_ij, some 2^-121: 1e-8 of it, and the acceleration's sums keep 1e-6 of the largest.
+    x, v, rho, m, fluid, h = cloud(dim, 900, 37, ratio=2.0)
+    rho = np.full(len(x), RHO0)
+    s = pairSums(dim, h, True, limited=False)
+    s.update(x, m, fluid)
+    zero = np.zeros(len(x))
+    whole = s.pairAccelerations(v, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
+    small = s.pairAccelerations(v * 2.0 ** -118, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
+    assert np.abs(small * 2.0 ** 118 - whole).max() < 1e-6 * np.abs(whole).max()

@@ -69,6 +69,7 @@ struct LaunchArgs {
     float floorDet;
     const float *densities; // Xsph: the densities it divides by; null for the frame's
     int threads;            // threads per particle in the sweeps: 1, 2, 4 or 8
+    int tabled;             // the table's rows were long enough for every particle when it was sized
     int *maxCount;          // List: the largest neighbour count goes here (atomic max), when given
 };
 

@@ -41,6 +41,11 @@ constexpr int preciseMinBlocks() { return D == 2 ? 5 : 4; }
 template <int D>
 constexpr int gradientMinBlocks() { return D == 2 ? 5 : 3; }
 
+// the filter and the wall pressure, of few sums: 7 in 2D, 6 in 3D (0.25 ms for the wall pressure on the 10-ppd
+// ridge against 0.28 at 5)
+template <int D>
+constexpr int lightMinBlocks() { return D == 2 ? 7 : 6; }
+
 // ------------------------------------------------------------------------------------------
 // The neighbour table
 // ------------------------------------------------------------------------------------------
@@ -48,24 +53,6 @@ constexpr int gradientMinBlocks() { return D == 2 ? 5 : 3; }
 #ifndef SPH_LIST_TRIM
 #define SPH_LIST_TRIM 1
 #endif
-
-// Whether a slot is fluid, and whether a run of slots holds a boundary slot, from the slots' bits (32 a
-// word, so a run of a stencil row is a few words).
-__device__ __forceinline__ bool isFluid(const Frame &F, int j)
-{
-    return !(fetch(&F.wallBits[j >> 5]) >> (j & 31) & 1);
-}
-__device__ __forceinline__ bool runHasWalls(const Frame &F, int first, int end)
-{
-    unsigned any = 0;
-    for (int w = first >> 5; w <= (end - 1) >> 5; ++w) {
-        unsigned bits = fetch(&F.wallBits[w]);
-        if (w == first >> 5) bits &= 0xFFFFFFFFu << (first & 31);
-        if (w == (end - 1) >> 5) bits &= 0xFFFFFFFFu >> (31 - ((end - 1) & 31));
-        any |= bits;
-    }
-    return any != 0;
-}
 
 // Each slot's neighbours in the walk's order (sumPairs', with its tests), from a group of
 // L lanes: lane t tests candidates t, t + L, ... of each run of the stencil, and the group's ballot
@@ -144,7 +131,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(
                     const float4 A = fetch(&F.pa[j]);
                     float pj[3];
                     pointIn<D>(A, pj);
-                    if (WALLED) fluidJ = isFluid(F, j);
+                    if (WALLED) fluidJ = isFluid(F.wallBits, j);
                     const float coarse = !WALLED || fluidJ || !fluidOnly ? coarseDistance2<D>(at, pj) : searchLimit;
                     if (PRECISE && !image && level == 0 && coarse < sure) {
                         accepted = true;
@@ -198,7 +185,7 @@ __global__ void __launch_bounds__(kBlock, D == 2 && !MIXED ? 11 : 1) listKernel(
                     const int row = box.first + (zz * box.ny + yy) * box.nx;
                     runFirst = fetch(&F.cellStart[row + xa]);
                     runEnd = fetch(&F.cellStart[row + xb + 1]);
-                    runWalls = runHasWalls(F, runFirst, runEnd);
+                    runWalls = runHas(F.wallBits, runFirst, runEnd, true);
                 }
             }
             const unsigned walledRows = __ballot_sync(G.mask, runWalls) >> shift;
@@ -472,7 +459,6 @@ __global__ void __launch_bounds__(kBlock) cellListKernel(Params P, Frame F, cons
 
 template <int D, int K, bool FINE>
 struct ShepardVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = true, kKinetic = D == 2, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
     Smoothing<K, D, FINE> S;
@@ -486,7 +472,7 @@ struct ShepardVisit {
 };
 
 template <int D, int K, int T, bool FINE>
-__global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shepardKernel(Params P, Frame F, const Control *ctl)
+__global__ void __launch_bounds__(kBlock, lightMinBlocks<D>()) shepardKernel(Params P, Frame F, const Control *ctl)
 {
     awaitPrevious();
     stampStages(const_cast<Control *>(ctl), P.stages);
@@ -535,7 +521,6 @@ __global__ void applyShepardKernel(Params P, Frame F, const Control *ctl)
 
 template <int D, int K, bool FINE>
 struct WallVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = true, kKinetic = false, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
     const Params &P; const Frame &F;
@@ -554,7 +539,7 @@ struct WallVisit {
 // Boundary rows only write their own entries and only fluid entries are read, so the frame is
 // updated in place.  writeDensity: the master float64 density takes Tait^-1(p_w) too.
 template <int D, int K, int T, bool FINE>
-__global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>())
+__global__ void __launch_bounds__(kBlock, lightMinBlocks<D>())
 wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
 {
     awaitPrevious();
@@ -595,9 +580,9 @@ wallPressureKernel(Params P, Frame F, const Control *ctl, int writeDensity)
 template <int D>
 __device__ __forceinline__ constexpr int packed(int a, int b) { return a * D - a * (a - 1) / 2 + (b - a); }
 
-template <int D, int K, bool FINE, bool RHO>
+template <int D, int K, bool FINE, bool RHO, bool TABLED>
 struct GradientVisit {
-    static constexpr bool kCopied = D == 3 && !FINE;
+    static constexpr bool kAlone = TABLED;
     static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
@@ -671,7 +656,8 @@ __device__ __forceinline__ float groupSum(const float2 &value, unsigned mask)
     return groupSum<T>(__fadd_rn(value.x, value.y), mask);
 }
 
-template <int D, int K, int T, bool FINE, bool RHO>
+// TABLED: few rows walk (LaunchArgs::tabled), in 3D with one smoothing length; sumPairs() says why.
+template <int D, int K, int T, bool FINE, bool RHO, bool TABLED>
 __global__ void __launch_bounds__(kBlock, gradientMinBlocks<D>())
 gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, float floorDet)
 {
@@ -691,7 +677,7 @@ gradientKernel(Params P, Frame F, const Control *ctl, int wantG, int wantL, floa
         if (RHO) F.gradRho[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
-    GradientVisit<D, K, FINE, RHO> visit{Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || RHO};
+    GradientVisit<D, K, FINE, RHO, TABLED> visit{Smoothing<K, D, FINE>(P, hs), wantG != 0, wantL != 0 || RHO};
     velocityOf<D>(F, i, visit.vi);
     visit.devI = deviationOf<D>(F, i);
     for (int a = 0; a < D; ++a) {
@@ -764,7 +750,6 @@ constexpr float kViscosityScale = 4294967296.0f;
 // its running error in comp.
 template <int D, int K, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 struct MomentumVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = true, kKinetic = true, kAux = true, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
@@ -1045,7 +1030,6 @@ __global__ void kickKernel(Params P, Frame F, Control *ctl)
 // Fluid pairs, whose velocity differences are small, keep float32 arithmetic.
 template <int D, int K, bool BUDGET, bool FINE, bool COMP, bool CLOSURE>
 struct ContinuityVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = true, kMass = true;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
@@ -1308,7 +1292,6 @@ continuityKernel(Params P, Frame F, Control *ctl, Enforcement E, int mode)
 
 template <int D, int K, bool FINE>
 struct XsphVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = true, kKinetic = true, kAux = true, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
     const float *densities;
@@ -1380,7 +1363,6 @@ __global__ void frameDensityKernel(Params P, Frame F, const Control *ctl)
 // grad C0, div r = -sum V_j r_ij . grad W_ij, grad rho from the deviations.
 template <int D, int K>
 struct ShiftFieldsVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kPaired = true;
     static constexpr bool kSkipCoincident = true;
@@ -1460,7 +1442,6 @@ __global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftFieldsKernel
 // kernel-weighted sum of their outward normals -grad C0 / |grad C0|.
 template <int D, int K>
 struct SurfaceVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = false, kKinetic = false, kAux = false, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = false;
     const Params &P; const Frame &F;
@@ -1485,7 +1466,6 @@ struct SurfaceVisit {
 // The velocity at the shifted position: sum_j V_j (v_j - v_i) (grad W_ij . shift) over fluid pairs.
 template <int D, int K>
 struct ShiftedVelocityVisit {
-    static constexpr bool kCopied = false;
     static constexpr bool kBody = false, kKinetic = true, kAux = false, kLow = false, kMass = false;
     static constexpr bool kSkipCoincident = true;
     Smoothing<K, D, false> S;
@@ -1506,7 +1486,7 @@ struct ShiftedVelocityVisit {
 // and the velocity change at the new position.  size: CFL Ma (2h)^2 with CFL = c0 dt / h, or
 // 2 h |v_i| dt (local).
 template <int D, int K, int T, bool FINE>
-__global__ void __launch_bounds__(kBlock, sweepMinBlocks<D>()) shiftKernel(Params P, Frame F, const Control *ctl)
+__global__ void __launch_bounds__(kBlock, 5) shiftKernel(Params P, Frame F, const Control *ctl)
 {
     awaitPrevious();
     if (ctl && !ctl->active) return;
@@ -1665,6 +1645,12 @@ static void launchMomentum(const LaunchArgs &A, int grid)
     else if (P.closure) launchNext(momentumKernel<D, K, T, false, FINE, false, true>, grid, kBlock, st, P, F, A.ctl, A.maxima);
     else launchNext(momentumKernel<D, K, T, false, FINE, false, false>, grid, kBlock, st, P, F, A.ctl, A.maxima);
 }
+template <int D, int K, int T, bool FINE, bool TABLED>
+static void launchGradients(const LaunchArgs &A, int grid)
+{
+    auto kernel = A.wantRho ? gradientKernel<D, K, T, FINE, true, TABLED> : gradientKernel<D, K, T, FINE, false, TABLED>;
+    launchNext(kernel, grid, kBlock, A.stream, A.P, A.F, A.ctl, A.wantG, A.wantL, A.floorDet);
+}
 template <int D, int K, int T, bool FINE>
 static void launchContinuity(const LaunchArgs &A, int grid)
 {
@@ -1690,8 +1676,8 @@ static void launchT(const LaunchArgs &A, Stage stage)
     case Stage::ShepardApply: launchNext(applyShepardKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;
     case Stage::Wall: launchNext(wallPressureKernel<D, K, T, FINE>, grid, kBlock, st, P, F, A.ctl, A.flag); break;
     case Stage::Gradients:
-        if (A.wantRho) launchNext(gradientKernel<D, K, T, FINE, true>, grid, kBlock, st, P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
-        else launchNext(gradientKernel<D, K, T, FINE, false>, grid, kBlock, st, P, F, A.ctl, A.wantG, A.wantL, A.floorDet);
+        if (D == 3 && !FINE && A.tabled) launchGradients<D, K, T, FINE, D == 3 && !FINE>(A, grid);
+        else launchGradients<D, K, T, FINE, false>(A, grid);
         break;
     case Stage::Momentum: launchMomentum<D, K, T, FINE>(A, grid); break;
     case Stage::Kick: launchNext(kickKernel<D>, pointwise, kBlock, st, P, F, A.ctl); break;

@@ -252,6 +252,25 @@ struct Origin {
     double shift64;
 };
 
+// Whether a slot is fluid, and whether a run of slots holds any of a kind, from the slots' bits (32 a word,
+// so a run of a stencil row is a few words).
+__device__ __forceinline__ bool isFluid(const unsigned *wallBits, int j)
+{
+    return !(fetch(&wallBits[j >> 5]) >> (j & 31) & 1);
+}
+__device__ __forceinline__ bool runHas(const unsigned *wallBits, int first, int end, bool walls)
+{
+    const unsigned flip = walls ? 0u : 0xFFFFFFFFu;
+    unsigned any = 0;
+    for (int w = first >> 5; w <= (end - 1) >> 5; ++w) {
+        unsigned bits = fetch(&wallBits[w]) ^ flip;
+        if (w == first >> 5) bits &= 0xFFFFFFFFu << (first & 31);
+        if (w == (end - 1) >> 5) bits &= 0xFFFFFFFFu >> (31 - ((end - 1) & 31));
+        any |= bits;
+    }
+    return any != 0;
+}
+
 // The candidates of a walk over the cells of slot i's searches, one at a time.  Search s is of grid
 // level s >> 1 (coarse, then fine when the particles carry two levels of smoothing length) from origin
 // s & 1 (the particle, then its periodic image when it lies near the seam).
@@ -293,31 +312,34 @@ struct Candidates {
         return true;
     }
 
+    // The next row's run, of slots j + 1 .. end - 1; false when there are none left.
+    __device__ __forceinline__ bool nextRow(const Params &P, const Origin &O, const float pi[3], const float li[3])
+    {
+        if (yy < y1) {
+            ++yy;
+        } else if (zz < z1) {
+            ++zz;
+            yy = y0;
+        } else {
+            constexpr int searches = FINE ? 4 : 2;
+            int s = search + 1;
+            while (s < searches && !startSearch(P, O, pi, li, s)) ++s;
+            return s < searches;
+        }
+        startRow();
+        return true;
+    }
+
     // The next candidate into (jOut, imageOut, levelOut); false when there are none left.
     __device__ __forceinline__ bool next(const Params &P, const Origin &O, const float pi[3], const float li[3],
                                          int &jOut, int &imageOut, int &levelOut)
     {
-        while (true) {
-            if (++j < end) {
-                jOut = j;
-                imageOut = search & 1;
-                levelOut = FINE ? search >> 1 : 0;
-                return true;
-            }
-            if (yy < y1) {
-                ++yy;
-            } else if (zz < z1) {
-                ++zz;
-                yy = y0;
-            } else {
-                constexpr int searches = FINE ? 4 : 2;
-                int s = search + 1;
-                while (s < searches && !startSearch(P, O, pi, li, s)) ++s;
-                if (s >= searches) return false;
-                continue;
-            }
-            startRow();
-        }
+        while (++j >= end)
+            if (!nextRow(P, O, pi, li)) return false;
+        jOut = j;
+        imageOut = search & 1;
+        levelOut = FINE ? search >> 1 : 0;
+        return true;
     }
 };
 
@@ -333,6 +355,16 @@ struct Paired {
 template <class V>
 struct Paired<V, std::void_t<decltype(V::kPaired)>> {
     static constexpr bool value = V::kPaired;
+};
+
+// Whether a visitor's pipeline copies the rows and its walk is each lane's own (kAlone; sumPairs() says when).
+template <class V, class = void>
+struct Alone {
+    static constexpr bool value = false;
+};
+template <class V>
+struct Alone<V, std::void_t<decltype(V::kAlone)>> {
+    static constexpr bool value = V::kAlone;
 };
 
 // A row's load, which stays where it is written: the compiler would otherwise move it down to its first
@@ -491,7 +523,7 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
         };
         auto entry = [&](const int *at) {
             int value;
-                        asm volatile("ld.global.L1::no_allocate.b32 %0, [%1];" : "=r"(value) : "l"(at));
+            asm volatile("ld.global.L1::no_allocate.b32 %0, [%1];" : "=r"(value) : "l"(at));
             return value;
         };
         int left = count > O.t ? (count - O.t - 1) / T + 1 : 0;
@@ -517,11 +549,11 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
             while (true) {
                 const int j0 = ring[0], j1 = ring[1];
                 Neighbours N;
-                // the rows' values that the sums need come first, or (kCopied) copies of the rows, so
-                // that the next rows load into the same registers meanwhile
+                // the rows' values that the sums need come first, or (kAlone) copies of the rows, so that the
+                // next rows load into the same registers meanwhile
                 BothRows C;
                 Taken<D, FINE, KIND, Visitor> taken;
-                if constexpr (Visitor::kCopied) C = BothRows{R0, R1};
+                if constexpr (Alone<Visitor>::value) C = BothRows{R0, R1};
                 else taken = takeBoth<D, 1, FINE, KIND>(P, O, j0, j1, left > 1, R0, R1, visit, N);
                 ring[0] = ring[2];
                 ring[1] = left == 3 ? ring[2] : ring[3];
@@ -535,7 +567,7 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
                 }
                 if (left > 4) ring[2] = e2;
                 if (left > 5) ring[3] = e3;
-                if constexpr (Visitor::kCopied)
+                if constexpr (Alone<Visitor>::value)
                     taken = takeBoth<D, 1, FINE, KIND>(P, O, j0, j1, left > 1, C.R0, C.R1, visit, N);
                 finishBoth<KIND>(N, taken, visit);
                 if (left <= 2) break;
@@ -556,40 +588,75 @@ __device__ __forceinline__ void sumPairs(const Params &P, const Frame &F, const 
         return;
     }
 
-    // the walk
+    // The walk: the group's lanes test T candidates of a row's run at a time, and a ballot hands the
+    // accepted ones to the lanes whose turn it is.  A row's run of one kind alone, as most are, is passed
+    // over for the other.  Without a table the 64-ppd beach steps in 1.13 ms so (2.28 with every lane
+    // testing all candidates of both kinds), the 8-ppd ridge in 27.0 (51.3).
+    //
+    // kAlone keeps that form, which has no ballot, for a sweep whose rows nearly all come from the table:
+    // beside a walk with ballots the 3D gradients take 2.00 ms on the 10-ppd ridge (2.57 with copied rows),
+    // beside this one 1.82.
+    constexpr bool kAlone = Alone<Visitor>::value;
+    constexpr int W = kAlone ? 1 : T;       // candidates a round
     const float limit = kCandidateMargin * O.reach * O.reach;
     // the coarse test's bound for fine candidates: no fine neighbour lies past hI + fineMax
     const float fineReach = O.hI + P.fineMax;
     const float fineLimit = kCandidateMargin * fineReach * fineReach;
     const Origin origin{F.cell[O.i], O.hI, O.seam, O.shift64};
+    const int lane = (threadIdx.x & 31) & ~(W - 1);     // the group's first lane
+    const unsigned group = W >= 32 ? 0xFFFFFFFFu : ((1u << W) - 1u) << lane;
     Candidates<D, FINE> C;
     C.cellStart = F.cellStart;
     C.startSearch(P, origin, O.pi, O.li, 0);
-    int counted = 0, j = 0, image = 0, level = 0, held = 0;
-    bool holds = false, ended = false;
+    int base = C.end, counted = 0, held = 0;
+    bool holds = false, ended = false, asks = false, first = true;
     while (true) {
-        ended = !C.next(P, origin, O.pi, O.li, j, image, level);
+        while (base >= C.end && !ended) {
+            if (!first) ended = !C.nextRow(P, origin, O.pi, O.li);
+            first = false;
+            base = C.j + 1;
+            if (ended || base >= C.end) continue;
+            asks = runHas(F.wallBits, base, C.end, fluid);      // the other kind
+            if (asks && !runHas(F.wallBits, base, C.end, !fluid)) base = C.end;
+        }
+        int entry = held;
         if (!ended) {
+            const int image = C.search & 1, level = FINE ? C.search >> 1 : 0, j = base + O.t % W;
             const float offset = image ? (float)O.shift64 : 0.0f;   // the search's origin: particle or image
-            const float4 A = fetch(&F.pa[j]);
-            float pj[3], lj[3], d[3];
-            pointIn<D>(A, pj);
-            if (coarseDistance2<D>(O.pi, pj, offset) >= (FINE && level ? fineLimit : limit) || j == O.i) continue;
-            const float4 B = fetch(&F.pb[j]);
-            const float hs = signedLengthIn<D>(A, B);
-            if ((hs > 0.0f) != fluid) continue;     // the other kind
-            remainderIn<D>(A, B, lj);
-            const float r2 = separation2<D>(P, O.pi, O.li, pj, lj, offset, image, O.shift64, d);
-            if (r2 >= support2(FINE ? 0.5f * (O.hI + fabsf(hs)) : P.hMax)) continue;
-            if (T > 1 && counted++ % T != O.t) continue;
+            bool accepted = false;
+            if (j < C.end && j != O.i && !(asks && isFluid(F.wallBits, j) != fluid)) {
+                const float4 A = fetch(&F.pa[j]);
+                float pj[3], lj[3], d[3];
+                pointIn<D>(A, pj);
+                if (coarseDistance2<D>(O.pi, pj, offset) < (FINE && level ? fineLimit : limit)) {
+                    const float4 B = D == 3 || FINE ? fetch(&F.pb[j]) : A;
+                    remainderIn<D>(A, B, lj);
+                    const float r2 = separation2<D>(P, O.pi, O.li, pj, lj, offset, image, O.shift64, d);
+                    accepted = r2 < support2(FINE ? 0.5f * (O.hI + fabsf(signedLengthIn<D>(A, B))) : P.hMax);
+                }
+            }
+            int mine = j;
+            if constexpr (kAlone) {
+                accepted = accepted && (T == 1 || counted++ % T == O.t);
+            } else if constexpr (T > 1) {
+                // the accepted candidate whose count is this lane's turn, if there is one among these
+                unsigned bits = (__ballot_sync(group, accepted) & group) >> lane;
+                const int turn = (O.t - counted) & (T - 1);
+                counted += __popc(bits);
+                for (int q = 0; q < turn; ++q) bits &= bits - 1u;
+                accepted = bits != 0;
+                mine = base + __ffs(bits) - 1;
+            }
+            base += W;
+            if (!accepted) continue;
+            entry = image ? (mine | (int)0x80000000) : mine;
+            if (!holds) {
+                held = entry;
+                holds = true;
+                continue;
+            }
         } else if (!holds) {
             return;
-        }
-        const int entry = ended ? held : (image ? (j | (int)0x80000000) : j);
-        if (!ended && !holds) {
-            held = entry;
-            holds = true;
-            continue;
         }
         NeighbourRows R0, R1;
         loadRows<D, FINE, Visitor>(F, held & 0x7FFFFFFF, R0);

@@ -169,6 +169,7 @@ struct SphSystem {
     size_t surfaceBytes = 0;
     size_t nbrEntries = 0;
     int listCap = 0;
+    bool listCapped = false;    // memory keeps the rows shorter than the largest count
     bool listTogether = false;  // the rows' order as built (Params::together)
     bool graphTogether = false; // the rows' order the captured steps build
     int tableMode = 1;          // 0 never build the table, 1 build it when it fits the budget
@@ -546,6 +547,7 @@ struct SphSystem {
         A.E = enforcement;
         A.floorDet = (float)pow(0.25, dim);
         A.threads = threads;
+        A.tabled = A.P.listCap > 0 && !listCapped;
         return A;
     }
 
@@ -593,6 +595,7 @@ struct SphSystem {
         if (!dMaxCount) TRY(deviceAlloc(&dMaxCount, 1));
         CUDA_TRY(cudaMemsetAsync(dMaxCount, 0, sizeof(int), stream));
         const int keep = listCap;
+        const bool keepCapped = listCapped;
         listCap = 0;    // count only
         listTogether = classic();
         LaunchArgs A = args(nullptr);
@@ -602,6 +605,7 @@ struct SphSystem {
         CUDA_TRY(cudaMemcpyAsync(&most, dMaxCount, sizeof(int), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
         int cap = ((most + most / 4 + 8) + 7) & ~7;
+        listCapped = false;
         size_t entries = (size_t)cap * (size_t)capacity;
         if (entries > nbrEntries) {
             cudaFree(nbr);
@@ -612,6 +616,7 @@ struct SphSystem {
             const size_t room = freeBytes / 4 * 3 / sizeof(int) / (size_t)std::max(capacity, 1);
             const bool capped = (size_t)cap > room;
             if (capped) cap = (int)(room & ~(size_t)7);
+            listCapped = cap < most;
             entries = (size_t)cap * (size_t)capacity;
             if ((capped && cap < kMinTableRow) || deviceAlloc(&nbr, entries) != SPH_OK) {
                 nbr = nullptr;
@@ -622,7 +627,7 @@ struct SphSystem {
             }
         }
         listCap = cap;
-        if (listCap != keep) graphDirty = true;
+        if (listCap != keep || listCapped != keepCapped) graphDirty = true;
         if (listCap > 0) {
             A = args(nullptr);
             launchStage(A, Stage::List);

@@ -5,8 +5,7 @@
 // pairs of neighbours of sph_sweep_kernels.cu.  Their Shepard filter rounds the fluid's densities to
 // float32 every few steps, so a rounding of one sum, which elsewhere stays below 1e-9 of a density, shows
 // as a step of 6e-8 in it: the order of the sums and their roundings are part of the scheme's results.
-// Supports are short here (h = 1.3 dx: some 20 neighbours in 2D), so a lane's five or so neighbours
-// leave a pipeline over pairs little to overlap.
+// The default scheme's supports are short (h = 1.3 dx: some 20 neighbours in 2D, five or so a lane).
 //
 //   M  momentum     src/pysurf/sphSolver.py:1122-1149, 1192-1230; src/pysurf/sphGpu.py:303-414
 //   D  continuity   src/pysurf/sphSolver.py:623-654; src/pysurf/sphGpu.py:430-545, 1111-1140
@@ -47,10 +46,28 @@ __device__ __forceinline__ float gradient(float q, const KernelAt &k)
     return __fdividef(-0.75f * k.gradC * rest * rest, q);
 }
 
+// A neighbour's rows as far as the visitor reads them: kKinetic, kAux (3D) and kLow the rows, kMass the mass
+// alone (3D).  `early` keeps the loads where they stand.
+template <int D, bool early, class Visitor>
+__device__ __forceinline__ void loadRows(const Frame &F, int j, const float4 &A, NeighbourRows &R)
+{
+    auto row = [](const float4 *at) { return early ? loadEarly(at) : fetch(at); };
+    R.A = A;
+    R.B = row(&F.pb[j]);
+    if (Visitor::kKinetic) R.K = row(&F.kin[j]);
+    if (D == 3 && Visitor::kAux) R.X = row(&F.aux[j]);
+    if (D == 3 && Visitor::kMass) R.X.z = fetch(&F.aux[j].z);
+    if (Visitor::kLow) R.L = row(&F.low[j]);
+}
+
 // Visits slot i's neighbours in the walk's order: of those counted (a boundary row's are its fluid
 // neighbours, unless `whole`), lane t of T takes those whose count k has k / 4 = t mod T, from the table's
 // row (all of them from its front; P.together) when it holds them, else from the cells.  The visitor gets
 // (j, d, r, whether j is fluid, whether the pair lies across the seam, j's rows) when accept(fluidJ).
+//
+// From the table, a lane's next neighbour's rows load while one is summed, and its next chunk of entries a
+// chunk ahead; the visits keep their order, and so the bits.  The 12-ppd ridge's momentum takes 3.2 ms so and
+// 4.2 without, its continuity and XSPH 7.9 and 9.2; the 64-ppd beach's 0.065 and 0.074, 0.123 and 0.143.
 template <int D, int T, class Visitor>
 __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F, int i, int t, bool whole, Visitor &visit)
 {
@@ -59,65 +76,91 @@ __device__ __forceinline__ void forEachNeighbour(const Params &P, const Frame &F
     pointOf<D>(F, i, pi);
     remainderOf<D>(F, i, li);
     const float reach = 2.0f * P.hMax, limit = kCandidateMargin * reach * reach;
-    Origin O{F.cell[i], P.hMax, false, 0.0};
+    Origin O{0, P.hMax, false, 0.0};
     if (D == 3 && P.period > 0.0 && (pi[1] < reach || pi[1] > P.periodF - reach)) {
         O.seam = true;
         O.shift64 = pi[1] < 0.5f * P.periodF ? P.period : -P.period;
     }
+    // a neighbour within the support, its separation taken
+    auto take = [&](int j, int image, const float d[3], float r2, const NeighbourRows &R) {
+        const float r = r2 > 0.0f ? r2 * rsqrtf(r2) : 0.0f;
+        if (Visitor::kSkipCoincident && r < 1.0e-12f) return;
+        visit(j, d, r, signedLengthIn<D>(R.A, R.B) > 0.0f, image, R);
+    };
+    auto separation = [&](const NeighbourRows &R, int image, float d[3]) {
+        float pj[3], lj[3];
+        pointIn<D>(R.A, pj);
+        remainderIn<D>(R.A, R.B, lj);
+        return separation2<D>(P, pi, li, pj, lj, image ? (float)O.shift64 : 0.0f, image, O.shift64, d);
+    };
     const int held = P.listCap > 0 && !(whole && boundaryRow) ? fetch(&F.ncount[i]).x : P.listCap + 1;
-    const bool walking = P.listCap == 0 || held > P.listCap;
-    const int4 *column = reinterpret_cast<const int4 *>(F.nbr) + i;
-    Candidates<D, false> C;
-    if (walking) {
-        C.cellStart = F.cellStart;
-        C.startSearch(P, O, pi, li, 0);
-    }
-    int counted = 0, j = 0, image = 0, level = 0, k = 4 * t;
-    int4 chunk = make_int4(0, 0, 0, 0);
-    while (true) {
-        if (walking) {
-            if (!C.next(P, O, pi, li, j, image, level)) return;
-        } else {
-            if (k >= held) return;
-            if ((k & 3) == 0) chunk = fetch(column + (size_t)(k >> 2) * P.listStride);
-            j = chunk.x & 0x7FFFFFFF;
-            image = chunk.x < 0 ? 1 : 0;
+    if (P.listCap > 0 && held <= P.listCap) {
+        const int4 *column = reinterpret_cast<const int4 *>(F.nbr) + i;
+        int k = 4 * t;
+        if (k >= held) return;
+        int4 chunk = make_int4(0, 0, 0, 0), ahead = fetch(column + (size_t)t * P.listStride);
+        auto next = [&](int &entry) {
+            if (k >= held) return false;
+            if ((k & 3) == 0) {
+                chunk = ahead;
+                const int after = (k >> 2) + T;
+                if (4 * after < held) ahead = fetch(column + (size_t)after * P.listStride);
+            }
+            entry = chunk.x;
             chunk.x = chunk.y; chunk.y = chunk.z; chunk.z = chunk.w;
             k = (k & 3) == 3 ? k + 1 + 4 * (T - 1) : k + 1;
-        }
-        const float offset = image ? (float)O.shift64 : 0.0f;     // the search's origin: particle or image
-        const float4 A = fetch(&F.pa[j]);
-        float pj[3];
-        pointIn<D>(A, pj);
-        if (walking && (coarseDistance2<D>(pi, pj, offset) >= limit || j == i)) continue;
+            return true;
+        };
+        int entry = 0;
         NeighbourRows R;
-        R.A = A;
-        R.B = fetch(&F.pb[j]);
-        if (Visitor::kKinetic || D == 2) R.K = fetch(&F.kin[j]);
-        const bool fluidJ = signedLengthIn<D>(A, R.B) > 0.0f;
-        if (walking && fluidOnly && !fluidJ) continue;     // not in the row: not counted either
-        if ((T == 1 || !walking) && !visit.accept(fluidJ)) continue;
-        float lj[3], d[3];
-        remainderIn<D>(A, R.B, lj);
-        const float r2 = separation2<D>(P, pi, li, pj, lj, offset, image, O.shift64, d);
-        if (walking) {
-            if (r2 >= support2(P.hMax)) continue;
-            if (T > 1) {
-                if ((counted++ >> 2) % T != t) continue;
-                if (!visit.accept(fluidJ)) continue;
+        bool more = next(entry);
+        loadRows<D, true, Visitor>(F, entry & 0x7FFFFFFF, loadEarly(&F.pa[entry & 0x7FFFFFFF]), R);
+        while (more) {
+            int entryAfter = 0;
+            NeighbourRows after;
+            more = next(entryAfter);
+            if (more) loadRows<D, true, Visitor>(F, entryAfter & 0x7FFFFFFF, loadEarly(&F.pa[entryAfter & 0x7FFFFFFF]), after);
+            if (visit.accept(signedLengthIn<D>(R.A, R.B) > 0.0f)) {
+                const int image = entry < 0 ? 1 : 0;
+                float d[3];
+                const float r2 = separation(R, image, d);
+                take(entry & 0x7FFFFFFF, image, d, r2, R);
             }
+            entry = entryAfter;
+            R = after;
         }
-        const float r = r2 > 0.0f ? r2 * rsqrtf(r2) : 0.0f;
-        if (Visitor::kSkipCoincident && r < 1.0e-12f) continue;
-        if (D == 3) R.X = fetch(&F.aux[j]);
-        visit(j, d, r, fluidJ, image, R);
+        return;
+    }
+    O.cell = F.cell[i];
+    Candidates<D, false> C;
+    C.cellStart = F.cellStart;
+    C.startSearch(P, O, pi, li, 0);
+    int counted = 0, j = 0, image = 0, level = 0;
+    while (C.next(P, O, pi, li, j, image, level)) {
+        const float4 A = fetch(&F.pa[j]);
+        float pj[3], d[3];
+        pointIn<D>(A, pj);
+        const float offset = image ? (float)O.shift64 : 0.0f;     // the search's origin: particle or image
+        if (coarseDistance2<D>(pi, pj, offset) >= limit || j == i) continue;
+        NeighbourRows R;
+        loadRows<D, false, Visitor>(F, j, A, R);
+        const bool fluidJ = signedLengthIn<D>(A, R.B) > 0.0f;
+        if (fluidOnly && !fluidJ) continue;     // not in the row: not counted either
+        if (T == 1 && !visit.accept(fluidJ)) continue;
+        const float r2 = separation(R, image, d);
+        if (r2 >= support2(P.hMax)) continue;
+        if (T > 1) {
+            if ((counted++ >> 2) % T != t) continue;
+            if (!visit.accept(fluidJ)) continue;
+        }
+        take(j, image, d, r2, R);
     }
 }
 
 template <int D, int K>
 struct ShepardVisit {
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = false;
+    static constexpr bool kKinetic = D == 2, kAux = false, kMass = true, kLow = false;
     const Frame &F;
     KernelAt k;
     float num, den;
@@ -158,7 +201,7 @@ __global__ void __launch_bounds__(kBlock, 6) shepardKernel(Params P, Frame F, co
 template <int D, int K, bool BUDGET>
 struct MomentumVisit {
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kKinetic = true;
+    static constexpr bool kKinetic = true, kAux = true, kMass = false, kLow = false;
     const Params &P; const Frame &F;
     KernelAt k;
     float vi[3], rhoI, own, viscosityScale;   // viscosityScale: -alpha c0
@@ -238,7 +281,7 @@ __global__ void __launch_bounds__(kBlock, BUDGET ? 4 : D == 2 ? 8 : 6) momentumK
 template <int D, int K, bool BUDGET>
 struct ContinuityVisit {
     static constexpr bool kSkipCoincident = true;
-    static constexpr bool kKinetic = true;
+    static constexpr bool kKinetic = true, kAux = false, kMass = true, kLow = true;
     const Params &P; const Frame &F;
     KernelAt k;
     int self;               // this particle's slot
@@ -252,8 +295,7 @@ struct ContinuityVisit {
     {
         float vj[3];
         velocityIn<D>(R.K, vj);
-        const float4 lowJ = fetch(&F.low[j]);
-        const float vlJ[3] = {lowJ.x, lowJ.y, lowJ.z};
+        const float vlJ[3] = {R.L.x, R.L.y, R.L.z};
         if (boundaryI == fluidJ) {
             float pi[3], li[3], pj[3], lj[3];
             pointOf<D>(F, self, pi);
@@ -293,7 +335,7 @@ struct ContinuityVisit {
 
 // mode 0: the rate only; 1: advance the density (XSPH drifts).
 template <int D, int K, int T, bool BUDGET>
-__global__ void __launch_bounds__(kBlock, BUDGET ? 4 : 5) continuityKernel(Params P, Frame F, Control *ctl, int mode)
+__global__ void __launch_bounds__(kBlock, BUDGET || D == 3 ? 4 : 5) continuityKernel(Params P, Frame F, Control *ctl, int mode)
 {
     awaitPrevious();
     if (ctl && !ctl->active) return;
@@ -333,7 +375,7 @@ __global__ void __launch_bounds__(kBlock, BUDGET ? 4 : 5) continuityKernel(Param
 template <int D, int K>
 struct XsphVisit {
     static constexpr bool kSkipCoincident = false;
-    static constexpr bool kKinetic = true;
+    static constexpr bool kKinetic = true, kAux = true, kMass = false, kLow = false;
     const float *densities;
     KernelAt k;
     float vi[3], rhoI, corr[3];

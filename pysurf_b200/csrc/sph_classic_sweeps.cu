@@ -422,28 +422,28 @@ xsphKernel(Params P, Frame F, Control *ctl, Enforcement E, const float *densitie
 }
 
 template <int D, int K, int T>
-static bool launchT(const LaunchArgs &A, Stage stage)
+static void launchT(const LaunchArgs &A, Stage stage)
 {
     const int grid = (int)(((long long)A.P.n * T + kBlock - 1) / kBlock);
     cudaStream_t st = A.stream;
     switch (stage) {
-    case Stage::ShepardSum: launchNext(shepardKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl); return true;
+    case Stage::ShepardSum: launchNext(shepardKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl); break;
     case Stage::Momentum:
         if (A.P.budget && A.maxima) launchNext(momentumKernel<D, K, T, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxima);
         else launchNext(momentumKernel<D, K, T, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.maxima);
-        return true;
+        break;
     case Stage::Continuity:
         // the budget's parts matter only where the step advances the density
         if (A.P.budget && A.flag != 0) launchNext(continuityKernel<D, K, T, true>, grid, kBlock, st, A.P, A.F, A.ctl, A.flag);
         else launchNext(continuityKernel<D, K, T, false>, grid, kBlock, st, A.P, A.F, A.ctl, A.flag);
-        return true;
-    case Stage::Xsph: launchNext(xsphKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl, A.E, A.densities, A.flag); return true;
-    default: return false;
+        break;
+    case Stage::Xsph: launchNext(xsphKernel<D, K, T>, grid, kBlock, st, A.P, A.F, A.ctl, A.E, A.densities, A.flag); break;
+    default: break;
     }
 }
 
 template <int D, int K>
-static bool launchDK(const LaunchArgs &A, Stage stage)
+static void launchDK(const LaunchArgs &A, Stage stage)
 {
     if (A.threads >= 8) return launchT<D, K, 8>(A, stage);
     if (A.threads == 4) return launchT<D, K, 4>(A, stage);
@@ -453,9 +453,9 @@ static bool launchDK(const LaunchArgs &A, Stage stage)
 
 }  // namespace classic
 
-bool launchClassicStage(const LaunchArgs &A, Stage stage)
+void launchClassicStage(const LaunchArgs &A, Stage stage)
 {
-    if (A.P.n == 0) return true;
+    if (A.P.n == 0) return;
     if (A.P.dim == 2) return A.P.kind == 0 ? classic::launchDK<2, 0>(A, stage) : classic::launchDK<2, 1>(A, stage);
     return A.P.kind == 0 ? classic::launchDK<3, 0>(A, stage) : classic::launchDK<3, 1>(A, stage);
 }

@@ -69,25 +69,29 @@ struct LaunchArgs {
     float floorDet;
     const float *densities; // Xsph: the densities it divides by; null for the frame's
     int threads;            // threads per particle in the sweeps: 1, 2, 4 or 8
+    int classic;            // the classic scheme's sweeps, where it has its own
     int tabled;             // the table's rows were long enough for every particle when it was sized
     int *maxCount;          // List: the largest neighbour count goes here (atomic max), when given
 };
 
 // The stages of a 2D or a 3D system with the cubic spline (0) or the Wendland kernel (1)
 // (sph_sweep_kernels.cu; the Wendland units build the table for both), and of the classic scheme, where it
-// has its own (sph_classic_sweeps.cu; false where it has none).
+// has its own (sph_classic_sweeps.cu).
 void launchStage2_0(const LaunchArgs &A, Stage stage);
 void launchStage2_1(const LaunchArgs &A, Stage stage);
 void launchStage3_0(const LaunchArgs &A, Stage stage);
 void launchStage3_1(const LaunchArgs &A, Stage stage);
-bool launchClassicStage(const LaunchArgs &A, Stage stage);
+void launchClassicStage(const LaunchArgs &A, Stage stage);
+inline bool isClassic(Stage stage)
+{
+    return stage == Stage::ShepardSum || stage == Stage::Momentum || stage == Stage::Continuity || stage == Stage::Xsph;
+}
 inline void launchStage(const LaunchArgs &A, Stage stage)
 {
     LaunchArgs B = A;
-    if (A.P.together) {
-        if (launchClassicStage(A, stage)) return;
-        if (stage != Stage::List) B.P.listCap = 0;      // the paired sweeps' rows part the kinds: walk the cells
-    }
+    const bool classic = A.classic && isClassic(stage);
+    if (stage != Stage::List && (A.P.together != 0) != classic) B.P.listCap = B.tabled = 0;  // the other order's rows: walk
+    if (classic) return launchClassicStage(B, stage);
     const bool wendland = A.P.kind == 1 || stage == Stage::List;
     if (A.P.dim == 2) wendland ? launchStage2_1(B, stage) : launchStage2_0(B, stage);
     else wendland ? launchStage3_1(B, stage) : launchStage3_0(B, stage);

@@ -507,9 +507,8 @@ struct SphSystem {
         P.shiftDt = 0.0;
         P.wallExtrapolated = wallExtrapolated;
         P.xsphEpsilon = (float)xsphEpsilon;
-        P.together = classic() ? 1 : 0;
-        // rows of the other order (an option changed since they were built) are not read
-        P.listCap = listTogether == classic() ? listCap : 0;
+        P.together = listTogether ? 1 : 0;
+        P.listCap = listCap;
         P.listStride = capacity;
         P.budget = budget && energy ? 1 : 0;
         P.energyStride = energyCap;
@@ -547,7 +546,8 @@ struct SphSystem {
         A.E = enforcement;
         A.floorDet = (float)pow(0.25, dim);
         A.threads = threads;
-        A.tabled = A.P.listCap > 0 && !listCapped;
+        A.classic = classic() ? 1 : 0;
+        A.tabled = listCap > 0 && !listCapped;
         return A;
     }
 
@@ -1121,6 +1121,16 @@ static int needFrame(SphSystem *sys)
     return SPH_OK;
 }
 
+// The table's rows in the order that host sums read: the classic scheme's own sums take both kinds from the
+// front, every other sum (and every sum of another scheme) takes them parted.  The rows stay for the next
+// call, so a run of one kind of sum builds them once.
+static void needRows(SphSystem *sys, bool together)
+{
+    if (sys->n == 0 || sys->listCap == 0 || sys->listTogether == together) return;
+    sys->listTogether = together;
+    launchStage(sys->args(nullptr), Stage::List);
+}
+
 // Upload caller-order fields into the frame.
 static int loadFields(SphSystem *sys, const double *v, const double *rho, const double *p)
 {
@@ -1157,6 +1167,7 @@ int sph_pair_accelerations(SphSystem *sys, const double *velocities, const doubl
         return fail(SPH_ERR_INVALID, "null argument");
     if (sys->n == 0) return SPH_OK;
     TRY(loadFields(sys, velocities, densities, pressures));
+    needRows(sys, sys->classic());
     LaunchArgs A = sys->args(nullptr);
     A.P.c0 = (float)sound_speed;
     A.P.alpha = (float)alpha;
@@ -1182,6 +1193,7 @@ int sph_continuity_rate(SphSystem *sys, const double *velocities, const double *
     if (needsDensity && !densities)
         return fail(SPH_ERR_INVALID, "the diffusive term and the correction need the densities");
     TRY(loadFields(sys, velocities, needsDensity ? densities : nullptr, nullptr));
+    needRows(sys, sys->classic());
     LaunchArgs A = sys->args(nullptr);
     if (sys->corrected || sys->diffusionMode == 3) {
         A.wantL = 1;
@@ -1202,6 +1214,7 @@ int sph_xsph_velocity(SphSystem *sys, const double *velocities, const double *de
     if (sys->n == 0) return SPH_OK;
     if (!velocities || !densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, velocities, densities, nullptr));
+    needRows(sys, sys->classic());
     LaunchArgs A = sys->args(nullptr);
     A.P.xsphEpsilon = (float)epsilon;
     A.flag = 0;
@@ -1219,6 +1232,7 @@ int sph_wall_pressure(SphSystem *sys, const double *densities, const double *pre
     if (sys->n == 0) return SPH_OK;
     if (!densities || !pressures || !gravity || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, nullptr, densities, pressures));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     for (int a = 0; a < 3; ++a) A.P.g[a] = a < sys->dim ? (float)gravity[a] : 0.0f;
     A.P.rho0 = reference_density;
@@ -1236,6 +1250,7 @@ int sph_shepard_density(SphSystem *sys, const double *densities, double *out)
     if (sys->n == 0) return SPH_OK;
     if (!densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, nullptr, densities, nullptr));
+    needRows(sys, sys->classic());
     LaunchArgs A = sys->args(nullptr);
     launchStage(A, Stage::ShepardSum);
     launchScatterFloat(sys->n, A.F.orig, sys->scalar, sys->stage(SphSystem::kOutSlot), sys->stream);
@@ -1249,6 +1264,7 @@ int sph_velocity_gradients(SphSystem *sys, const double *velocities, const doubl
     if (sys->n == 0) return SPH_OK;
     if (!velocities || !densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, velocities, densities, nullptr));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     A.wantG = kWholeGradients;
     launchStage(A, Stage::Gradients);
@@ -1265,6 +1281,7 @@ int sph_closure_coefficients(SphSystem *sys, const double *velocities, const dou
     if (sys->n == 0) return SPH_OK;
     if (!velocities || !densities || !alphas || !deltas) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, velocities, densities, nullptr));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     A.wantG = 1;
     launchStage(A, Stage::Gradients);
@@ -1293,6 +1310,7 @@ int sph_shifting_displacement(SphSystem *sys, const double *densities, double ti
     if (!densities || !velocities || !shifts || !density_changes || !velocity_changes)
         return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, velocities, densities, nullptr));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     A.P.shiftDt = time_step;
     launchStage(A, Stage::ShiftFields);
@@ -1322,6 +1340,7 @@ int sph_correction_matrices(SphSystem *sys, const double *densities, double *out
     if (sys->n == 0) return SPH_OK;
     if (!densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, nullptr, densities, nullptr));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     A.wantL = 1;
     launchStage(A, Stage::Gradients);
@@ -1336,6 +1355,7 @@ int sph_density_gradients(SphSystem *sys, const double *densities, double *out)
     if (sys->n == 0) return SPH_OK;
     if (!densities || !out) return fail(SPH_ERR_INVALID, "null argument");
     TRY(loadFields(sys, nullptr, densities, nullptr));
+    needRows(sys, false);
     LaunchArgs A = sys->args(nullptr);
     A.wantRho = 1;
     launchStage(A, Stage::Gradients);

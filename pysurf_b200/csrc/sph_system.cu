@@ -143,7 +143,7 @@ struct SphSystem {
     int fineCells = 0;
     // device memory
     MasterView master[2]{};
-    float4 *pa = nullptr, *pb = nullptr, *kin = nullptr, *G[3] = {}, *L[3] = {}, *gradRho = nullptr, *acc = nullptr,
+    float4 *pa = nullptr, *pb = nullptr, *kin = nullptr, *L[3] = {}, *gradRho = nullptr, *acc = nullptr,
            *vec = nullptr, *S0 = nullptr;
     float2 *S1 = nullptr;
     float4 *aux = nullptr, *low = nullptr;
@@ -201,7 +201,7 @@ struct SphSystem {
             cudaFree(M.rho); cudaFree(M.m); cudaFree(M.h); cudaFree(M.fluid); cudaFree(M.orig);
             M = MasterView{};
         }
-        void *ptrs[] = {pa, pb, kin, S0, S1, G[0], G[1], G[2], L[0], L[1], L[2], gradRho, acc, vec, aux, low, pres, rate,
+        void *ptrs[] = {pa, pb, kin, S0, S1, L[0], L[1], L[2], gradRho, acc, vec, aux, low, pres, rate,
                         scalar, cell, sortBuffers.slotCell, sortBuffers.slotWithin, sortBuffers.perm,
                         sortBuffers.bucket, dStage, dStageU8, dRank, nbr, ncount, wallBits, eddy, shiftGrad, shiftPlain,
                         shiftRhoGrad, shiftOut, shiftDv};
@@ -216,7 +216,7 @@ struct SphSystem {
         listDirty = true;
         pa = pb = kin = gradRho = acc = vec = S0 = nullptr;
         S1 = nullptr;
-        for (int a = 0; a < 3; ++a) G[a] = L[a] = nullptr;
+        for (int a = 0; a < 3; ++a) L[a] = nullptr;
         aux = low = nullptr; pres = rate = scalar = nullptr; cell = nullptr;
         sortBuffers.slotCell = sortBuffers.slotWithin = sortBuffers.perm = nullptr;
         sortBuffers.bucket = nullptr;
@@ -280,7 +280,7 @@ struct SphSystem {
         TRY(deviceAlloc(&aux, cap));
         TRY(deviceAlloc(&low, cap));
         TRY(deviceAlloc(&pres, cap));
-        for (int a = 0; a < 3; ++a) { TRY(deviceAlloc(&G[a], cap)); TRY(deviceAlloc(&L[a], cap)); }
+        for (int a = 0; a < 3; ++a) TRY(deviceAlloc(&L[a], cap));
         TRY(deviceAlloc(&S0, cap));
         if (dim == 3) TRY(deviceAlloc(&S1, cap));
         TRY(deviceAlloc(&gradRho, cap));
@@ -521,7 +521,9 @@ struct SphSystem {
         Frame F{};
         F.pa = pa; F.pb = pb; F.kin = kin; F.aux = aux; F.low = low; F.pres = pres;
         F.cell = cell; F.cellStart = cellStart;
-        F.G0 = G[0]; F.G1 = G[1]; F.G2 = G[2];
+        // the whole gradients are for one call's caller (sph_velocity_gradients): they take the place of the
+        // shifting's fields, which each use of them writes anew
+        F.G0 = shiftGrad; F.G1 = shiftPlain; F.G2 = shiftRhoGrad;
         F.S0 = S0; F.S1 = S1;
         F.L0 = L[0]; F.L1 = L[1]; F.L2 = L[2];
         F.gradRho = gradRho; F.acc = acc; F.rate = rate; F.scalar = scalar; F.vec = vec; F.eddy = eddy;

@@ -31,9 +31,11 @@ namespace sph {
 // two neighbours' rows, and the next two's in flight, so it wants 90 to 160 registers; each bound is the
 // fastest of those measured around it on the 64-ppd beach (2D) and the 20-ppd and the refined 11-ppd
 // ridge (3D), with a neighbour's rows in an earlier layout (now 0.061 and 19.0 ms for continuity, 0.060 and
-// 14.8 ms for gradients, at the same bounds).  The energy budget's sweeps carry more sums.
+// 14.8 ms for gradients, at the same bounds).
+// the energy budget's sweeps, which carry more sums: 4 (3D momentum and continuity on the 8-ppd ridge 1.03 and
+// 1.37 ms against 1.25 and 1.61 at 3)
 template <int D>
-constexpr int budgetMinBlocks() { return D == 2 ? 4 : 3; }
+constexpr int budgetMinBlocks() { return 4; }
 // continuity: 5 in 2D (0.082 ms against 0.084 at 4), 4 in 3D (20.3 ms against 21.3 at 3)
 template <int D>
 constexpr int preciseMinBlocks() { return D == 2 ? 5 : 4; }

@@ -1617,11 +1617,11 @@ static void launchListAs(const LaunchArgs &A)
     }
 }
 
-// Particles too few to fill the chip take more of it each: 4 in place of 8 members a batch in 3D (below
-// 65,536 particles, 8,192 warps of 8; the 27,000-particle channel's table 0.322 -> 0.270 ms, while the
-// 760,000-particle ridge's goes from 3.17 to 3.65), 16 in place of 8 lanes a slot in 2D (below 24,576
-// particles; the 10,000-particle beach's table 0.0449 -> 0.0367 ms, the 114,000-particle one's 0.133 ->
-// 0.143).
+// Particles too few to fill the chip take more of it each: 4 in place of 8 members a batch in 3D, 16 in place
+// of 8 lanes a slot in 2D.  Each line lies where the two take the same time.  Sort and table, ms:
+//   2D   10,144 particles 0.0274 at 16 lanes, 0.0358 at 8; 32,546 0.0467, 0.0490; 42,081 0.0550, 0.0555;
+//        59,823 0.0691, 0.0674
+//   3D   26,866 0.256 at 4 a batch, 0.298 at 8; 46,056 0.344, 0.380; 69,084 0.455, 0.442; 130,492 0.734, 0.663
 template <int D>
 static void launchList(const LaunchArgs &A)
 {
@@ -1629,7 +1629,7 @@ static void launchList(const LaunchArgs &A)
         if (A.P.n < 65536) launchListAs<D, 4>(A);
         else launchListAs<D, 8>(A);
     } else {
-        if (A.P.n < 24576) launchListAs<D, 16>(A);
+        if (A.P.n < 45056) launchListAs<D, 16>(A);
         else launchListAs<D, 8>(A);
     }
 }

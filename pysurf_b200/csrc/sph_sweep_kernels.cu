@@ -1618,10 +1618,13 @@ static void launchListAs(const LaunchArgs &A)
 }
 
 // Particles too few to fill the chip take more of it each: 4 in place of 8 members a batch in 3D, 16 in place
-// of 8 lanes a slot in 2D.  Each line lies where the two take the same time.  Sort and table, ms:
-//   2D   10,144 particles 0.0274 at 16 lanes, 0.0358 at 8; 32,546 0.0467, 0.0490; 42,081 0.0550, 0.0555;
-//        59,823 0.0691, 0.0674
-//   3D   26,866 0.256 at 4 a batch, 0.298 at 8; 46,056 0.344, 0.380; 69,084 0.455, 0.442; 130,492 0.734, 0.663
+// of 8 lanes a slot in 2D.  Sort and table, ms:
+//   3D   26,866 particles 0.256 at 4 a batch, 0.298 at 8; 46,056 0.344, 0.380; 69,084 0.455, 0.442; 130,492
+//        0.734, 0.663
+//   2D   10,144 particles 0.0274 at 16 lanes, 0.0358 at 8; 22,701 0.0399, 0.0410; 25,798 0.0404, 0.0412;
+//        32,546 0.0467, 0.0490; 59,823 0.0691, 0.0674, all with some 100 neighbours; with 20, whose rows of
+//        cells give 16 lanes little, a 35,018-particle dam's span of 16 steps takes 1.583 ms at 16 and 1.521
+//        at 8
 template <int D>
 static void launchList(const LaunchArgs &A)
 {

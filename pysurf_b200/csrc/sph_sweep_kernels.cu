@@ -1632,7 +1632,7 @@ static void launchList(const LaunchArgs &A)
         if (A.P.n < 65536) launchListAs<D, 4>(A);
         else launchListAs<D, 8>(A);
     } else {
-        if (A.P.n < 45056) launchListAs<D, 16>(A);
+        if (A.P.n < 24576) launchListAs<D, 16>(A);
         else launchListAs<D, 8>(A);
     }
 }

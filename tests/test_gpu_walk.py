@@ -79,10 +79,3 @@ def test_rows_too_short_for_their_counts(dim, threads, scheme):
     if lengths is None:
         assert over.any() and not over.all()
     sameBits(*runs)
-
-
-@pytest.mark.parametrize('n', [45055, 45056])
-def test_the_2d_tables_lanes(n):
-    # either side of the size at which the 2D table kernel takes 8 lanes a slot in place of 16
-    x, v, rho, m, fluid, h = cloud(2, n, 6, ratio=1.3)
-    sameBits(*(sums(pairSums(2, h, table), x, v, rho, m, fluid) for table in (False, True)))

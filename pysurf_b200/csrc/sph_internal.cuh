@@ -34,9 +34,11 @@
 namespace sph {
 
 constexpr int kBlock = 128;                 // threads per sweep block
-// Resident sweep blocks an SM, which caps a sweep's registers: the momentum sweep runs fastest at 5 in 2D
-// (0.084 ms on the 64-ppd beach against 0.088 at 6) and 4 in 3D (16.5 ms on the 20-ppd ridge against 20.1
-// at 5).
+// Resident sweep blocks an SM, which caps a sweep's registers (momentum, XSPH and the shifting's fields).
+// Momentum, ms: 3D 4 (17.1 on the 20-ppd ridge, 21.2 at 3, 20.1 at 5); 2D 5 (0.078 on the 64-ppd beach,
+// 0.090 at 4).  At 6 in 2D, with continuity at 6 too, the beach's plain form takes 0.073 and its step 2% less,
+// but the forms that carry more spill: the closure's, the compensated, the mixed lengths' and the cubic
+// spline's steps and those of 10,000 particles take 3 to 14% more.
 template <int D>
 constexpr int sweepMinBlocks() { return D == 2 ? 5 : 4; }
 constexpr float kViscositySoftening = 0.01f;   // mu_ij's r^2 + 0.01 h^2 (src/pysurf/sphSolver.py:213)

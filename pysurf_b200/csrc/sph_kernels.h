@@ -33,7 +33,7 @@ struct Enforcement {
 };
 
 // Launches a kernel that begins with awaitPrevious(): its blocks are set up while the kernel before it in
-// the stream still runs, which takes the launch's latency off each of a step's 13 kernels.  A step with
+// the stream still runs, which takes the launch's latency off each of a step's 12 to 15 kernels.  A step with
 // plain launches and event nodes between its stages, and now: the 600-particle tank 0.098 -> 0.060 ms, the
 // 10,000-particle beach 0.115 -> 0.078, the 114,000-particle one 0.360 -> 0.326; a 760,000-particle ridge's
 // 9.7 ms do not change.

@@ -27,19 +27,18 @@
 
 namespace sph {
 
-// Resident blocks of 128 threads an SM each sweep is built for, which caps its registers.  A sweep holds
-// two neighbours' rows, and the next two's in flight, so it wants 90 to 160 registers; each bound is the
-// fastest of those measured around it on the 64-ppd beach (2D) and the 20-ppd and the refined 11-ppd
-// ridge (3D), with a neighbour's rows in an earlier layout (now 0.061 and 19.0 ms for continuity, 0.060 and
-// 14.8 ms for gradients, at the same bounds).
+// Resident blocks of 128 threads an SM each sweep is built for, which caps its registers (sweepMinBlocks()
+// for the others).  A sweep holds two neighbours' rows, and the next two's in flight, so it wants 90 to 160
+// registers.  ms on the 64-ppd beach (2D) and the 20-ppd ridge (3D):
 // the energy budget's sweeps, which carry more sums: 4 (3D momentum and continuity on the 8-ppd ridge 1.03 and
 // 1.37 ms against 1.25 and 1.61 at 3)
 template <int D>
 constexpr int budgetMinBlocks() { return 4; }
-// continuity: 5 in 2D (0.082 ms against 0.084 at 4), 4 in 3D (20.3 ms against 21.3 at 3)
+// continuity: 5 in 2D (0.058, 0.066 at 4; sweepMinBlocks() says why not 6), 4 in 3D (18.3, 22.3 at 3, 30.3 at
+// 5)
 template <int D>
 constexpr int preciseMinBlocks() { return D == 2 ? 5 : 4; }
-// gradients: 5 in 2D (0.061 ms against 0.070 at 6), 3 in 3D (15.9 ms against 16.6 at 4)
+// gradients: 5 in 2D (0.056, 0.062 at 6), 3 in 3D (15.1, 24.2 at 4)
 template <int D>
 constexpr int gradientMinBlocks() { return D == 2 ? 5 : 3; }
 

@@ -282,13 +282,13 @@ def measuredPeaks() -> dict:
 
 def profiledTraffic(case, kernel: str, refined: bool, fluid: int) -> float | None:
     """DRAM bytes a launch of `kernel` (gradients, momentum, continuity) from the committed ncu summary of
-    this workload: the beach at its own size; the refined ridge captured at 12 ppd (the bench's size
+    this workload: the beach at its own size; the refined ridge captured at 8 ppd (the bench's size
     is too large to capture), whose traffic -- the neighbour table, which grows with the particles --
     is scaled to this run by its fluid particles after the split."""
     if case.dimensions == 2:
         name = 'sweeps_solitaryBeach64.md'
     elif refined:
-        name = 'sweeps_ridgeWave3D12_refined.md'
+        name = 'sweeps_ridgeWave3D8_refined.md'
     else:
         return None
     path = os.path.join(ROOT, 'profiles', name)

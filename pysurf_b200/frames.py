@@ -8,8 +8,9 @@ the caller adds.  This module writes the same files, so the reference's ``readIn
 
     FrameWriter.write          a frame from a particle state on the host, as the reference writes it
     FrameWriter.writeDevice    the same frame from a ``PairSums``' device state: the device rounds
-                               positions and speeds to float32 itself (``sph_frame``), so 17 bytes a
-                               particle cross the bus instead of a float64 pull's 48
+                               positions and speeds to float32 and packs the fluid's rows
+                               (``sph_fluid_frame``), so 12 bytes a fluid particle in 2D and 16 in 3D
+                               cross the bus
     readIndex, readFrame       a run's index and one frame's arrays
 """
 from __future__ import annotations

@@ -1194,7 +1194,7 @@ struct ContinuityVisit {
         const double *dd = taken.dd[Q], *dv = taken.dv[Q];
         double r2 = 0.0;
         for (int a = 0; a < D; ++a) r2 = fma(dd[a], dd[a], r2);
-        const double rr = preciseRoot(r2, Q ? N.inverse.y : N.inverse.x);
+        const double rr = preciseRoot<true>(r2, Q ? N.inverse.y : N.inverse.x);
         const double weight = __dmul_rn((double)taken.mass[Q], kernelGradient64<K>(rr, N.k.of(Q)));
         if (corrected) {
             for (int a = 0; a < D; ++a) {

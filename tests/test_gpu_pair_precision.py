@@ -92,3 +92,25 @@ def test_the_smallest_viscosity_is_not_lost(dim):
     whole = s.pairAccelerations(v, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
     small = s.pairAccelerations(v * 2.0 ** -118, rho, zero, C0, 0.05, 0.5, np.zeros(dim))
     assert np.abs(small * 2.0 ** 118 - whole).max() < 1e-6 * np.abs(whole).max()
+
+
+@pytest.mark.parametrize('dim', [2, 3])
+def test_a_wall_pair_far_from_the_origin(dim):
+    # With separations from the float32 points alone, whose places at 2^18 are 2^-5 = h / 4 apart, a pair's
+    # float32 distance can be less than half its own.  The wall's term takes its distance in float64 from
+    # that one: it stays within its value at no distance, m (5 sigma / h^2) |(v_i - v_j) . (x_i - x_j)|.
+    from pysurf_b200.sphGpu import PairSums
+    rng = np.random.default_rng(70 + dim)
+    h = 2.0 ** -3
+    side = 64 if dim == 2 else 16
+    places = np.stack(np.meshgrid(*[np.arange(side)] * dim, indexing='ij'), -1).reshape(-1, dim)
+    n = len(places)
+    centres = 2.0 ** 18 + (places + 1) * (8 * h) + rng.uniform(-0.5, 0.5, (n, dim)) * h
+    x = np.concatenate([centres, centres + rng.uniform(-0.6, 0.6, (n, dim)) * h])
+    v = rng.uniform(-1.0, 1.0, (2 * n, dim))
+    sums = PairSums(dim, h, x.min(axis=0) - h, x.max(axis=0) + h, kernelType='wendlandC2',
+                    separationPrecision='float32')
+    sums.update(x, np.ones(2 * n), np.arange(2 * n) < n)
+    rate = np.abs(sums.continuityRate(v)[:n])
+    bound = 5.0 * sums.sigmaUnit / h ** dim / h ** 2 * np.abs(((v[:n] - v[n:]) * (x[:n] - x[n:])).sum(axis=1))
+    assert rate.max() > 0.0 and np.all(rate <= bound * (1.0 + 1e-6))

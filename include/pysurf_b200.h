@@ -306,7 +306,7 @@ int sph_finish_steps(SphSystem *sys, double *time, int64_t *step, double *last_d
 
 /* Timing of the last sph_advance call (milliseconds, device events), and, from its kernels' stamps of
  * the device timer, of each stage of the
- * last step that ran (cells, filter, wall, gradients, momentum, kick, continuity: *count of them,
+ * last step of the device loop that ran (cells, filter, wall, gradients, momentum, kick, continuity: *count of them,
  * named by sph_stage_name), and the kernels one step launches. */
 int sph_last_advance_ms(const SphSystem *sys, double *ms);
 int sph_stage_times(SphSystem *sys, double *ms, int64_t capacity, int64_t *count);

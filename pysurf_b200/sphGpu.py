@@ -676,7 +676,7 @@ class PairSums:
         return [self._lib.sph_stage_name(k).decode() for k in range(count.value)]
 
     def stageTimes(self) -> list:
-        """Milliseconds of each stage of the last step that ran (its kernels' stamps of the device timer)."""
+        """Milliseconds of each stage of the device loop's last step that ran (its kernels' stamps of the device timer)."""
         count = _lib.C.c_int64(0)
         self._lib.sph_stage_times(self._handle, None, 0, _lib.C.byref(count))
         ms = np.zeros(count.value)
